@@ -25,6 +25,21 @@ struct HexGeo {
   const int* adv_cells;  // [E][advW]
   const int* n_adv;      // [E]
   const int* kite_slot;  // [C][maxE]
+  // Stencil records: what a neighbour loop needs of one neighbour, packed for
+  // one or two loads.  Entities are given as word offsets (index x S) into
+  // their [entity][level] fields; S is a multiple of 8, so the low bits of an
+  // offset are free and a slot's bit 0 holds the edge's sign (1: csign = -1).
+  int nbrW;              // pairs per edge: (maxE2 + 1) / 2
+  const int4* nbr;       // [E][nbrW] two TRiSK neighbours: offset, weight, offset, weight
+  const int* adv_off;    // [E][advW] advection stencil: cell offset
+  const float2* adv_pm;  // [E][advW] A + X, A - X (X = coef3 x third-order weight)
+  const int2* slot;      // [C][maxE] edge offset and sign, offset of the cell across the edge
+  const float* sdv;      // [C][maxE] csign x dv
+  const int2* vslot;     // [C][maxE] vertex offset, kite area
+  const int2* eslot;     // [C][maxE] edge offset, dc x dv
+  const int4* vedge;     // [V][3] edge offset, vsign x dc, dc x dv, 0
+  const int2* ends;      // [E] offsets of the edge's two cells
+  const int2* vends;     // [E] offsets of the edge's two vertices
   // per-entity FP32 (already rounded to RKIND exactly as the reference does)
   const float* csign;     // [C][maxE] edgesOnCell_sign (+1 cell1, -1 cell2)
   const float* vsign;     // [V][3]

@@ -35,13 +35,41 @@ __device__ __forceinline__ float neg0(float x) { return x < 0.0f ? x : 0.0f; }
 __device__ __forceinline__ float pymin(float a, float b) { return b < a ? b : a; }
 __device__ __forceinline__ float pymax(float a, float b) { return b > a ? b : a; }
 
-__device__ __forceinline__ float flux4f(float qm2, float qm1, float q0, float qp1, float vel) {
-  return vel * (7.0f * (q0 + qm1) - (qp1 + qm2)) / 12.0f;
+// The two terms of the third-order fluxes are divided by 12.  x / 12 is
+// x RH + x RL with RH the 24-bit truncation of 1/12 and RL the rest: the sum
+// in one fused operation is within 2^-46 of the quotient, which never lies
+// nearer than 1/6 ulp to a rounding boundary (2 x 2^j is even, 3 (2 n + 1)
+// odd), so it rounds as IEEE division does, for x = +-0, infinities, NaN
+// and every |x| >= 2^-118 (below, x RL loses bits).  Both constants are
+// positive, so zeros keep their sign.  Two operations instead of the
+// division's reciprocal sequence, range check and branch.
+#define HEX_DIV12_SMALL 0x04800000u  // 2^-118
+__device__ __forceinline__ float div12_wide(float x) {
+  return __fmaf_rn(x, __uint_as_float(0x3DAAAAAAu), __fmul_rn(x, __uint_as_float(0x31AAAAABu)));
 }
-// hexcore/dynamics.py:71 flux3 and hexcore/transport.py:440 (both add the
-// coefficient term).
-__device__ __forceinline__ float flux3f(float qm2, float qm1, float q0, float qp1, float vel, float coef) {
-  return flux4f(qm2, qm1, q0, qp1, vel) + coef * fabsf(vel) * ((qp1 - qm2) - 3.0f * (q0 - qm1)) / 12.0f;
+// x / 12 of any x, by way of 64 bits: x times 1/12 rounded to 53 bits is
+// within 2^-52 of the quotient, whose rounding boundaries (also in the
+// subnormal range) lie 1/12 of a step away or more, or it is a boundary
+// itself, a double that the product then rounds to (1/12 is rounded down by
+// one part in 2^54).
+__device__ __forceinline__ float div12_any(float x) { return (float)((double)x * (1.0 / 12.0)); }
+// Orders |x| with zero last: below div12_key(2^-118) exactly for the x that
+// div12_wide does not divide.
+__device__ __forceinline__ unsigned div12_key(float x) { return (__float_as_uint(x) << 1) - 1u; }
+#define HEX_DIV12_KEY ((HEX_DIV12_SMALL << 1) - 1u)
+// out[i] = x[i] / 12 + y[i] / 12; one branch for all of them.
+template <int N>
+__device__ __forceinline__ void div12_sum(const float (&x)[N], const float (&y)[N], float (&out)[N]) {
+  unsigned key = 0xffffffffu;
+#pragma unroll
+  for (int i = 0; i < N; ++i) key = umin(key, umin(div12_key(x[i]), div12_key(y[i])));
+  if (key >= HEX_DIV12_KEY) {
+#pragma unroll
+    for (int i = 0; i < N; ++i) out[i] = div12_wide(x[i]) + div12_wide(y[i]);
+  } else {
+#pragma unroll
+    for (int i = 0; i < N; ++i) out[i] = div12_any(x[i]) + div12_any(y[i]);
+  }
 }
 
 // ------------------------------------------------------------ recovery

@@ -17,17 +17,8 @@
 #define HEX_VEC_MIN_BLOCKS 4
 #endif
 #define HEX_VEC_BOUNDS __launch_bounds__(256, HEX_VEC_MIN_BLOCKS)
-// Third-order stencil weights A + (coef3 sign v) B selected from A + X and
-// A - X per level (1) or formed per level (0): the same words.  Measured:
-// the tracer edge values 162.6 -> 155.3 us per launch with the selection,
-// the theta/w edge values 58.5 -> 60.5 (kept per level).
-#ifndef HEX_PM_SELECT_EDGE_ADV
-#define HEX_PM_SELECT_EDGE_ADV 0
-#endif
-#ifndef HEX_PM_SELECT_TR_EDGE
-#define HEX_PM_SELECT_TR_EDGE 1
-#endif
-// Kernels measured faster at another cap: the momentum tendency (a
+// Kernels measured faster at another cap: the cell tendencies at 3 blocks
+// (80 registers, no spills: 80.8 vs 81.5 us), the edge diagnostics at 6, the momentum tendency (a
 // latency-bound ten-point gather) at 6 blocks (40 registers), the tracer
 // edge values (three tracers' accumulators per thread) at 2 (128), the
 // limited antidiffusive flux at 6 and the standard tracer update at 5.
@@ -134,22 +125,45 @@ __device__ __forceinline__ void st4m(float* p, const V4& v, int k0, int lo, int 
 #endif
 }
 
-// Column window col[k0-4 .. k0+7] around a thread's chunk; entries outside
-// [0, S) read as zero and are never used by a formula.
+// Stencil records (dycore_geo.cuh): a float kept as bits; a slot's edge
+// offset and sign.
+// c + s x with s = +-1: the product is exact, so the fused operation rounds
+// once, as c + (s x) does.
+__device__ __forceinline__ float fma_sign(float s, float x, float c) { return __fmaf_rn(s, x, c); }
+__device__ __forceinline__ float fbits(int x) { return __int_as_float(x); }
+__device__ __forceinline__ int slot_edge(int x) { return x & ~1; }
+__device__ __forceinline__ float slot_sign(int x) { return __int_as_float(0x3f800000 | (x << 31)); }
+
+// A divisor at level k: one in the padding levels, where the operands are
+// zero and 0 / 0 would take the division's slow path in every warp that
+// holds a column's top chunk (the masked stores drop those words).
+__device__ __forceinline__ float inside(float x, int k, int L) { return k < L ? x : 1.0f; }
+
+// Column window col[k0-2 .. k0+5] around a thread's chunk, of which LO
+// levels below the chunk and HI above it are loaded (0 to 2 each); entries
+// outside [0, S) read as zero and are used by no formula.
 struct Win {
-  float a[12];
-  __device__ __forceinline__ float operator()(int d) const { return a[d + 4]; }
+  float a[8];
+  __device__ __forceinline__ float operator()(int d) const { return a[d + 2]; }
 };
+template <int LO, int HI>
 __device__ __forceinline__ Win win(const float* __restrict__ col, int k0, int S) {
   Win w;
-  const V4 m = ld4(col + k0);
-  const V4 lo = k0 >= 4 ? ld4(col + k0 - 4) : v4zero();
-  const V4 hi = k0 + 4 < S ? ld4(col + k0 + 4) : v4zero();
+  const V4 v = ld4(col + k0);
 #pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    w.a[j] = lo.a[j];
-    w.a[j + 4] = m.a[j];
-    w.a[j + 8] = hi.a[j];
+  for (int j = 0; j < 4; ++j) w.a[j + 2] = v.a[j];
+  w.a[0] = w.a[1] = w.a[6] = w.a[7] = 0.0f;
+  if (LO == 1 && k0 > 0) w.a[1] = __ldg(col + k0 - 1);
+  if (LO == 2 && k0 > 0) {
+    const float2 t = __ldg(reinterpret_cast<const float2*>(col + k0 - 2));
+    w.a[0] = t.x;
+    w.a[1] = t.y;
+  }
+  if (HI == 1 && k0 + 4 < S) w.a[6] = __ldg(col + k0 + 4);
+  if (HI == 2 && k0 + 4 < S) {
+    const float2 t = __ldg(reinterpret_cast<const float2*>(col + k0 + 4));
+    w.a[6] = t.x;
+    w.a[7] = t.y;
   }
   return w;
 }
@@ -202,8 +216,9 @@ __global__ void HEX_VEC_BOUNDS kv_moist_edge(HexGeo g, const float* __restrict__
   HEX_VEC_PARALLEL(g.nE)
   const int e = ent, S = g.S;
   const size_t tstride = (size_t)g.nC * S;
-  const float* q0 = q + g.coe[2 * e] * S + k0;
-  const float* q1 = q + g.coe[2 * e + 1] * S + k0;
+  const int2 ends = __ldg(g.ends + e);
+  const float* q0 = q + ends.x + k0;
+  const float* q1 = q + ends.y + k0;
   V4 acc = v4zero();
   HEX_GATHER
   for (int t = 0; t < nT; ++t) {
@@ -227,10 +242,9 @@ __global__ void HEX_VEC_BOUNDS kv_diag_vertex(HexGeo g, const float* __restrict_
   V4 vort = v4zero(), ke[3];
 #pragma unroll
   for (int s = 0; s < 3; ++s) {
-    const int e = g.eov[3 * v + s];
-    const float vd = g.vsign[3 * v + s] * g.dc[e];
-    const float dd = g.dc[e] * g.dv[e];
-    const V4 ue = ld4(u + e * S + k0);
+    const int4 r = __ldg(g.vedge + 3 * v + s);
+    const float vd = fbits(r.y), dd = fbits(r.z);
+    const V4 ue = ld4(u + k0 + r.x);
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       vort.a[j] = vort.a[j] + vd * ue.a[j];
@@ -260,16 +274,18 @@ __global__ void HEX_VEC_BOUNDS kv_diag_cell(HexGeo g, const float* __restrict__ 
   const int c = ent, S = g.S;
   const int n = g.deg[c];
   const float ia = g.inv_area[c];
+  const int2* slots = g.vslot + c * g.maxE;
+  const int2* eslots = g.eslot + c * g.maxE;
   V4 ke = v4zero(), dv = v4zero();
   HEX_GATHER
   for (int s = 0; s < n; ++s) {
-    const int e = g.eoc[c * g.maxE + s];
-    const float dd = g.dc[e] * g.dv[e];
-    const V4 ue = ld4(u + e * S + k0);
+    const int2 r = __ldg(eslots + s);
+    const float dd = fbits(r.y);
+    const V4 ue = ld4(u + k0 + r.x);
 #pragma unroll
     for (int j = 0; j < 4; ++j) ke.a[j] = ke.a[j] + 0.25f * (dd * (ue.a[j] * ue.a[j]));
     if (DIV) {
-      const float sd = g.csign[c * g.maxE + s] * g.dv[e];
+      const float sd = __ldg(g.sdv + c * g.maxE + s);
 #pragma unroll
       for (int j = 0; j < 4; ++j) dv.a[j] = dv.a[j] + sd * ue.a[j];
     }
@@ -281,31 +297,27 @@ __global__ void HEX_VEC_BOUNDS kv_diag_cell(HexGeo g, const float* __restrict__ 
   }
 #pragma unroll
   for (int j = 0; j < 4; ++j) ke.a[j] = ke.a[j] * ia * 0.625f;
+  V4 pvc = v4zero();
   HEX_GATHER
   for (int s = 0; s < n; ++s) {
-    const int vtx = g.voc[c * g.maxE + s];
-    const float kt = (1.0f - 0.625f) * g.kite[3 * vtx + g.kite_slot[c * g.maxE + s]];
-    const V4 kv = ld4(ke_vertex + vtx * S + k0);
+    const int2 r = __ldg(slots + s);
+    const float kite = fbits(r.y);
+    const float kt = (1.0f - 0.625f) * kite;
+    const V4 kv = ld4(ke_vertex + k0 + r.x);
 #pragma unroll
     for (int j = 0; j < 4; ++j) ke.a[j] = ke.a[j] + kt * kv.a[j] * ia;
-  }
-  st4m(ke_out + c * S + k0, ke, k0, 0, g.L);
-  if (g.apvm_on) {
-    V4 pvc = v4zero();
-    HEX_GATHER
-    for (int s = 0; s < n; ++s) {
-      const int vtx = g.voc[c * g.maxE + s];
-      const float kite = g.kite[3 * vtx + g.kite_slot[c * g.maxE + s]];
-      const V4 pv = ld4(pv_vertex + vtx * S + k0);
+    if (g.apvm_on) {
+      const V4 pv = ld4(pv_vertex + k0 + r.x);
 #pragma unroll
       for (int j = 0; j < 4; ++j) pvc.a[j] = pvc.a[j] + kite * pv.a[j] * ia;
     }
-    st4m(pv_cell + c * S + k0, pvc, k0, 0, g.L);
   }
+  st4m(ke_out + c * S + k0, ke, k0, 0, g.L);
+  if (g.apvm_on) st4m(pv_cell + c * S + k0, pvc, k0, 0, g.L);
 }
 
 // Tangential velocity (TRiSK weights) and edge PV with APVM upwinding.
-__global__ void HEX_VEC_BOUNDS kv_diag_edge(HexGeo g, const float* __restrict__ u, const float* __restrict__ pv_vertex,
+__global__ void __launch_bounds__(256, 6) kv_diag_edge(HexGeo g, const float* __restrict__ u, const float* __restrict__ pv_vertex,
                              const float* __restrict__ pv_cell, float* __restrict__ v, float* __restrict__ pv_edge,
                              int recompute_v) {
   HEX_VEC_PARALLEL(g.nE)
@@ -314,25 +326,34 @@ __global__ void HEX_VEC_BOUNDS kv_diag_edge(HexGeo g, const float* __restrict__ 
   if (recompute_v) {
     vt = v4zero();
     const int n = g.neoe[e];
+    const int4* nbr = g.nbr + (size_t)e * g.nbrW;
     HEX_GATHER
-    for (int s = 0; s < n; ++s) {
-      const float w = g.weights[e * g.maxE2 + s];
-      const V4 un = ld4(u + g.eoe[e * g.maxE2 + s] * S + k0);
+    for (int s = 0; s + 1 < n; s += 2) {
+      const int4 r = __ldg(nbr + (s >> 1));
+      const V4 ua = ld4(u + k0 + r.x), ub = ld4(u + k0 + r.z);
 #pragma unroll
-      for (int j = 0; j < 4; ++j) vt.a[j] = vt.a[j] + w * un.a[j];
+      for (int j = 0; j < 4; ++j) vt.a[j] = vt.a[j] + fbits(r.y) * ua.a[j];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) vt.a[j] = vt.a[j] + fbits(r.w) * ub.a[j];
+    }
+    if (n & 1) {
+      const int4 r = __ldg(nbr + (n >> 1));
+      const V4 un = ld4(u + k0 + r.x);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) vt.a[j] = vt.a[j] + fbits(r.y) * un.a[j];
     }
     st4m(v + e * S + k0, vt, k0, 0, g.L);
   } else {
     vt = ld4rw(v + e * S + k0);
   }
-  const int v0 = g.voe[2 * e], v1 = g.voe[2 * e + 1];
-  const V4 p0 = ld4(pv_vertex + v0 * S + k0), p1 = ld4(pv_vertex + v1 * S + k0);
+  const int2 ve = __ldg(g.vends + e);
+  const V4 p0 = ld4(pv_vertex + k0 + ve.x), p1 = ld4(pv_vertex + k0 + ve.y);
   V4 pve;
 #pragma unroll
   for (int j = 0; j < 4; ++j) pve.a[j] = 0.5f * (p0.a[j] + p1.a[j]);
   if (g.apvm_on) {
-    const int c0 = g.coe[2 * e], c1 = g.coe[2 * e + 1];
-    const V4 q0 = ld4(pv_cell + c0 * S + k0), q1 = ld4(pv_cell + c1 * S + k0);
+    const int2 ce = __ldg(g.ends + e);
+    const V4 q0 = ld4(pv_cell + k0 + ce.x), q1 = ld4(pv_cell + k0 + ce.y);
     const V4 ue = ld4(u + e * S + k0);
     const float idv = g.inv_dv[e], idc = g.inv_dc[e];
 #pragma unroll
@@ -358,7 +379,8 @@ __global__ void HEX_VEC_BOUNDS kv_euler_edge(HexGeo g, const float* __restrict__
                               float* __restrict__ euler_ru) {
   HEX_VEC_PARALLEL(g.nE)
   const int e = ent, S = g.S;
-  const int i0 = g.coe[2 * e] * S + k0, i1 = g.coe[2 * e + 1] * S + k0;
+  const int2 ends = __ldg(g.ends + e);
+  const int i0 = ends.x + k0, i1 = ends.y + k0;
   const V4 p0 = ld4(pp + i0), p1 = ld4(pp + i1), r0 = ld4(rp + i0), r1 = ld4(rp + i1);
   // moisture terms of dpdz are read only with native moist coefficients
   const bool m = g.moist;
@@ -372,7 +394,7 @@ __global__ void HEX_VEC_BOUNDS kv_euler_edge(HexGeo g, const float* __restrict__
   for (int j = 0; j < 4; ++j) {
     const float d0 = dpdz_of(g, r0.a[j], q0.a[j], b0.a[j]);
     const float d1 = dpdz_of(g, r1.a[j], q1.a[j], b1.a[j]);
-    out.a[j] = -cq.a[j] * ((p1.a[j] - p0.a[j]) * idc / (0.5f * (z1.a[j] + z0.a[j])) - 0.5f * zx.a[j] * (d0 + d1));
+    out.a[j] = -cq.a[j] * ((p1.a[j] - p0.a[j]) * idc / inside(0.5f * (z1.a[j] + z0.a[j]), k0 + j, g.L) - 0.5f * zx.a[j] * (d0 + d1));
   }
   st4m(euler_ru + e * S + k0, out, k0, 0, g.L);
 }
@@ -383,9 +405,8 @@ __device__ __forceinline__ V4 mass_flux_div4(const HexGeo& g, const float* __res
   const int n = g.deg[c];
   HEX_GATHER
   for (int s = 0; s < n; ++s) {
-    const int e = g.eoc[c * g.maxE + s];
-    const float sd = g.csign[c * g.maxE + s] * g.dv[e];
-    const V4 r = ld4(ru + e * g.S + k0);
+    const float sd = __ldg(g.sdv + c * g.maxE + s);
+    const V4 r = ld4(ru + k0 + __ldg(g.eslot + c * g.maxE + s).x);
 #pragma unroll
     for (int j = 0; j < 4; ++j) acc.a[j] = acc.a[j] + sd * r.a[j];
   }
@@ -404,10 +425,10 @@ __global__ void HEX_VEC_BOUNDS kv_euler_cell(HexGeo g, const float* __restrict__
   HEX_VEC_PARALLEL(g.nC)
   const int c = ent, S = g.S, L = g.L;
   const V4 hd = mass_flux_div4(g, ru, c, k0);
-  const Win rww = win(rw + c * S, k0, S);
-  const Win ppw = win(pp + c * S, k0, S), rpw = win(rp + c * S, k0, S);
+  const Win rww = win<0, 1>(rw + c * S, k0, S);
+  const Win ppw = win<1, 0>(pp + c * S, k0, S), rpw = win<1, 0>(rp + c * S, k0, S);
   const bool m = g.moist;
-  const Win qtw = m ? win(qtot + c * S, k0, S) : Win{}, rbw = m ? win(g.rho_base + c * S, k0, S) : Win{};
+  const Win qtw = m ? win<1, 0>(qtot + c * S, k0, S) : Win{}, rbw = m ? win<1, 0>(g.rho_base + c * S, k0, S) : Win{};
   const V4 cq = m ? ld4(cqw + c * S + k0) : v4zero();
   V4 tr, er;
 #pragma unroll
@@ -453,73 +474,66 @@ __global__ void __launch_bounds__(256, HEX_EDGE_ADV_MIN_BLOCKS) kv_edge_adv(HexG
   HEX_VEC_PARALLEL(g.nE)
   const int e = ent, S = g.S;
   const int n = g.n_adv[e];
-  const int* cells = g.adv_cells + (size_t)e * g.advW;
-  const float* a1 = g.adv + (size_t)e * g.advW;
-  const float* a3 = g.adv3 + (size_t)e * g.advW;
+  const int* off = g.adv_off + (size_t)e * g.advW;
+  const float2* pm = g.adv_pm + (size_t)e * g.advW;
   const V4 r = ld4(ru + e * S + k0);
   const float rm = k0 > 0 ? ru[e * S + k0 - 1] : 0.0f;
-#if HEX_PM_SELECT_EDGE_ADV
-  // The stencil weight A + (coef3 sign(v)) B is A + X or A - X with
-  // X = coef3 B (a product's sign is exact, and a - b == a + (-b)): both are
-  // formed once per stencil point and each level selects by the sign bit
-  // of its velocity, the words of the per-level form.
+  const V4 fm = ld4(g.fzm + k0), fp = ld4(g.fzp + k0);
+  // The stencil weight A + (coef3 sign(v)) B is one of the record's two
+  // sums, by the sign bit of the level's velocity.
   bool nt[4], nw[4];
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
-    const int k = k0 + j;
     nt[j] = signbit(r.a[j]);
     const float rprev = j == 0 ? rm : r.a[j - 1];
-    nw[j] = signbit(g.fzm[k] * r.a[j] + g.fzp[k] * rprev);
+    nw[j] = signbit(fm.a[j] * r.a[j] + fp.a[j] * rprev);
   }
   V4 at = v4zero(), aw = v4zero();
   HEX_UNROLL_N(HEX_EDGE_ADV_UNROLL)
   for (int s = 0; s < n; ++s) {
-    const int cs = cells[s] * S + k0;
-    const float A = a1[s], X = g.coef3 * a3[s];
-    const float P = A + X, M = A - X;
-    const V4 th = ld4(theta + cs), wv = ld4(w + cs);
+    const int o = __ldg(off + s);
+    const float2 c = __ldg(pm + s);
+    const V4 th = ld4(theta + k0 + o), wv = ld4(w + k0 + o);
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      at.a[j] = at.a[j] + (nt[j] ? M : P) * th.a[j];
-      aw.a[j] = aw.a[j] + (nw[j] ? M : P) * wv.a[j];
+      at.a[j] = at.a[j] + (nt[j] ? c.y : c.x) * th.a[j];
+      aw.a[j] = aw.a[j] + (nw[j] ? c.y : c.x) * wv.a[j];
     }
   }
-#else
-  float ct[4], cw[4];
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    const int k = k0 + j;
-    ct[j] = g.coef3 * copysignf(1.0f, r.a[j]);
-    const float rprev = j == 0 ? rm : r.a[j - 1];
-    const float rui = g.fzm[k] * r.a[j] + g.fzp[k] * rprev;
-    cw[j] = g.coef3 * copysignf(1.0f, rui);
-  }
-  V4 at = v4zero(), aw = v4zero();
-  HEX_UNROLL_N(HEX_EDGE_ADV_UNROLL)
-  for (int s = 0; s < n; ++s) {
-    const int cs = cells[s] * S + k0;
-    const float A = a1[s], B = a3[s];
-    const V4 th = ld4(theta + cs), wv = ld4(w + cs);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      at.a[j] = at.a[j] + (A + ct[j] * B) * th.a[j];
-      aw.a[j] = aw.a[j] + (A + cw[j] * B) * wv.a[j];
-    }
-  }
-#endif
   st4m(edge_theta + e * S + k0, at, k0, 0, g.L);
   st4m(edge_w + e * S + k0, aw, k0, 1, g.L);
 }
 
-// wduz at interface j of the edge (hexcore/dynamics.py:227), from windows of
-// u (edge) and rw at both cells; d = j - k0 in [0, 4].
-__device__ __forceinline__ float wduz_win(const HexGeo& g, const Win& uw, const Win& r0, const Win& r1, int k0,
-                                          int d) {
-  const int j = k0 + d, L = g.L;
-  if (j <= 0 || j >= L) return 0.0f;
-  const float rwe = 0.5f * (r0(d) + r1(d));
-  if (j == 1 || j == L - 1) return rwe * (g.fzm[j] * uw(d) + g.fzp[j] * uw(d - 1));
-  return flux3f(uw(d - 2), uw(d - 1), uw(d), uw(d + 1), rwe, 1.0f);
+// Third-order fluxes (hexcore/dynamics.py:71, hexcore/transport.py:440) at
+// the interfaces k0 .. k0+4 of a window q with the velocities vel:
+// vel (7 (q0 + qm1) - (qp1 + qm2)) / 12 + coef |vel| ((qp1 - qm2) - 3 (q0 - qm1)) / 12,
+// every interface alike; the caller replaces those at a column's ends.
+__device__ __forceinline__ void flux3_chunk(const Win& q, const float (&vel)[5], float coef, float (&out)[5]) {
+  float x[5], y[5];
+#pragma unroll
+  for (int d = 0; d < 5; ++d) {
+    x[d] = vel[d] * (7.0f * (q(d) + q(d - 1)) - (q(d + 1) + q(d - 2)));
+    y[d] = coef * fabsf(vel[d]) * ((q(d + 1) - q(d - 2)) - 3.0f * (q(d) - q(d - 1)));
+  }
+  div12_sum(x, y, out);
+}
+// A column's ends in a chunk's interfaces k0 .. k0+4: interface 1 and L-1
+// take `edge(d)`, interfaces 0 and L and beyond are zero.  Only the chunks
+// holding those interfaces enter the branches.
+template <class F>
+__device__ __forceinline__ void column_ends(int k0, int L, float (&f)[5], F edge) {
+  if (k0 == 0) {
+    f[0] = 0.0f;
+    f[1] = edge(1);
+  }
+  const int top = L - 1 - k0;
+  if (top <= 4) {
+#pragma unroll
+    for (int d = 0; d < 5; ++d) {
+      if (d == top) f[d] = edge(d);
+      if (d > top) f[d] = 0.0f;
+    }
+  }
 }
 
 // tend_ru: vertical transport + hexcore/dynamics_v841.py:121 momentum + saved Euler.
@@ -534,25 +548,29 @@ __global__ void __launch_bounds__(256, HEX_TEND_U_MIN_BLOCKS) kv_tend_u(HexGeo g
                           float* __restrict__ ru_avg0) {
   HEX_VEC_PARALLEL(g.nE)
   const int e = ent, S = g.S;
-  const int c0 = g.coe[2 * e], c1 = g.coe[2 * e + 1];
-  const Win uw = win(u + e * S, k0, S);
-  const Win r0 = win(rw + c0 * S, k0, S), r1 = win(rw + c1 * S, k0, S);
-  float wd[5];
-#pragma unroll
-  for (int d = 0; d < 5; ++d) wd[d] = wduz_win(g, uw, r0, r1, k0, d);
+  const int2 ends = __ldg(g.ends + e);
   const int n = g.neoe[e];
   const V4 pve = ld4(pv_edge + e * S + k0);
   V4 q = v4zero();
-  HEX_UNROLL_N(HEX_TEND_U_UNROLL)
-  for (int s = 0; s < n; ++s) {
-    const int nb = g.eoe[e * g.maxE2 + s];
-    const float w = g.weights[e * g.maxE2 + s];
-    const V4 un = ld4(u + nb * S + k0), pn = ld4(pv_edge + nb * S + k0);
+  const int4* nbr = g.nbr + (size_t)e * g.nbrW;
+  const auto coriolis = [&](const V4& un, const V4& pn, float w) {
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const float work_pv = 0.5f * (pve.a[j] + pn.a[j]);
       q.a[j] = q.a[j] + w * un.a[j] * work_pv;
     }
+  };
+  HEX_UNROLL_N(HEX_TEND_U_UNROLL)
+  for (int s = 0; s + 1 < n; s += 2) {
+    const int4 r = __ldg(nbr + (s >> 1));
+    const V4 ua = ld4(u + k0 + r.x), pa = ld4(pv_edge + k0 + r.x);
+    const V4 ub = ld4(u + k0 + r.z), pb = ld4(pv_edge + k0 + r.z);
+    coriolis(ua, pa, fbits(r.y));
+    coriolis(ub, pb, fbits(r.w));
+  }
+  if (n & 1) {
+    const int4 r = __ldg(nbr + (n >> 1));
+    coriolis(ld4(u + k0 + r.x), ld4(pv_edge + k0 + r.x), fbits(r.y));
   }
   // Perturbation-Coriolis subtraction.  With all-zero reference winds every
   // subtracted term is a signed zero, and q - (+-0) == q bit for bit unless
@@ -564,7 +582,6 @@ __global__ void __launch_bounds__(256, HEX_TEND_U_MIN_BLOCKS) kv_tend_u(HexGeo g
   for (int j = 0; j < 4; ++j) need = need || (k0 + j < g.L && !(fabsf(q.a[j]) > 0.0f));
   if (need) {
     const float fe = g.f_edge[e];
-    HEX_UNROLL_N(HEX_TEND_U_UNROLL)
     for (int s = 0; s < n; ++s) {
       const int nb = g.eoe[e * g.maxE2 + s];
       const float w = g.weights[e * g.maxE2 + s];
@@ -577,16 +594,26 @@ __global__ void __launch_bounds__(256, HEX_TEND_U_MIN_BLOCKS) kv_tend_u(HexGeo g
       }
     }
   }
-  const V4 rh0 = ld4(rho + c0 * S + k0), rh1 = ld4(rho + c1 * S + k0);
-  const V4 ke0 = ld4(ke + c0 * S + k0), ke1 = ld4(ke + c1 * S + k0);
-  const V4 hd0 = ld4(hdiv + c0 * S + k0), hd1 = ld4(hdiv + c1 * S + k0);
+  const Win uw = win<2, 2>(u + e * S, k0, S);
+  const Win r0 = win<0, 1>(rw + ends.x, k0, S), r1 = win<0, 1>(rw + ends.y, k0, S);
+  // the vertical transport's flux at interface j (hexcore/dynamics.py:227)
+  float wd[5], rwe[5];
+#pragma unroll
+  for (int d = 0; d < 5; ++d) rwe[d] = 0.5f * (r0(d) + r1(d));
+  flux3_chunk(uw, rwe, 1.0f, wd);
+  column_ends(k0, g.L, wd, [&](int d) { return rwe[d] * (g.fzm[k0 + d] * uw(d) + g.fzp[k0 + d] * uw(d - 1)); });
+  const int i0 = ends.x + k0, i1 = ends.y + k0;
+  const V4 rh0 = ld4(rho + i0), rh1 = ld4(rho + i1);
+  const V4 ke0 = ld4(ke + i0), ke1 = ld4(ke + i1);
+  const V4 hd0 = ld4(hdiv + i0), hd1 = ld4(hdiv + i1);
+  const V4 rz = ld4(g.rdzw + k0);
   const V4 eu = ld4(euler_ru + e * S + k0);
   const float idc = g.inv_dc[e];
   V4 out;
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
     const int k = k0 + j;
-    const float tv = -g.rdzw[k] * (wd[j + 1] - wd[j]);
+    const float tv = -rz.a[j] * (wd[j + 1] - wd[j]);
     const float rho_edge = 0.5f * (rh0.a[j] + rh1.a[j]);
     float horizontal = rho_edge * (q.a[j] - (ke1.a[j] - ke0.a[j]) * idc);
     horizontal = tv + horizontal;
@@ -617,31 +644,9 @@ __global__ void __launch_bounds__(256, HEX_TEND_U_MIN_BLOCKS) kv_tend_u(HexGeo g
   }
 }
 
-// theta vertical flux at interface j = k0 + d (hexcore/driver.py:1048-1076).
-__device__ __forceinline__ float vflux_theta_win(const HexGeo& g, const Win& th, const Win& ths, const Win& rw,
-                                                 const Win& rws, int k0, int d) {
-  const int j = k0 + d, L = g.L;
-  if (j <= 0 || j >= L) return 0.0f;
-  if (j == 1) {
-    const float vf = rw(d) * (g.fzm[j] * th(d) + g.fzp[j] * th(d - 1));
-    return vf + (rws(d) - rw(d)) * (g.fzm[j] * ths(d) + g.fzp[j] * ths(d - 1));
-  }
-  if (j == L - 1) return rws(d) * (g.fzm[j] * th(d) + g.fzp[j] * th(d - 1));
-  const float vf = flux3f(th(d - 2), th(d - 1), th(d), th(d + 1), rw(d), g.coef3);
-  return vf + (rws(d) - rw(d)) * (g.fzm[j] * ths(d) + g.fzp[j] * ths(d - 1));
-}
-
-// w vertical flux at interface j = k0 + d (hexcore/driver.py:1176-1200).
-__device__ __forceinline__ float vflux_w_win(const HexGeo& g, const Win& w, const Win& rw, int k0, int d) {
-  const int j = k0 + d, L = g.L;
-  if (j <= 0 || j >= L) return 0.0f;
-  if (j == 1 || j == L - 1) return 0.25f * (rw(d) + rw(d - 1)) * (w(d) + w(d - 1));
-  return flux3f(w(d - 2), w(d - 1), w(d), w(d + 1), 0.5f * (rw(d) + rw(d - 1)), 1.0f);
-}
-
 // tend_rt (hexcore/driver.py:933), tend_rw (:1081) + Euler w, then
 // hexcore/acoustic.py:246 convert_w_tendency_to_omega.
-__global__ void HEX_VEC_BOUNDS kv_tend_cell(HexGeo g, const float* __restrict__ ru, const float* __restrict__ ru_s,
+__global__ void __launch_bounds__(256, 3) kv_tend_cell(HexGeo g, const float* __restrict__ ru, const float* __restrict__ ru_s,
                              const float* __restrict__ rw, const float* __restrict__ rws,
                              const float* __restrict__ theta, const float* __restrict__ theta_s,
                              const float* __restrict__ w, const float* __restrict__ edge_theta,
@@ -653,34 +658,35 @@ __global__ void HEX_VEC_BOUNDS kv_tend_cell(HexGeo g, const float* __restrict__ 
   const int c = ent, S = g.S, L = g.L;
   const int n = g.deg[c];
   const float ia = g.inv_area[c];
-  const int* eoc = g.eoc + c * g.maxE;
-  const float* cs = g.csign + c * g.maxE;
+  const int2* slots = g.slot + c * g.maxE;
+  const V4 fm = ld4(g.fzm + k0), fp = ld4(g.fzp + k0);
   // horizontal parts: rho-theta flux divergence, RK>1 correction, w flux
   V4 res = v4zero(), hres = v4zero();
   HEX_GATHER
   for (int s = 0; s < n; ++s) {
-    const int e = eoc[s];
-    const float sg = cs[s];
-    const V4 r = ld4(ru + e * S + k0), et = ld4(edge_theta + e * S + k0), ew = ld4(edge_w + e * S + k0);
-    const float rm = k0 > 0 ? ru[e * S + k0 - 1] : 0.0f;
+    const int sl = __ldg(&slots[s].x), eo = slot_edge(sl);
+    const float sg = slot_sign(sl);
+    const V4 r = ld4(ru + k0 + eo), et = ld4(edge_theta + k0 + eo), ew = ld4(edge_w + k0 + eo);
+    const float rm = k0 > 0 ? (ru + k0 - 1)[eo] : 0.0f;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      const int k = k0 + j;
-      res.a[j] = res.a[j] - sg * r.a[j] * et.a[j];
+      // sg is +-1: sg x y rounds once, and adding or subtracting it in one
+      // fused operation rounds as the separate sum does
+      res.a[j] = fma_sign(-sg, r.a[j] * et.a[j], res.a[j]);
       const float rprev = j == 0 ? rm : r.a[j - 1];
-      const float rui = g.fzm[k] * r.a[j] + g.fzp[k] * rprev;
-      hres.a[j] = hres.a[j] - sg * rui * ew.a[j];
+      const float rui = fm.a[j] * r.a[j] + fp.a[j] * rprev;
+      hres.a[j] = fma_sign(-sg, rui * ew.a[j], hres.a[j]);
     }
   }
   if (rk_step > 1) {
     const V4 tc = ld4(theta_s + c * S + k0);
     HEX_GATHER
     for (int s = 0; s < n; ++s) {
-      const int e = eoc[s];
-      const int e0 = g.coe[2 * e], e1 = g.coe[2 * e + 1];
-      const float dvs = cs[s] * g.dv[e];
-      const V4 r = ld4(ru + e * S + k0), rs = ld4(ru_s + e * S + k0);
-      const V4 tn = ld4(theta_s + (e0 == c ? e1 : e0) * S + k0);
+      const int2 sl = __ldg(slots + s);
+      const int eo = slot_edge(sl.x);
+      const float dvs = __ldg(g.sdv + c * g.maxE + s);
+      const V4 r = ld4(ru + k0 + eo), rs = ld4(ru_s + k0 + eo);
+      const V4 tn = ld4(theta_s + k0 + sl.y);
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         // theta_s[e1] + theta_s[e0] with this cell as one operand (IEEE
@@ -690,53 +696,62 @@ __global__ void HEX_VEC_BOUNDS kv_tend_cell(HexGeo g, const float* __restrict__ 
       }
     }
   }
-  const Win th = win(theta + c * S, k0, S), ths = win(theta_s + c * S, k0, S);
-  const Win rww = win(rw + c * S, k0, S), rwsw = win(rws + c * S, k0, S);
-  const Win ww = win(w + c * S, k0, S), zzw = win(g.zz + c * S, k0, S);
+  const Win th = win<2, 2>(theta + c * S, k0, S), ths = win<1, 1>(theta_s + c * S, k0, S);
+  const Win rww = win<1, 1>(rw + c * S, k0, S), rwsw = win<0, 1>(rws + c * S, k0, S);
+  const Win ww = win<2, 2>(w + c * S, k0, S), zzw = win<1, 0>(g.zz + c * S, k0, S);
   const V4 er = ld4(euler_rw + c * S + k0);
-  float vt[5], vw[5];
+  // theta flux at the interfaces (hexcore/driver.py:1048-1076)
+  float vt[5], vw[5], vel[5];
+#pragma unroll
+  for (int d = 0; d < 5; ++d) vel[d] = rww(d);
+  flux3_chunk(th, vel, g.coef3, vt);
+  const float fm5[5] = {fm.a[0], fm.a[1], fm.a[2], fm.a[3], k0 + 4 < S ? g.fzm[k0 + 4] : 0.0f};
+  const float fp5[5] = {fp.a[0], fp.a[1], fp.a[2], fp.a[3], k0 + 4 < S ? g.fzp[k0 + 4] : 0.0f};
+  column_ends(k0, L, vt, [&](int d) {
+    return (k0 + d == 1 ? rww(d) : rwsw(d)) * (fm5[d] * th(d) + fp5[d] * th(d - 1));
+  });
 #pragma unroll
   for (int d = 0; d < 5; ++d) {
-    vt[d] = vflux_theta_win(g, th, ths, rww, rwsw, k0, d);
-    vw[d] = vflux_w_win(g, ww, rww, k0, d);
+    const float with = vt[d] + (rwsw(d) - rww(d)) * (fm5[d] * ths(d) + fp5[d] * ths(d - 1));
+    vt[d] = k0 + d >= 1 && k0 + d < L - 1 ? with : vt[d];
   }
+  // w flux (hexcore/driver.py:1176-1200)
+#pragma unroll
+  for (int d = 0; d < 5; ++d) vel[d] = 0.5f * (rww(d) + rww(d - 1));
+  flux3_chunk(ww, vel, 1.0f, vw);
+  column_ends(k0, L, vw, [&](int d) { return 0.25f * (rww(d) + rww(d - 1)) * (ww(d) + ww(d - 1)); });
+  const V4 rz = ld4(g.rdzw + k0), rzu = ld4(g.rdzu + k0);
   V4 trt, trw;
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
-    const int k = k0 + j;
-    trt.a[j] = res.a[j] * ia - g.rdzw[k] * (vt[j + 1] - vt[j]);
-    if (k >= 1 && k < L) {
-      const float rsw = hres.a[j] * ia - g.rdzu[k] * (vw[j + 1] - vw[j]);
-      trw.a[j] = rsw + er.a[j];
-    } else {
-      trw.a[j] = 0.0f + er.a[j];
-    }
+    trt.a[j] = res.a[j] * ia - rz.a[j] * (vt[j + 1] - vt[j]);
+    const float rsw = hres.a[j] * ia - rzu.a[j] * (vw[j + 1] - vw[j]);
+    trw.a[j] = rsw + er.a[j];
   }
   // omega conversion (interfaces 1..L-1)
   HEX_GATHER
   for (int s = 0; s < n; ++s) {
-    const int e = eoc[s];
-    const float sg = cs[s];
-    const V4 t = ld4(tend_ru + e * S + k0);
-    const float tm = k0 > 0 ? tend_ru[e * S + k0 - 1] : 0.0f;
+    const int sl = __ldg(&slots[s].x), eo = slot_edge(sl);
+    const float sg = slot_sign(sl);
+    const V4 t = ld4(tend_ru + k0 + eo);
+    const float tm = k0 > 0 ? (tend_ru + k0 - 1)[eo] : 0.0f;
     const int zi = (c * g.maxE + s) * S + k0;
     const V4 zb = ld4(g.zb + zi), zb3 = ld4(g.zb3 + zi);
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      const int k = k0 + j;
-      if (k >= 1 && k < L) {
-        const float tprev = j == 0 ? tm : t.a[j - 1];
-        const float flux = sg * (g.fzm[k] * t.a[j] + g.fzp[k] * tprev);
-        const float up = copysignf(1.0f, t.a[j]);
-        trw.a[j] = trw.a[j] - (zb.a[j] + up * zb3.a[j]) * flux;
-      }
+      const float tprev = j == 0 ? tm : t.a[j - 1];
+      const float flux = fm.a[j] * t.a[j] + fp.a[j] * tprev;
+      const float zt = fma_sign(copysignf(1.0f, t.a[j]), zb3.a[j], zb.a[j]);
+      trw.a[j] = fma_sign(-sg, zt * flux, trw.a[j]);
     }
   }
+  // levels 0 and L hold 0 + the saved Euler term (every level ran the sums
+  // above: no branch splits a warp between its columns' ends and insides)
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
     const int k = k0 + j;
-    if (k >= 1 && k < L) trw.a[j] = trw.a[j] * (g.fzm[k] * zzw(j) + g.fzp[k] * zzw(j - 1));
-    if (k > L) trw.a[j] = 0.0f;
+    const float in = trw.a[j] * (fm.a[j] * zzw(j) + fp.a[j] * zzw(j - 1));
+    trw.a[j] = k >= 1 && k < L ? in : (k > L ? 0.0f : 0.0f + er.a[j]);
   }
   if (phys.on) {
     // physics hand-off (hexcore/cuda_driver.py:4459-4494): at RK stage 3 the
@@ -827,8 +842,10 @@ __global__ void HEX_VEC_BOUNDS kv_mix_edge2(HexGeo g, const float* __restrict__ 
                              float* __restrict__ mix_u) {
   HEX_VEC_PARALLEL(g.nE)
   const int e = ent, S = g.S;
-  const int i0 = g.coe[2 * e] * S + k0, i1 = g.coe[2 * e + 1] * S + k0;
-  const int j0 = g.voe[2 * e] * S + k0, j1 = g.voe[2 * e + 1] * S + k0;
+  const int2 ends = __ldg(g.ends + e);
+  const int i0 = ends.x + k0, i1 = ends.y + k0;
+  const int2 ve = __ldg(g.vends + e);
+  const int j0 = ve.x + k0, j1 = ve.y + k0;
   const V4 d0 = ld4(div + i0), d1 = ld4(div + i1), z0 = ld4(vort + j0), z1 = ld4(vort + j1);
   const V4 k0v = ld4(kdiff + i0), k1v = ld4(kdiff + i1), r0 = ld4(rho + i0), r1 = ld4(rho + i1);
   const V4 eu = ld4(euler_ru + e * S + k0);
@@ -938,8 +955,10 @@ __global__ void HEX_VEC_BOUNDS kv_mix_edge4(HexGeo g, const float* __restrict__ 
                              float* __restrict__ mix_u) {
   HEX_VEC_PARALLEL(g.nE)
   const int e = ent, S = g.S;
-  const int i0 = g.coe[2 * e] * S + k0, i1 = g.coe[2 * e + 1] * S + k0;
-  const int j0 = g.voe[2 * e] * S + k0, j1 = g.voe[2 * e + 1] * S + k0;
+  const int2 ends = __ldg(g.ends + e);
+  const int i0 = ends.x + k0, i1 = ends.y + k0;
+  const int2 ve = __ldg(g.vends + e);
+  const int j0 = ve.x + k0, j1 = ve.y + k0;
   const V4 d0 = ld4(delsq_div + i0), d1 = ld4(delsq_div + i1);
   const V4 z0 = ld4(delsq_vort + j0), z1 = ld4(delsq_vort + j1);
   const V4 r0 = ld4(rho + i0), r1 = ld4(rho + i1);
@@ -1014,7 +1033,8 @@ __global__ void HEX_VEC_BOUNDS kv_ac_edge(HexGeo g, int mode, int old_is_zero, f
     st4m(ru_avg + jj, r, k0, 0, g.L);
     return;
   }
-  const int i0 = g.coe[2 * e] * S + k0, i1 = g.coe[2 * e + 1] * S + k0;
+  const int2 ends = __ldg(g.ends + e);
+  const int i0 = ends.x + k0, i1 = ends.y + k0;
   // smdiv_base * (1/dts), the damping coefficient of the edge's mesh
   const float damp_coef = g.smdiv_edge[e] * inv_dts;
   V4 r = ld4rw(ru_p + jj);
@@ -1026,7 +1046,7 @@ __global__ void HEX_VEC_BOUNDS kv_ac_edge(HexGeo g, int mode, int old_is_zero, f
   for (int j = 0; j < 4; ++j) {
     const float d0 = n0.a[j] - o0.a[j];
     const float d1 = n1.a[j] - o1.a[j];
-    r.a[j] = r.a[j] + damp_coef * (d0 - d1) * (1.0f - 0.0f) / (t0.a[j] + t1.a[j]);
+    r.a[j] = r.a[j] + damp_coef * (d0 - d1) * (1.0f - 0.0f) / inside(t0.a[j] + t1.a[j], k0 + j, g.L);
   }
   if (mode == 1) {
     const V4 z0 = ld4(g.zz + i0), z1 = ld4(g.zz + i1), x0 = ld4(exner_s + i0), x1 = ld4(exner_s + i1);
@@ -1036,7 +1056,7 @@ __global__ void HEX_VEC_BOUNDS kv_ac_edge(HexGeo g, int mode, int old_is_zero, f
     const float idc = g.inv_dc[e];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      float pg = (n1.a[j] - n0.a[j]) * idc / (0.5f * (z1.a[j] + z0.a[j]));
+      float pg = (n1.a[j] - n0.a[j]) * idc / inside(0.5f * (z1.a[j] + z0.a[j]), k0 + j, g.L);
       pg = cq.a[j] * 0.5f * g.c2 * (x0.a[j] + x1.a[j]) * pg;
       pg = pg + 0.5f * zx.a[j] * g.g * (p0.a[j] + p1.a[j]);
       r.a[j] = r.a[j] + dts * (t.a[j] - pg);
@@ -1064,7 +1084,8 @@ __global__ void HEX_VEC_BOUNDS kv_recover_edge(HexGeo g, const float* __restrict
   HEX_VEC_PARALLEL(g.nE)
   const int e = ent, S = g.S;
   const int jj = e * S + k0;
-  const int i0 = g.coe[2 * e] * S + k0, i1 = g.coe[2 * e + 1] * S + k0;
+  const int2 ends = __ldg(g.ends + e);
+  const int i0 = ends.x + k0, i1 = ends.y + k0;
   V4 rp = ld4rw(ru_p + jj);
   if (damp) {
     const float damp_coef = g.smdiv_edge[e] * inv_dts;
@@ -1076,7 +1097,7 @@ __global__ void HEX_VEC_BOUNDS kv_recover_edge(HexGeo g, const float* __restrict
     for (int j = 0; j < 4; ++j) {
       const float d0 = n0.a[j] - o0.a[j];
       const float d1 = n1.a[j] - o1.a[j];
-      rp.a[j] = rp.a[j] + damp_coef * (d0 - d1) * (1.0f - 0.0f) / (t0.a[j] + t1.a[j]);
+      rp.a[j] = rp.a[j] + damp_coef * (d0 - d1) * (1.0f - 0.0f) / inside(t0.a[j] + t1.a[j], k0 + j, g.L);
     }
     st4m(ru_p + jj, rp, k0, 0, g.L);
   }
@@ -1089,7 +1110,7 @@ __global__ void HEX_VEC_BOUNDS kv_recover_edge(HexGeo g, const float* __restrict
     const float rho0 = a0.a[j] + b0.a[j] + c0.a[j];
     const float rho1 = a1.a[j] + b1.a[j] + c1.a[j];
     ru.a[j] = rs.a[j] + rp.a[j];
-    uo.a[j] = 2.0f * ru.a[j] / (rho0 + rho1);
+    uo.a[j] = 2.0f * ru.a[j] / inside(rho0 + rho1, k0 + j, g.L);
   }
   st4m(ru_out + jj, ru, k0, 0, g.L);
   st4m(u_out + jj, uo, k0, 0, g.L);
@@ -1121,11 +1142,12 @@ __global__ void HEX_VEC_BOUNDS kv_recover_cell(HexGeo g, int stage3, const float
   HEX_VEC_PARALLEL(g.nC)
   const int c = ent, S = g.S, L = g.L;
   const int ii = c * S + k0;
-  // candidate density on the window k0-4 .. k0+7 (recomputed, not read back)
-  const Win rpw = win(rp_s + c * S, k0, S), ppw = win(rho_pp + c * S, k0, S), rbw = win(g.rho_base + c * S, k0, S);
-  float rho_w[12];
+  // candidate density at the levels k0-1 .. k0+3 (recomputed, not read back)
+  const Win rpw = win<1, 0>(rp_s + c * S, k0, S), ppw = win<1, 0>(rho_pp + c * S, k0, S);
+  const Win rbw = win<1, 0>(g.rho_base + c * S, k0, S);
+  float rho_w[5];
 #pragma unroll
-  for (int d = -4; d < 8; ++d) rho_w[d + 4] = rpw(d) + ppw(d) + rbw(d);
+  for (int d = -1; d < 4; ++d) rho_w[d + 1] = rpw(d) + ppw(d) + rbw(d);
   {
     const V4 tp = ld4(rtp_s + ii), tq = ld4(rtpp + ii), tb = ld4(g.rtheta_base + ii);
     V4 rho, rt, rp, rtp, th;
@@ -1136,7 +1158,7 @@ __global__ void HEX_VEC_BOUNDS kv_recover_cell(HexGeo g, int stage3, const float
       rtp.a[j] = tp.a[j] + tq.a[j];
       rho.a[j] = rp.a[j] + rbw(j);
       rt.a[j] = rtp.a[j] + tb.a[j];
-      th.a[j] = rt.a[j] / rho.a[j];
+      th.a[j] = rt.a[j] / inside(rho.a[j], k0 + j, L);
       if (k0 + j < L && (!(rho.a[j] > 0.0f) || !(rt.a[j] > 0.0f))) bad = true;
     }
     if (bad) atomicOr(flag, HEX_FLAG_DENSITY);
@@ -1176,28 +1198,29 @@ __global__ void HEX_VEC_BOUNDS kv_recover_cell(HexGeo g, int stage3, const float
   }
   st4m(out.rho_w + ii, rwv, k0, 0, g.L + 1);
   const int n = g.deg[c];
-  const Win zzw = win(g.zz + c * S, k0, S);
+  const Win zzw = win<1, 0>(g.zz + c * S, k0, S);
   float acc[4];
   bool bottom = k0 == 0;
   float bacc = 0.0f;
+  const V4 fm = ld4(g.fzm + k0), fp = ld4(g.fzp + k0);
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
     const int k = k0 + j;
-    acc[j] = 0.0f;
-    if (k >= 1 && k < L) acc[j] = rwv.a[j] / (g.fzm[k] * zzw(j) + g.fzp[k] * zzw(j - 1));
+    // (outside the inner interfaces: 0 / 1, not used)
+    const float den = fm.a[j] * zzw(j) + fp.a[j] * zzw(j - 1);
+    acc[j] = rwv.a[j] / (k >= 1 && k < L ? den : 1.0f);
   }
   // the next stage's mass-flux divergence of ru_new (mass_flux_div4, the
   // same operands in the same order) accumulates in the same edge loop
   V4 hd = v4zero();
   HEX_GATHER
   for (int s = 0; s < n; ++s) {
-    const int e = g.eoc[c * g.maxE + s];
-    const float sign = g.csign[c * g.maxE + s];
-    const V4 r = ld4(ru_new + e * S + k0);
-    const float sd = sign * g.dv[e];
+    const int sl = __ldg(&g.slot[c * g.maxE + s].x), eo = slot_edge(sl);
+    const float sign = slot_sign(sl), sd = __ldg(g.sdv + c * g.maxE + s);
+    const V4 r = ld4(ru_new + k0 + eo);
 #pragma unroll
     for (int j = 0; j < 4; ++j) hd.a[j] = hd.a[j] + sd * r.a[j];
-    const float rm = k0 > 0 ? ru_new[e * S + k0 - 1] : 0.0f;
+    const float rm = k0 > 0 ? (ru_new + k0 - 1)[eo] : 0.0f;
     const int zi = (c * g.maxE + s) * S + k0;
     const V4 zb = ld4(g.zb + zi), zb3 = ld4(g.zb3 + zi);
     if (bottom) {
@@ -1206,26 +1229,27 @@ __global__ void HEX_VEC_BOUNDS kv_recover_cell(HexGeo g, int stage3, const float
     }
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      const int k = k0 + j;
-      if (k >= 1 && k < L) {
-        const float rprev = j == 0 ? rm : r.a[j - 1];
-        const float flux = g.fzm[k] * r.a[j] + g.fzp[k] * rprev;
-        acc[j] = acc[j] + sign * (zb.a[j] + copysignf(1.0f, flux) * zb3.a[j]) * flux;
-      }
+      const float rprev = j == 0 ? rm : r.a[j - 1];
+      const float flux = fm.a[j] * r.a[j] + fp.a[j] * rprev;
+      const float zt = fma_sign(copysignf(1.0f, flux), zb3.a[j], zb.a[j]);
+      acc[j] = fma_sign(sign, zt * flux, acc[j]);
     }
   }
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
     const int k = k0 + j;
-    float wk = 0.0f;
+    // level 0 takes the bottom flux and density; interfaces past the last
+    // inner one are zero, divided by one
+    float num = acc[j], den = fm.a[j] * rho_w[j + 1] + fp.a[j] * rho_w[j];
     if (k == 0) {
-      const float bd = g.cf1 * rho_w[4] + g.cf2 * rho_w[5] + g.cf3 * rho_w[6];
-      wk = bacc / bd;
-    } else if (k < L) {
-      const float irho = g.fzm[k] * rho_w[j + 4] + g.fzp[k] * rho_w[j + 3];
-      wk = acc[j] / irho;
+      num = bacc;
+      den = g.cf1 * rho_w[1] + g.cf2 * rho_w[2] + g.cf3 * rho_w[3];
     }
-    wv.a[j] = wk;
+    if (k >= L) {
+      num = 0.0f;
+      den = 1.0f;
+    }
+    wv.a[j] = num / den;
   }
   st4m(side.w + ii, wv, k0, 0, g.L + 1);
   {
@@ -1269,33 +1293,21 @@ __global__ void __launch_bounds__(256, HEX_TR_EDGE_MIN_BLOCKS) kv_tr_edge(HexGeo
   const size_t tstride = (size_t)g.nC * S;
   const float* qg = q + (size_t)t0 * tstride + k0;
   const int n = g.n_adv[e];
-  const int* cells = g.adv_cells + (size_t)e * g.advW;
-  const float* a1 = g.adv + (size_t)e * g.advW;
-  const float* a3 = g.adv3 + (size_t)e * g.advW;
+  const int* off = g.adv_off + (size_t)e * g.advW;
+  const float2* pm = g.adv_pm + (size_t)e * g.advW;
   const V4 vel = ld4(hv + e * S + k0);
-#if HEX_PM_SELECT_TR_EDGE
-  // A + (coef3 sign(vel)) B as A + X or A - X, X = coef3 B (see kv_edge_adv)
+  // A + (coef3 sign(vel)) B is one of the record's two sums (see kv_edge_adv)
   bool neg[4];
 #pragma unroll
   for (int j = 0; j < 4; ++j) neg[j] = signbit(vel.a[j]);
 #define HEX_TR_WEIGHTS(s_)                                   \
-  const float A = a1[s_], X = g.coef3 * a3[s_];              \
-  const float P = A + X, M = A - X;                          \
+  const float* qc = qg + __ldg(off + (s_));                  \
+  const float2 c = __ldg(pm + (s_));                         \
   float w[4];                                                \
-  _Pragma("unroll") for (int j = 0; j < 4; ++j) w[j] = neg[j] ? M : P;
-#else
-  float cs[4];
-#pragma unroll
-  for (int j = 0; j < 4; ++j) cs[j] = g.coef3 * copysignf(1.0f, vel.a[j]);
-#define HEX_TR_WEIGHTS(s_)                                   \
-  const float A = a1[s_], B = a3[s_];                        \
-  float w[4];                                                \
-  _Pragma("unroll") for (int j = 0; j < 4; ++j) w[j] = A + cs[j] * B;
-#endif
+  _Pragma("unroll") for (int j = 0; j < 4; ++j) w[j] = neg[j] ? c.y : c.x;
   V4 res[TG];
   if (mono && n == 10) {
     {
-      const float* qc = qg + cells[0] * S;
       HEX_TR_WEIGHTS(0)
 #pragma unroll
       for (int t = 0; t < TG; ++t)
@@ -1307,7 +1319,6 @@ __global__ void __launch_bounds__(256, HEX_TR_EDGE_MIN_BLOCKS) kv_tr_edge(HexGeo
     }
     HEX_UNROLL_N(HEX_TR_EDGE_UNROLL)
     for (int s = 1; s < 10; ++s) {
-      const float* qc = qg + cells[s] * S;
       HEX_TR_WEIGHTS(s)
 #pragma unroll
       for (int t = 0; t < TG; ++t)
@@ -1326,7 +1337,6 @@ __global__ void __launch_bounds__(256, HEX_TR_EDGE_MIN_BLOCKS) kv_tr_edge(HexGeo
     for (int t = 0; t < TG; ++t) res[t] = v4zero();
     HEX_UNROLL_N(HEX_TR_EDGE_UNROLL)
     for (int s = 0; s < n; ++s) {
-      const float* qc = qg + cells[s] * S;
       HEX_TR_WEIGHTS(s)
 #pragma unroll
       for (int j = 0; j < 4; ++j)
@@ -1346,15 +1356,11 @@ __global__ void __launch_bounds__(256, HEX_TR_EDGE_MIN_BLOCKS) kv_tr_edge(HexGeo
 #undef HEX_TR_WEIGHTS
 }
 
-// transport vertical flux at interface j = k0 + d (hexcore/transport.py:1389).
-__device__ __forceinline__ float tr_vflux_win(const HexGeo& g, const Win& q, const Win& ww, int k0, int d) {
-  const int j = k0 + d, L = g.L;
-  if (j <= 0 || j >= L) return 0.0f;
-  if (j == 1 || j == L - 1) return ww(d) * (g.fzm[j] * q(d) + g.fzp[j] * q(d - 1));
-  const float vel = ww(d);
-  const float base = vel * (7.0f * (q(d) + q(d - 1)) - (q(d + 1) + q(d - 2))) / 12.0f;
-  const float corr = g.coef3 * fabsf(vel) * ((q(d + 1) - q(d - 2)) - 3.0f * (q(d) - q(d - 1))) / 12.0f;
-  return base + corr;
+// transport vertical fluxes at the interfaces k0 .. k0+4 (hexcore/transport.py:1389).
+__device__ __forceinline__ void tr_vflux_chunk(const HexGeo& g, const Win& q, const Win& ww, int k0, float (&f)[5]) {
+  const float vel[5] = {ww(0), ww(1), ww(2), ww(3), ww(4)};
+  flux3_chunk(q, vel, g.coef3, f);
+  column_ends(k0, g.L, f, [&](int d) { return ww(d) * (g.fzm[k0 + d] * q(d) + g.fzp[k0 + d] * q(d - 1)); });
 }
 
 // hexcore/transport.py:1649 advance_scalars (RK1/RK2 of split transport).
@@ -1372,26 +1378,26 @@ __global__ void __launch_bounds__(256, HEX_TR_STD_MIN_BLOCKS) kv_tr_std(HexGeo g
   V4 t = v4zero();
   HEX_GATHER
   for (int s = 0; s < n; ++s) {
-    const int e = g.eoc[c * g.maxE + s];
-    const float ts = -g.csign[c * g.maxE + s];
-    const V4 h = ld4(hv + e * S + k0), x = ld4(ev + e * S + k0);
+    const int sl = __ldg(&g.slot[c * g.maxE + s].x), eo = slot_edge(sl);
+    const float ts = -slot_sign(sl);
+    const V4 h = ld4(hv + k0 + eo), x = ld4(ev + k0 + eo);
 #pragma unroll
-    for (int j = 0; j < 4; ++j) t.a[j] = t.a[j] + ts * h.a[j] * x.a[j];
+    for (int j = 0; j < 4; ++j) t.a[j] = fma_sign(ts, h.a[j] * x.a[j], t.a[j]);
   }
   const float ia = g.inv_area[c];
-  const Win qw = win(q_stage + toff + c * S, k0, S), www = win(ww + c * S, k0, S);
+  const Win qw = win<2, 2>(q_stage + toff + c * S, k0, S), www = win<0, 1>(ww + c * S, k0, S);
   const V4 ro = ld4(rho_old + ii), rn = ld4(rho_new + ii), qo = ld4(q_old + toff + ii);
   float vf[5];
-#pragma unroll
-  for (int d = 0; d < 5; ++d) vf[d] = tr_vflux_win(g, qw, www, k0, d);
+  tr_vflux_chunk(g, qw, www, k0, vf);
+  const V4 rz = ld4(g.rdzw + k0);
   V4 out;
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
     const int k = k0 + j;
     const float tt = t.a[j] * ia + 0.0f;
     const float target = (1.0f - wn) * ro.a[j] + wn * rn.a[j];
-    const float num = qo.a[j] * ro.a[j] + step * (tt - g.rdzw[k] * (vf[j + 1] - vf[j]));
-    out.a[j] = num * (1.0f / target);
+    const float num = qo.a[j] * ro.a[j] + step * (tt - rz.a[j] * (vf[j + 1] - vf[j]));
+    out.a[j] = num * (1.0f / inside(target, k, g.L));
   }
   st4m(q_out + toff + ii, out, k0, 0, g.L);
 }
@@ -1408,14 +1414,12 @@ __global__ void HEX_VEC_BOUNDS kv_fct_target(HexGeo g, float step, const float* 
   V4 hd = v4zero();
   HEX_GATHER
   for (int s = 0; s < n; ++s) {
-    const int e = g.eoc[c * g.maxE + s];
-    const float ts = -g.csign[c * g.maxE + s];
-    const float dv = g.dv[e];
-    const V4 h = ld4(hv + e * S + k0);
+    const float tdv = -__ldg(g.sdv + c * g.maxE + s);  // (ts h) dv = h (ts dv), ts = -csign exact
+    const V4 h = ld4(hv + k0 + __ldg(g.eslot + c * g.maxE + s).x);
 #pragma unroll
-    for (int j = 0; j < 4; ++j) hd.a[j] = hd.a[j] + ts * h.a[j] * dv * ia;
+    for (int j = 0; j < 4; ++j) hd.a[j] = hd.a[j] + h.a[j] * tdv * ia;
   }
-  const Win www = win(ww + c * S, k0, S);
+  const Win www = win<0, 1>(ww + c * S, k0, S);
   const V4 ro = ld4(rho_old + ii);
   V4 td;
   bool bad = false;
@@ -1433,14 +1437,6 @@ __global__ void HEX_VEC_BOUNDS kv_fct_target(HexGeo g, float step, const float* 
 __device__ __forceinline__ float fct_fcol_win(float step, const Win& o, const Win& ww, int d) {
   return step * (pos0(ww(d)) * (o(d - 1) + 0.0f) + neg0(ww(d)) * (o(d) + 0.0f));
 }
-__device__ __forceinline__ float fct_vres_win(const HexGeo& g, float step, const Win& q, const Win& o,
-                                              const Win& ww, int k0, int d) {
-  const float h = step * tr_vflux_win(g, q, ww, k0, d);
-  const int j = k0 + d;
-  if (j <= 0 || j >= g.L) return h;
-  return h - fct_fcol_win(step, o, ww, d);
-}
-
 // hexcore/transport.py:1919-2118 (v8.4.1 order): bounds, low-order mass,
 // incoming/outgoing antidiffusive totals and the scale factors.
 // ACROSS: cellsOnCell[c][s] is the cell across edgesOnCell[c][s] for every
@@ -1461,7 +1457,8 @@ __global__ void HEX_VEC_BOUNDS kv_fct_cell1(HexGeo g, int nT, float step, const 
   const size_t toff = (size_t)tr * g.nC * S;
   const float* ot = q_old + toff;
   const float* he = high_e + (size_t)tr * g.nE * S;
-  const Win ow = win(ot + c * S, k0, S), qw = win(q_stage + toff + c * S, k0, S), www = win(ww + c * S, k0, S);
+  const Win ow = win<1, 1>(ot + c * S, k0, S), qw = win<2, 2>(q_stage + toff + c * S, k0, S);
+  const Win www = win<0, 1>(ww + c * S, k0, S);
   float mn[4], mx[4];
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
@@ -1484,10 +1481,16 @@ __global__ void HEX_VEC_BOUNDS kv_fct_cell1(HexGeo g, int nT, float step, const 
       }
     }
   }
-  const V4 ro = ld4(rho_old + ii), td = ld4(target + ii);
+  const V4 ro = ld4(rho_old + ii), td = ld4(target + ii), rz = ld4(g.rdzw + k0);
   float mass[4], s_in[4], s_out[4], vr[5];
+  float fc[5];  // the low-order upwind flux at the inner interfaces
+  tr_vflux_chunk(g, qw, www, k0, vr);
 #pragma unroll
-  for (int d = 0; d < 5; ++d) vr[d] = fct_vres_win(g, step, qw, ow, www, k0, d);
+  for (int d = 0; d < 5; ++d) {
+    fc[d] = fct_fcol_win(step, ow, www, d);
+    const float h = step * vr[d];
+    vr[d] = k0 + d >= 1 && k0 + d < L ? h - fc[d] : h;
+  }
   // interfaces k0..k0+3 for the limited update (every interface of the
   // column is some thread's k0 + d, d < 4)
   st4(vres_out + toff + ii, V4{{vr[0], vr[1], vr[2], vr[3]}});
@@ -1495,24 +1498,26 @@ __global__ void HEX_VEC_BOUNDS kv_fct_cell1(HexGeo g, int nT, float step, const 
   for (int j = 0; j < 4; ++j) {
     const int k = k0 + j;
     float m = (ow(j) + 0.0f) * ro.a[j];
-    if (k < L - 1) m = m - fct_fcol_win(step, ow, www, j + 1) * g.rdzw[k];
-    if (k >= 1) m = m + fct_fcol_win(step, ow, www, j) * g.rdzw[k];
-    mass[j] = m;
-    s_in[j] = -g.rdzw[k] * (neg0(vr[j + 1]) - pos0(vr[j]));
-    s_out[j] = -g.rdzw[k] * (pos0(vr[j + 1]) - neg0(vr[j]));
+    const float up = m - fc[j + 1] * rz.a[j];
+    m = k < L - 1 ? up : m;
+    const float down = m + fc[j] * rz.a[j];
+    mass[j] = k >= 1 ? down : m;
+    s_in[j] = -rz.a[j] * (neg0(vr[j + 1]) - pos0(vr[j]));
+    s_out[j] = -rz.a[j] * (pos0(vr[j + 1]) - neg0(vr[j]));
   }
   const float ia = g.inv_area[c];
   HEX_GATHER
   for (int s = 0; s < n; ++s) {
-    const int e = g.eoc[c * g.maxE + s];
-    const float cs = g.csign[c * g.maxE + s];
+    const int2 sl = __ldg(g.slot + c * g.maxE + s);
+    const int eo = slot_edge(sl.x);
+    const float cs = slot_sign(sl.x);
     const float ts = -cs;
-    const float dvs = g.dv[e] * step;
-    const V4 vel = ld4(hv + e * S + k0), h = ld4(he + e * S + k0);
+    const float dvs = cs * __ldg(g.sdv + c * g.maxE + s) * step;  // dv step
+    const V4 vel = ld4(hv + k0 + eo), h = ld4(he + k0 + eo);
     V4 o0, o1;
     if (ACROSS) {
       // csign > 0: this cell is the edge's first cell
-      const V4 on = ld4(ot + g.coc[c * g.maxE + s] * S + k0);
+      const V4 on = ld4(ot + k0 + sl.y);
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         mn[j] = pymin(mn[j], on.a[j] + 0.0f);
@@ -1521,13 +1526,14 @@ __global__ void HEX_VEC_BOUNDS kv_fct_cell1(HexGeo g, int nT, float step, const 
         o1.a[j] = cs > 0.0f ? on.a[j] : ow(j);
       }
     } else {
-      o0 = ld4(ot + g.coe[2 * e] * S + k0);
-      o1 = ld4(ot + g.coe[2 * e + 1] * S + k0);
+      const int2 ends = __ldg(g.ends + g.eoc[c * g.maxE + s]);
+      o0 = ld4(ot + k0 + ends.x);
+      o1 = ld4(ot + k0 + ends.y);
     }
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const float upw = dvs * (pos0(vel.a[j]) * (o0.a[j] + 0.0f) + neg0(vel.a[j]) * (o1.a[j] + 0.0f));
-      mass[j] = mass[j] + ts * upw * ia;
+      mass[j] = fma_sign(ts, upw * ia, mass[j]);
       const float hres = step * h.a[j] - upw;
       const float sr = -ts * hres;
       s_out[j] = s_out[j] - pos0(sr) * ia;
@@ -1556,7 +1562,8 @@ __global__ void __launch_bounds__(256, HEX_FCT_EDGE_MIN_BLOCKS) kv_fct_edge(HexG
   const int e = ent, S = g.S;
   const size_t toff = (size_t)tr * g.nC * S;
   const size_t eoff = (size_t)tr * g.nE * S;
-  const int i0 = g.coe[2 * e] * S + k0, i1 = g.coe[2 * e + 1] * S + k0;
+  const int2 ends = __ldg(g.ends + e);
+  const int i0 = ends.x + k0, i1 = ends.y + k0;
   const V4 vel = ld4(hv + e * S + k0), h = ld4(high_e + eoff + e * S + k0);
   const V4 o0 = ld4(q_old + toff + i0), o1 = ld4(q_old + toff + i1);
   const V4 so0 = ld4(scale_out + toff + i0), si1 = ld4(scale_in + toff + i1);
@@ -1588,13 +1595,13 @@ __global__ void HEX_VEC_BOUNDS kv_fct_cell2(HexGeo g, int nT, const float* __res
   const float ia = g.inv_area[c];
   HEX_GATHER
   for (int s = 0; s < n; ++s) {
-    const int e = g.eoc[c * g.maxE + s];
-    const float ts = -g.csign[c * g.maxE + s];
-    const V4 h = ld4(hl + e * S + k0);
+    const int sl = __ldg(&g.slot[c * g.maxE + s].x);
+    const float ts = -slot_sign(sl);
+    const V4 h = ld4(hl + k0 + slot_edge(sl));
 #pragma unroll
-    for (int j = 0; j < 4; ++j) mass.a[j] = mass.a[j] + ts * h.a[j] * ia;
+    for (int j = 0; j < 4; ++j) mass.a[j] = fma_sign(ts, h.a[j] * ia, mass.a[j]);
   }
-  const Win siw = win(scale_in + toff + c * S, k0, S), sow = win(scale_out + toff + c * S, k0, S);
+  const Win siw = win<1, 1>(scale_in + toff + c * S, k0, S), sow = win<1, 1>(scale_out + toff + c * S, k0, S);
   // interface k0 + 4 belongs to the next chunk; past the column's last chunk
   // it only feeds a padding level, never stored
   const float* vc = vres + toff + c * S;
@@ -1614,7 +1621,7 @@ __global__ void HEX_VEC_BOUNDS kv_fct_cell2(HexGeo g, int nT, const float* __res
   for (int j = 0; j < 4; ++j) {
     const int k = k0 + j;
     const float m = mass.a[j] - g.rdzw[k] * (vl[j + 1] - vl[j]);
-    out.a[j] = pos0(m / td.a[j]);
+    out.a[j] = pos0(m / inside(td.a[j], k, g.L));
   }
   st4m(q_out + toff + ii, out, k0, 0, g.L);
 }
@@ -1868,10 +1875,9 @@ __global__ void HEX_VEC_BOUNDS kv_ac_cell(HexGeo g, int first, float dts, float 
     const V4 tc = ld4(theta_s + ii);
     HEX_GATHER
     for (int s = 0; s < n; ++s) {
-      const int e = g.eoc[c * g.maxE + s];
-      const int e0 = g.coe[2 * e], e1 = g.coe[2 * e + 1];
-      const float sdd = g.csign[c * g.maxE + s] * dts * g.dv[e];
-      const V4 r = ld4(ru_p + e * S + k0), tn = ld4(theta_s + (e0 == c ? e1 : e0) * S + k0);
+      const int2 sl = __ldg(g.slot + c * g.maxE + s);
+      const float sdd = __ldg(g.sdv + c * g.maxE + s) * dts;  // (csign dts) dv
+      const V4 r = ld4(ru_p + k0 + slot_edge(sl.x)), tn = ld4(theta_s + k0 + sl.y);
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         const float flux = sdd * r.a[j] * ia;

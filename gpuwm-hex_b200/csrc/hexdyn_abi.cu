@@ -413,6 +413,61 @@ int build(HexDynHandle* h, const HexDynDesc& d, const std::vector<float>* smdiv_
   UP(g.dss, pad_levels(d.dss, L, nC, S)) UP(g.rho_base, pad_levels(d.rho_base, L, nC, S))
   UP(g.rtheta_base, pad_levels(d.rho_theta_base, L, nC, S)) UP(g.exner_base, pad_levels(d.exner_base, L, nC, S))
   {
+    // stencil records (dycore_geo.cuh); every product formed here is one FP32
+    // operation of the kernels' expressions (signs are exact, so csign x dv
+    // and its later factors round as the reference's (csign x dts) x dv)
+    auto bits = [](float x) {
+      int i;
+      memcpy(&i, &x, sizeof i);
+      return i;
+    };
+    g.nbrW = (g.maxE2 + 1) / 2;
+    std::vector<int4> nbr((size_t)nE * g.nbrW, int4{0, 0, 0, 0}), vedge(3 * (size_t)nV);
+    std::vector<int> adv_off((size_t)nE * g.advW, 0);
+    std::vector<float2> adv_pm((size_t)nE * g.advW, float2{0.0f, 0.0f});
+    std::vector<int2> slot((size_t)nC * mE, int2{0, 0}), vslot(slot), eslot(slot), ends(nE), vends(nE);
+    std::vector<float> sdv((size_t)nC * mE, 0.0f);
+    for (int ei = 0; ei < nE; ++ei) {
+      for (int s = 0; s < neoe[ei]; ++s) {
+        int4& r = nbr[(size_t)ei * g.nbrW + s / 2];
+        const int off = eoe[(size_t)ei * g.maxE2 + s] * S, w = bits(d.weights_on_edge[(size_t)ei * g.maxE2 + s]);
+        if (s & 1) {
+          r.z = off;
+          r.w = w;
+        } else {
+          r.x = off;
+          r.y = w;
+        }
+      }
+      for (int s = 0; s < nadv[ei]; ++s) {
+        const size_t i = (size_t)ei * g.advW + s;
+        const float A = d.adv_coefs[i], B = d.adv_coefs_3rd[i], c3 = d.coef_3rd_order;
+        // A + (+-coef3) B, rounded as the build's kernels would (fast: one FMA)
+        const float X = c3 * B;
+        adv_off[i] = advc[i] * S;
+        adv_pm[i] = d.numerics ? float2{fmaf(c3, B, A), fmaf(-c3, B, A)} : float2{A + X, A - X};
+      }
+      ends[ei] = int2{coe[2 * ei] * S, coe[2 * ei + 1] * S};
+      vends[ei] = int2{voe[2 * ei] * S, voe[2 * ei + 1] * S};
+    }
+    for (int ci = 0; ci < nC; ++ci)
+      for (int s = 0; s < deg[ci]; ++s) {
+        const size_t i = (size_t)ci * mE + s;
+        const int e0 = eoc[i], v0 = voc[i], across = coe[2 * e0] == ci ? coe[2 * e0 + 1] : coe[2 * e0];
+        slot[i] = int2{(e0 * S) | (csign[i] < 0.0f ? 1 : 0), across * S};
+        sdv[i] = csign[i] * d.dv_edge[e0];
+        vslot[i] = int2{v0 * S, bits(d.kite_areas[3 * (size_t)v0 + kite_slot[i]])};
+        eslot[i] = int2{e0 * S, bits(d.dc_edge[e0] * d.dv_edge[e0])};
+      }
+    for (size_t i = 0; i < 3 * (size_t)nV; ++i) {
+      const int e0 = eov[i];
+      vedge[i] = int4{e0 * S, bits(vsign[i] * d.dc_edge[e0]), bits(d.dc_edge[e0] * d.dv_edge[e0]), 0};
+    }
+    UP(g.nbr, nbr) UP(g.adv_off, adv_off) UP(g.adv_pm, adv_pm) UP(g.slot, slot) UP(g.sdv, sdv)
+    UP(g.vslot, vslot) UP(g.eslot, eslot) UP(g.vedge, vedge)
+    UP(g.ends, ends) UP(g.vends, vends)
+  }
+  {
     // [L+1][C][maxE] -> [C][maxE][S]
     std::vector<float> zb((size_t)nC * mE * S, 0.0f), zb3((size_t)nC * mE * S, 0.0f);
     for (int k = 0; k <= L; ++k)
