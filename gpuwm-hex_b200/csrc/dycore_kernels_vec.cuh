@@ -10,33 +10,69 @@
 //
 // Thread layout: blockDim = (S/4, EPB4); x selects the chunk k0 = 4*x.
 
-// Blocks hold at most 256 threads (S/4 <= 256, checked at create).  The
-// resident-block target per SM sets the register cap: 4 blocks allow 64
-// registers a thread, 3 allow 80.
-#ifndef HEX_VEC_MIN_BLOCKS
-#define HEX_VEC_MIN_BLOCKS 4
-#endif
-#define HEX_VEC_BOUNDS __launch_bounds__(256, HEX_VEC_MIN_BLOCKS)
-// Kernels measured faster at another cap: the cell tendencies at 3 blocks
-// (80 registers, no spills: 80.8 vs 81.5 us), the edge diagnostics at 6, the momentum tendency (a
-// latency-bound ten-point gather) at 6 blocks (40 registers), the tracer
-// edge values (three tracers' accumulators per thread) at 2 (128), the
-// limited antidiffusive flux at 6 and the standard tracer update at 5.
-#ifndef HEX_TEND_U_MIN_BLOCKS
-#define HEX_TEND_U_MIN_BLOCKS 6
-#endif
-#ifndef HEX_EDGE_ADV_MIN_BLOCKS
-#define HEX_EDGE_ADV_MIN_BLOCKS HEX_VEC_MIN_BLOCKS
-#endif
-#ifndef HEX_TR_EDGE_MIN_BLOCKS
-#define HEX_TR_EDGE_MIN_BLOCKS 2
-#endif
-#ifndef HEX_FCT_EDGE_MIN_BLOCKS
-#define HEX_FCT_EDGE_MIN_BLOCKS 6
-#endif
-#ifndef HEX_TR_STD_MIN_BLOCKS
-#define HEX_TR_STD_MIN_BLOCKS 5
-#endif
+// Blocks hold at most 256 threads (S/4 <= 256, checked at create).  HEX_B_x
+// is the target of resident 256-thread blocks per SM of kernel x, which sets
+// its register cap (3: 80 registers, 4: 64, 5: 48, 6: 40, 8: 32), HEX_U_x the
+// unroll of its neighbour loops.  These kernels wait on gathered loads, and
+// how many warps are resident counts for more than how many loads one thread
+// has in flight.  Swept together on the x1.40962 workload (us per launch):
+// the tracer edge values 141 unrolled by one (60 registers), 175 by two, 181
+// by three; the momentum tendency 73 at 6 blocks, 76 at 4 and 5, 79 at 8; the
+// cell tendencies 77 at 3 blocks unrolled by six, 80 by two, 92 by one, 104 at
+// 6; the cell recovery 66 by one, 69 by two; the limiter's bounds 233 by one,
+// 250 by two, 449 at 8; the standard tracer update 110 at 6 blocks by two,
+// 115 at 5, 128 at 3; the limited fluxes 113 at 8, 129 at 6; the edge
+// diagnostics 27 at 8, 31 at 6; the acoustic cell pass 62 at 3 (128 threads),
+// 66 at 4; the vertical coefficients 56 at 5, 62 at 4.
+#define HEX_B_diag_vertex 4
+#define HEX_B_diag_cell 4
+#define HEX_U_diag_cell 1
+#define HEX_B_diag_edge 8
+#define HEX_U_diag_edge 1
+#define HEX_B_euler_edge 4
+#define HEX_B_euler_cell 4
+#define HEX_B_hdiv 4
+#define HEX_U_mass_flux 3
+#define HEX_B_moist_cell 4
+#define HEX_U_moist_cell 2
+#define HEX_B_moist_edge 4
+#define HEX_U_moist_edge 1
+#define HEX_B_edge_adv 4
+#define HEX_U_edge_adv 2
+#define HEX_B_tend_u 6
+#define HEX_U_tend_u 1
+#define HEX_B_tend_cell 3
+#define HEX_U_tend_cell 6
+#define HEX_B_vcoef 5
+#define HEX_B_ac_edge 4
+#define HEX_B_ac_cell 3
+#define HEX_U_ac_cell 2
+#define HEX_B_recover_edge 4
+#define HEX_B_recover_cell 4
+#define HEX_U_recover_cell 1
+#define HEX_B_tr_edge 4
+#define HEX_U_tr_edge 1
+#define HEX_B_tr_std 6
+#define HEX_U_tr_std 2
+#define HEX_B_fct_target 4
+#define HEX_U_fct_target 2
+#define HEX_B_fct_cell1 4
+#define HEX_U_fct_cell1 1
+#define HEX_B_fct_edge 8
+#define HEX_B_fct_cell2 8
+#define HEX_U_fct_cell2 1
+#define HEX_B_clamp_scalars 4
+#define HEX_B_smag_kdiff 4
+#define HEX_U_smag_kdiff 2
+#define HEX_B_mix_edge2 4
+#define HEX_B_mix_cell2 3
+#define HEX_U_mix_cell2 2
+#define HEX_B_mix_lap_vertex 4
+#define HEX_B_mix_lap_cell 4
+#define HEX_U_mix_lap_cell 2
+#define HEX_B_mix_edge4 4
+#define HEX_B_mix_cell4 4
+#define HEX_U_mix_cell4 2
 
 #define HEX_VEC_PARALLEL(n)                                \
   const int k0 = threadIdx.x * 4;                          \
@@ -52,33 +88,8 @@
   const int ent = (blockIdx.x / (nT)) * blockDim.y + threadIdx.y; \
   if (ent >= (n)) return;
 
-// Neighbour gathers: each iteration loads an index and then the neighbour's
-// levels, so unrolling lets the loads of several neighbours be in flight
-// together.  HEX_GATHER_UNROLL sets the unroll factor (0: the compiler's choice).
-#ifndef HEX_GATHER_UNROLL
-#define HEX_GATHER_UNROLL 2
-#endif
-// Per-kernel unroll of the neighbour loop (default HEX_GATHER_UNROLL).
-// Swept on the x1.40962 workload: the theta/w edge values run fastest
-// unrolled by five (55.5 vs 58.3 us per launch; three 57.7); the momentum
-// tendency by four or five (with 64 registers) and the tracer edge values by
-// three or five were slower than two.
-#ifndef HEX_TEND_U_UNROLL
-#define HEX_TEND_U_UNROLL HEX_GATHER_UNROLL
-#endif
-#ifndef HEX_TR_EDGE_UNROLL
-#define HEX_TR_EDGE_UNROLL HEX_GATHER_UNROLL
-#endif
-#ifndef HEX_EDGE_ADV_UNROLL
-#define HEX_EDGE_ADV_UNROLL 5
-#endif
 #define HEX_PRAGMA(x) _Pragma(#x)
 #define HEX_UNROLL_N(n) HEX_PRAGMA(unroll n)
-#if HEX_GATHER_UNROLL > 0
-#define HEX_GATHER HEX_UNROLL_N(HEX_GATHER_UNROLL)
-#else
-#define HEX_GATHER
-#endif
 
 struct V4 {
   float a[4];
@@ -171,7 +182,7 @@ __device__ __forceinline__ Win win(const float* __restrict__ col, int k0, int S)
 // End-of-step clamp of negative mixing ratios (hexcore/cuda_driver.py:5311,
 // `putmask(scalars, scalars < 0, 0)`): -0 and NaN compare false and stay.
 // blockIdx.z selects the scalar.
-__global__ void HEX_VEC_BOUNDS kv_clamp_scalars(HexGeo g, float* __restrict__ q) {
+__global__ void __launch_bounds__(256, HEX_B_clamp_scalars) kv_clamp_scalars(HexGeo g, float* __restrict__ q) {
   HEX_VEC_PARALLEL(g.nC)
   float* p = q + ((size_t)blockIdx.z * g.nC + ent) * g.S + k0;
   V4 v = ld4rw(p);
@@ -186,7 +197,7 @@ __global__ void HEX_VEC_BOUNDS kv_clamp_scalars(HexGeo g, float* __restrict__ q)
 // qtot = sum of the scalars in scalar order, cqw = 1/(1 + (qtot(k) +
 // qtot(k-1))/2) above the surface, cqu = 1/(1 + sum of the two-cell means).
 // Scalars are stored [scalar][cell][S].
-__global__ void HEX_VEC_BOUNDS kv_moist_cell(HexGeo g, const float* __restrict__ q, int nT,
+__global__ void __launch_bounds__(256, HEX_B_moist_cell) kv_moist_cell(HexGeo g, const float* __restrict__ q, int nT,
                                              float* __restrict__ qtot, float* __restrict__ cqw) {
   HEX_VEC_PARALLEL(g.nC)
   const int c = ent, S = g.S;
@@ -194,7 +205,7 @@ __global__ void HEX_VEC_BOUNDS kv_moist_cell(HexGeo g, const float* __restrict__
   const float* qc = q + c * S + k0;
   V4 acc = v4zero();
   float below = 0.0f;  // qtot at level k0 - 1
-  HEX_GATHER
+  HEX_UNROLL_N(HEX_U_moist_cell)
   for (int t = 0; t < nT; ++t) {
     const V4 v = ld4(qc + t * tstride);
 #pragma unroll
@@ -211,7 +222,7 @@ __global__ void HEX_VEC_BOUNDS kv_moist_cell(HexGeo g, const float* __restrict__
   st4m(cqw + c * S + k0, cw, k0, 0, g.L);
 }
 
-__global__ void HEX_VEC_BOUNDS kv_moist_edge(HexGeo g, const float* __restrict__ q, int nT,
+__global__ void __launch_bounds__(256, HEX_B_moist_edge) kv_moist_edge(HexGeo g, const float* __restrict__ q, int nT,
                                              float* __restrict__ cqu) {
   HEX_VEC_PARALLEL(g.nE)
   const int e = ent, S = g.S;
@@ -220,7 +231,7 @@ __global__ void HEX_VEC_BOUNDS kv_moist_edge(HexGeo g, const float* __restrict__
   const float* q0 = q + ends.x + k0;
   const float* q1 = q + ends.y + k0;
   V4 acc = v4zero();
-  HEX_GATHER
+  HEX_UNROLL_N(HEX_U_moist_edge)
   for (int t = 0; t < nT; ++t) {
     const V4 a = ld4(q0 + t * tstride), b = ld4(q1 + t * tstride);
 #pragma unroll
@@ -235,7 +246,7 @@ __global__ void HEX_VEC_BOUNDS kv_moist_edge(HexGeo g, const float* __restrict__
 // ---------------------------------------------------------- diagnostics
 // hexcore/diagnostics.py:95 compute_solve_diagnostics, v8.4.1 stored inverses.
 
-__global__ void HEX_VEC_BOUNDS kv_diag_vertex(HexGeo g, const float* __restrict__ u, float* __restrict__ pv_vertex,
+__global__ void __launch_bounds__(256, HEX_B_diag_vertex) kv_diag_vertex(HexGeo g, const float* __restrict__ u, float* __restrict__ pv_vertex,
                                float* __restrict__ ke_vertex, float* __restrict__ vorticity) {
   HEX_VEC_PARALLEL(g.nV)
   const int v = ent, S = g.S;
@@ -267,7 +278,7 @@ __global__ void HEX_VEC_BOUNDS kv_diag_vertex(HexGeo g, const float* __restrict_
 // Cell kinetic energy (v8.4.1 kite blend 0.625) and, with APVM, cell PV;
 // DIV: also the divergence of u (the horizontal mixing's input).
 template <bool DIV>
-__global__ void HEX_VEC_BOUNDS kv_diag_cell(HexGeo g, const float* __restrict__ u, const float* __restrict__ pv_vertex,
+__global__ void __launch_bounds__(256, HEX_B_diag_cell) kv_diag_cell(HexGeo g, const float* __restrict__ u, const float* __restrict__ pv_vertex,
                              const float* __restrict__ ke_vertex, float* __restrict__ ke_out,
                              float* __restrict__ pv_cell, float* __restrict__ divergence) {
   HEX_VEC_PARALLEL(g.nC)
@@ -277,7 +288,7 @@ __global__ void HEX_VEC_BOUNDS kv_diag_cell(HexGeo g, const float* __restrict__ 
   const int2* slots = g.vslot + c * g.maxE;
   const int2* eslots = g.eslot + c * g.maxE;
   V4 ke = v4zero(), dv = v4zero();
-  HEX_GATHER
+  HEX_UNROLL_N(HEX_U_diag_cell)
   for (int s = 0; s < n; ++s) {
     const int2 r = __ldg(eslots + s);
     const float dd = fbits(r.y);
@@ -298,7 +309,7 @@ __global__ void HEX_VEC_BOUNDS kv_diag_cell(HexGeo g, const float* __restrict__ 
 #pragma unroll
   for (int j = 0; j < 4; ++j) ke.a[j] = ke.a[j] * ia * 0.625f;
   V4 pvc = v4zero();
-  HEX_GATHER
+  HEX_UNROLL_N(HEX_U_diag_cell)
   for (int s = 0; s < n; ++s) {
     const int2 r = __ldg(slots + s);
     const float kite = fbits(r.y);
@@ -317,7 +328,7 @@ __global__ void HEX_VEC_BOUNDS kv_diag_cell(HexGeo g, const float* __restrict__ 
 }
 
 // Tangential velocity (TRiSK weights) and edge PV with APVM upwinding.
-__global__ void __launch_bounds__(256, 6) kv_diag_edge(HexGeo g, const float* __restrict__ u, const float* __restrict__ pv_vertex,
+__global__ void __launch_bounds__(256, HEX_B_diag_edge) kv_diag_edge(HexGeo g, const float* __restrict__ u, const float* __restrict__ pv_vertex,
                              const float* __restrict__ pv_cell, float* __restrict__ v, float* __restrict__ pv_edge,
                              int recompute_v) {
   HEX_VEC_PARALLEL(g.nE)
@@ -327,7 +338,7 @@ __global__ void __launch_bounds__(256, 6) kv_diag_edge(HexGeo g, const float* __
     vt = v4zero();
     const int n = g.neoe[e];
     const int4* nbr = g.nbr + (size_t)e * g.nbrW;
-    HEX_GATHER
+    HEX_UNROLL_N(HEX_U_diag_edge)
     for (int s = 0; s + 1 < n; s += 2) {
       const int4 r = __ldg(nbr + (s >> 1));
       const V4 ua = ld4(u + k0 + r.x), ub = ld4(u + k0 + r.z);
@@ -374,7 +385,7 @@ __device__ __forceinline__ float dpdz_of(const HexGeo& g, float rp, float qt, fl
 }
 
 // hexcore/dynamics.py:188 pressure_gradient_euler_tendency.
-__global__ void HEX_VEC_BOUNDS kv_euler_edge(HexGeo g, const float* __restrict__ pp, const float* __restrict__ rp,
+__global__ void __launch_bounds__(256, HEX_B_euler_edge) kv_euler_edge(HexGeo g, const float* __restrict__ pp, const float* __restrict__ rp,
                               const float* __restrict__ qtot, const float* __restrict__ cqu,
                               float* __restrict__ euler_ru) {
   HEX_VEC_PARALLEL(g.nE)
@@ -394,7 +405,7 @@ __global__ void HEX_VEC_BOUNDS kv_euler_edge(HexGeo g, const float* __restrict__
   for (int j = 0; j < 4; ++j) {
     const float d0 = dpdz_of(g, r0.a[j], q0.a[j], b0.a[j]);
     const float d1 = dpdz_of(g, r1.a[j], q1.a[j], b1.a[j]);
-    out.a[j] = -cq.a[j] * ((p1.a[j] - p0.a[j]) * idc / inside(0.5f * (z1.a[j] + z0.a[j]), k0 + j, g.L) - 0.5f * zx.a[j] * (d0 + d1));
+    out.a[j] = -cq.a[j] * ((p1.a[j] - p0.a[j]) * idc / (0.5f * (z1.a[j] + z0.a[j])) - 0.5f * zx.a[j] * (d0 + d1));
   }
   st4m(euler_ru + e * S + k0, out, k0, 0, g.L);
 }
@@ -403,7 +414,7 @@ __global__ void HEX_VEC_BOUNDS kv_euler_edge(HexGeo g, const float* __restrict__
 __device__ __forceinline__ V4 mass_flux_div4(const HexGeo& g, const float* __restrict__ ru, int c, int k0) {
   V4 acc = v4zero();
   const int n = g.deg[c];
-  HEX_GATHER
+  HEX_UNROLL_N(HEX_U_mass_flux)
   for (int s = 0; s < n; ++s) {
     const float sd = __ldg(g.sdv + c * g.maxE + s);
     const V4 r = ld4(ru + k0 + __ldg(g.eslot + c * g.maxE + s).x);
@@ -417,7 +428,7 @@ __device__ __forceinline__ V4 mass_flux_div4(const HexGeo& g, const float* __res
 }
 
 // hexcore/dynamics.py:122 density_tendency and hexcore/driver.py:2804 Euler w.
-__global__ void HEX_VEC_BOUNDS kv_euler_cell(HexGeo g, const float* __restrict__ ru, const float* __restrict__ rw,
+__global__ void __launch_bounds__(256, HEX_B_euler_cell) kv_euler_cell(HexGeo g, const float* __restrict__ ru, const float* __restrict__ rw,
                               const float* __restrict__ pp, const float* __restrict__ rp,
                               const float* __restrict__ qtot, const float* __restrict__ cqw,
                               float* __restrict__ tend_rho, float* __restrict__ euler_rw,
@@ -461,14 +472,14 @@ __global__ void HEX_VEC_BOUNDS kv_euler_cell(HexGeo g, const float* __restrict__
 
 // ------------------------------------------------- stage tendencies
 // hexcore/dynamics.py:86 mass_flux_divergence of the stage rho*u.
-__global__ void HEX_VEC_BOUNDS kv_hdiv(HexGeo g, const float* __restrict__ ru, float* __restrict__ hdiv) {
+__global__ void __launch_bounds__(256, HEX_B_hdiv) kv_hdiv(HexGeo g, const float* __restrict__ ru, float* __restrict__ hdiv) {
   HEX_VEC_PARALLEL(g.nC)
   st4m(hdiv + ent * g.S + k0, mass_flux_div4(g, ru, ent, k0), k0, 0, g.L);
 }
 
 // Third-order edge values of theta_m (levels) and w (interfaces):
 // hexcore/driver.py:1023-1034 and :1159-1172.
-__global__ void __launch_bounds__(256, HEX_EDGE_ADV_MIN_BLOCKS) kv_edge_adv(HexGeo g, const float* __restrict__ ru, const float* __restrict__ theta,
+__global__ void __launch_bounds__(256, HEX_B_edge_adv) kv_edge_adv(HexGeo g, const float* __restrict__ ru, const float* __restrict__ theta,
                             const float* __restrict__ w, float* __restrict__ edge_theta,
                             float* __restrict__ edge_w) {
   HEX_VEC_PARALLEL(g.nE)
@@ -489,7 +500,7 @@ __global__ void __launch_bounds__(256, HEX_EDGE_ADV_MIN_BLOCKS) kv_edge_adv(HexG
     nw[j] = signbit(fm.a[j] * r.a[j] + fp.a[j] * rprev);
   }
   V4 at = v4zero(), aw = v4zero();
-  HEX_UNROLL_N(HEX_EDGE_ADV_UNROLL)
+  HEX_UNROLL_N(HEX_U_edge_adv)
   for (int s = 0; s < n; ++s) {
     const int o = __ldg(off + s);
     const float2 c = __ldg(pm + s);
@@ -540,7 +551,7 @@ __device__ __forceinline__ void column_ends(int k0, int L, float (&f)[5], F edge
 // RAYLEIGH: the upper Rayleigh damping of u is compiled in (an instance
 // without it keeps the common path's registers).
 template <bool RAYLEIGH>
-__global__ void __launch_bounds__(256, HEX_TEND_U_MIN_BLOCKS) kv_tend_u(HexGeo g, const float* __restrict__ u, const float* __restrict__ rw,
+__global__ void __launch_bounds__(256, HEX_B_tend_u) kv_tend_u(HexGeo g, const float* __restrict__ u, const float* __restrict__ rw,
                           const float* __restrict__ rho, const float* __restrict__ pv_edge,
                           const float* __restrict__ ke, const float* __restrict__ hdiv,
                           const float* __restrict__ euler_ru, float* __restrict__ tend_ru,
@@ -560,7 +571,7 @@ __global__ void __launch_bounds__(256, HEX_TEND_U_MIN_BLOCKS) kv_tend_u(HexGeo g
       q.a[j] = q.a[j] + w * un.a[j] * work_pv;
     }
   };
-  HEX_UNROLL_N(HEX_TEND_U_UNROLL)
+  HEX_UNROLL_N(HEX_U_tend_u)
   for (int s = 0; s + 1 < n; s += 2) {
     const int4 r = __ldg(nbr + (s >> 1));
     const V4 ua = ld4(u + k0 + r.x), pa = ld4(pv_edge + k0 + r.x);
@@ -646,7 +657,7 @@ __global__ void __launch_bounds__(256, HEX_TEND_U_MIN_BLOCKS) kv_tend_u(HexGeo g
 
 // tend_rt (hexcore/driver.py:933), tend_rw (:1081) + Euler w, then
 // hexcore/acoustic.py:246 convert_w_tendency_to_omega.
-__global__ void __launch_bounds__(256, 3) kv_tend_cell(HexGeo g, const float* __restrict__ ru, const float* __restrict__ ru_s,
+__global__ void __launch_bounds__(256, HEX_B_tend_cell) kv_tend_cell(HexGeo g, const float* __restrict__ ru, const float* __restrict__ ru_s,
                              const float* __restrict__ rw, const float* __restrict__ rws,
                              const float* __restrict__ theta, const float* __restrict__ theta_s,
                              const float* __restrict__ w, const float* __restrict__ edge_theta,
@@ -662,7 +673,7 @@ __global__ void __launch_bounds__(256, 3) kv_tend_cell(HexGeo g, const float* __
   const V4 fm = ld4(g.fzm + k0), fp = ld4(g.fzp + k0);
   // horizontal parts: rho-theta flux divergence, RK>1 correction, w flux
   V4 res = v4zero(), hres = v4zero();
-  HEX_GATHER
+  HEX_UNROLL_N(HEX_U_tend_cell)
   for (int s = 0; s < n; ++s) {
     const int sl = __ldg(&slots[s].x), eo = slot_edge(sl);
     const float sg = slot_sign(sl);
@@ -680,7 +691,7 @@ __global__ void __launch_bounds__(256, 3) kv_tend_cell(HexGeo g, const float* __
   }
   if (rk_step > 1) {
     const V4 tc = ld4(theta_s + c * S + k0);
-    HEX_GATHER
+    HEX_UNROLL_N(HEX_U_tend_cell)
     for (int s = 0; s < n; ++s) {
       const int2 sl = __ldg(slots + s);
       const int eo = slot_edge(sl.x);
@@ -729,7 +740,7 @@ __global__ void __launch_bounds__(256, 3) kv_tend_cell(HexGeo g, const float* __
     trw.a[j] = rsw + er.a[j];
   }
   // omega conversion (interfaces 1..L-1)
-  HEX_GATHER
+  HEX_UNROLL_N(HEX_U_tend_cell)
   for (int s = 0; s < n; ++s) {
     const int sl = __ldg(&slots[s].x), eo = slot_edge(sl);
     const float sg = slot_sign(sl);
@@ -795,13 +806,13 @@ __device__ __forceinline__ float np_min(float a, float b) { return a != a ? a : 
 
 // hexcore/mixing_v841.py:615 smagorinsky_2d: kdiff of every cell level from
 // the deformation of the edge normal (u) and tangential (v) velocities.
-__global__ void HEX_VEC_BOUNDS kv_smag_kdiff(HexGeo g, const float* __restrict__ u, const float* __restrict__ v,
+__global__ void __launch_bounds__(256, HEX_B_smag_kdiff) kv_smag_kdiff(HexGeo g, const float* __restrict__ u, const float* __restrict__ v,
                               float* __restrict__ kdiff) {
   HEX_VEC_PARALLEL(g.nC)
   const int c = ent, S = g.S;
   const int n = g.deg[c];
   V4 dudx = v4zero(), dudy = v4zero(), dvdx = v4zero(), dvdy = v4zero();
-  HEX_GATHER
+  HEX_UNROLL_N(HEX_U_smag_kdiff)
   for (int s = 0; s < n; ++s) {
     const int e = g.eoc[c * g.maxE + s];
     const float c2 = g.deform_c2[c * g.maxE + s], s2 = g.deform_s2[c * g.maxE + s];
@@ -836,7 +847,7 @@ __global__ void HEX_VEC_BOUNDS kv_smag_kdiff(HexGeo g, const float* __restrict__
 // hexcore/mixing.py:391-474 second-order momentum filter: delsq_u and the
 // Euler u term plus rho_edge kdiff delsq_u meshScalingDel2 (rho_edge the
 // diagnostics' h_edge of the subcycle's start density).
-__global__ void HEX_VEC_BOUNDS kv_mix_edge2(HexGeo g, const float* __restrict__ div, const float* __restrict__ vort,
+__global__ void __launch_bounds__(256, HEX_B_mix_edge2) kv_mix_edge2(HexGeo g, const float* __restrict__ div, const float* __restrict__ vort,
                              const float* __restrict__ kdiff, const float* __restrict__ rho,
                              const float* __restrict__ euler_ru, float* __restrict__ delsq_u,
                              float* __restrict__ mix_u) {
@@ -865,10 +876,7 @@ __global__ void HEX_VEC_BOUNDS kv_mix_edge2(HexGeo g, const float* __restrict__ 
 
 // hexcore/mixing.py:533 (w, interfaces 1..L-1) and :638 (theta) second-order
 // filters of a cell, with their Laplacians delsq_w and delsq_theta.
-#ifndef HEX_MIX_CELL2_MIN_BLOCKS
-#define HEX_MIX_CELL2_MIN_BLOCKS 3
-#endif
-__global__ void __launch_bounds__(256, HEX_MIX_CELL2_MIN_BLOCKS) kv_mix_cell2(HexGeo g, const float* __restrict__ kdiff, const float* __restrict__ rho,
+__global__ void __launch_bounds__(256, HEX_B_mix_cell2) kv_mix_cell2(HexGeo g, const float* __restrict__ kdiff, const float* __restrict__ rho,
                              const float* __restrict__ w, const float* __restrict__ theta,
                              float* __restrict__ w_mix, float* __restrict__ delsq_w,
                              float* __restrict__ theta_mix, float* __restrict__ delsq_theta) {
@@ -877,7 +885,7 @@ __global__ void __launch_bounds__(256, HEX_MIX_CELL2_MIN_BLOCKS) kv_mix_cell2(He
   const int n = g.deg[c];
   const float ia = g.inv_area[c];
   V4 tw = v4zero(), dw = v4zero(), tt = v4zero(), dt = v4zero();
-  HEX_GATHER
+  HEX_UNROLL_N(HEX_U_mix_cell2)
   for (int s = 0; s < n; ++s) {
     const int e = g.eoc[c * g.maxE + s];
     const int c0 = g.coe[2 * e], c1 = g.coe[2 * e + 1];
@@ -917,7 +925,7 @@ __global__ void __launch_bounds__(256, HEX_MIX_CELL2_MIN_BLOCKS) kv_mix_cell2(He
 
 // hexcore/mixing.py:464-476: the Laplacians of delsq_u at vertices
 // (vorticity form) and cells (divergence form).
-__global__ void HEX_VEC_BOUNDS kv_mix_lap_vertex(HexGeo g, const float* __restrict__ delsq_u,
+__global__ void __launch_bounds__(256, HEX_B_mix_lap_vertex) kv_mix_lap_vertex(HexGeo g, const float* __restrict__ delsq_u,
                                   float* __restrict__ delsq_vort) {
   HEX_VEC_PARALLEL(g.nV)
   const int v = ent, S = g.S;
@@ -932,13 +940,13 @@ __global__ void HEX_VEC_BOUNDS kv_mix_lap_vertex(HexGeo g, const float* __restri
   }
   st4m(delsq_vort + v * S + k0, acc, k0, 0, g.L);
 }
-__global__ void HEX_VEC_BOUNDS kv_mix_lap_cell(HexGeo g, const float* __restrict__ delsq_u,
+__global__ void __launch_bounds__(256, HEX_B_mix_lap_cell) kv_mix_lap_cell(HexGeo g, const float* __restrict__ delsq_u,
                                 float* __restrict__ delsq_div) {
   HEX_VEC_PARALLEL(g.nC)
   const int c = ent, S = g.S;
   const int n = g.deg[c];
   V4 acc = v4zero();
-  HEX_GATHER
+  HEX_UNROLL_N(HEX_U_mix_lap_cell)
   for (int s = 0; s < n; ++s) {
     const int e = g.eoc[c * g.maxE + s];
     const float factor = g.inv_area[c] * g.dv[e] * g.csign[c * g.maxE + s];
@@ -950,7 +958,7 @@ __global__ void HEX_VEC_BOUNDS kv_mix_lap_cell(HexGeo g, const float* __restrict
 }
 
 // hexcore/mixing.py:478-490 fourth-order momentum filter (subtracted).
-__global__ void HEX_VEC_BOUNDS kv_mix_edge4(HexGeo g, const float* __restrict__ rho,
+__global__ void __launch_bounds__(256, HEX_B_mix_edge4) kv_mix_edge4(HexGeo g, const float* __restrict__ rho,
                              const float* __restrict__ delsq_div, const float* __restrict__ delsq_vort,
                              float* __restrict__ mix_u) {
   HEX_VEC_PARALLEL(g.nE)
@@ -977,7 +985,7 @@ __global__ void HEX_VEC_BOUNDS kv_mix_edge4(HexGeo g, const float* __restrict__ 
 
 // hexcore/mixing.py:576-590 and :719-733 fourth-order w and theta filters
 // (when visc4 > 0), then the saved w term euler_rw + w filter (driver.py:2870).
-__global__ void HEX_VEC_BOUNDS kv_mix_cell4(HexGeo g, const float* __restrict__ delsq_w,
+__global__ void __launch_bounds__(256, HEX_B_mix_cell4) kv_mix_cell4(HexGeo g, const float* __restrict__ delsq_w,
                              const float* __restrict__ delsq_theta, const float* __restrict__ euler_rw,
                              const float* __restrict__ w_mix, float* __restrict__ theta_mix,
                              float* __restrict__ mix_w) {
@@ -987,7 +995,7 @@ __global__ void HEX_VEC_BOUNDS kv_mix_cell4(HexGeo g, const float* __restrict__ 
   if (g.smag_h4 > 0.0f) {
     const int n = g.deg[c];
     const float scale = g.smag_h4 * g.inv_area[c];
-    HEX_GATHER
+    HEX_UNROLL_N(HEX_U_mix_cell4)
     for (int s = 0; s < n; ++s) {
       const int e = g.eoc[c * g.maxE + s];
       const int c0 = g.coe[2 * e], c1 = g.coe[2 * e + 1];
@@ -1016,7 +1024,7 @@ __global__ void HEX_VEC_BOUNDS kv_mix_cell4(HexGeo g, const float* __restrict__ 
 // substep (hexcore/mixing.py:851, stored inverse of dts), then the ru_p
 // update of this substep (hexcore/acoustic_v841.py:416-460).  mode 0: first
 // substep (ru_p = dts*tend_ru); 1: damping + update; 2: damping only.
-__global__ void HEX_VEC_BOUNDS kv_ac_edge(HexGeo g, int mode, int old_is_zero, float dts, float inv_dts,
+__global__ void __launch_bounds__(256, HEX_B_ac_edge) kv_ac_edge(HexGeo g, int mode, int old_is_zero, float dts, float inv_dts,
                            const float* __restrict__ tend_ru, const float* __restrict__ rtpp_new,
                            const float* __restrict__ rtpp_old, const float* __restrict__ rho_pp,
                            const float* __restrict__ theta_s, const float* __restrict__ exner_s,
@@ -1046,7 +1054,7 @@ __global__ void HEX_VEC_BOUNDS kv_ac_edge(HexGeo g, int mode, int old_is_zero, f
   for (int j = 0; j < 4; ++j) {
     const float d0 = n0.a[j] - o0.a[j];
     const float d1 = n1.a[j] - o1.a[j];
-    r.a[j] = r.a[j] + damp_coef * (d0 - d1) * (1.0f - 0.0f) / inside(t0.a[j] + t1.a[j], k0 + j, g.L);
+    r.a[j] = r.a[j] + damp_coef * (d0 - d1) * (1.0f - 0.0f) / (t0.a[j] + t1.a[j]);
   }
   if (mode == 1) {
     const V4 z0 = ld4(g.zz + i0), z1 = ld4(g.zz + i1), x0 = ld4(exner_s + i0), x1 = ld4(exner_s + i1);
@@ -1056,7 +1064,7 @@ __global__ void HEX_VEC_BOUNDS kv_ac_edge(HexGeo g, int mode, int old_is_zero, f
     const float idc = g.inv_dc[e];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      float pg = (n1.a[j] - n0.a[j]) * idc / inside(0.5f * (z1.a[j] + z0.a[j]), k0 + j, g.L);
+      float pg = (n1.a[j] - n0.a[j]) * idc / (0.5f * (z1.a[j] + z0.a[j]));
       pg = cq.a[j] * 0.5f * g.c2 * (x0.a[j] + x1.a[j]) * pg;
       pg = pg + 0.5f * zx.a[j] * g.g * (p0.a[j] + p1.a[j]);
       r.a[j] = r.a[j] + dts * (t.a[j] - pg);
@@ -1074,7 +1082,7 @@ __global__ void HEX_VEC_BOUNDS kv_ac_edge(HexGeo g, int mode, int old_is_zero, f
 // damp: the divergence damping of the stage's last acoustic substep
 // (kv_ac_edge mode 2: rtpp_new/rtpp_old its output/input, old_is_zero when
 // it was the first) is applied to ru_p here, stored, and recovered from.
-__global__ void HEX_VEC_BOUNDS kv_recover_edge(HexGeo g, const float* __restrict__ ru_s, float* ru_p,
+__global__ void __launch_bounds__(256, HEX_B_recover_edge) kv_recover_edge(HexGeo g, const float* __restrict__ ru_s, float* ru_p,
                                 const float* __restrict__ ru_avg, const float* __restrict__ rp_s,
                                 const float* __restrict__ rho_pp, float* __restrict__ ru_out,
                                 float* __restrict__ u_out, float* __restrict__ flux_u, int flux_mode,
@@ -1097,7 +1105,7 @@ __global__ void HEX_VEC_BOUNDS kv_recover_edge(HexGeo g, const float* __restrict
     for (int j = 0; j < 4; ++j) {
       const float d0 = n0.a[j] - o0.a[j];
       const float d1 = n1.a[j] - o1.a[j];
-      rp.a[j] = rp.a[j] + damp_coef * (d0 - d1) * (1.0f - 0.0f) / inside(t0.a[j] + t1.a[j], k0 + j, g.L);
+      rp.a[j] = rp.a[j] + damp_coef * (d0 - d1) * (1.0f - 0.0f) / (t0.a[j] + t1.a[j]);
     }
     st4m(ru_p + jj, rp, k0, 0, g.L);
   }
@@ -1110,7 +1118,7 @@ __global__ void HEX_VEC_BOUNDS kv_recover_edge(HexGeo g, const float* __restrict
     const float rho0 = a0.a[j] + b0.a[j] + c0.a[j];
     const float rho1 = a1.a[j] + b1.a[j] + c1.a[j];
     ru.a[j] = rs.a[j] + rp.a[j];
-    uo.a[j] = 2.0f * ru.a[j] / inside(rho0 + rho1, k0 + j, g.L);
+    uo.a[j] = 2.0f * ru.a[j] / (rho0 + rho1);
   }
   st4m(ru_out + jj, ru, k0, 0, g.L);
   st4m(u_out + jj, uo, k0, 0, g.L);
@@ -1132,7 +1140,7 @@ __global__ void HEX_VEC_BOUNDS kv_recover_edge(HexGeo g, const float* __restrict
 // hexcore/driver.py:3166-3292 stage recovery, cell part: candidate state,
 // rw end conditions, theta_m, Exner and p' at stage 3, w from
 // hexcore/terrain.py:491 recover_velocities, and the split w-flux average.
-__global__ void HEX_VEC_BOUNDS kv_recover_cell(HexGeo g, int stage3, const float* __restrict__ rp_s,
+__global__ void __launch_bounds__(256, HEX_B_recover_cell) kv_recover_cell(HexGeo g, int stage3, const float* __restrict__ rp_s,
                                 const float* __restrict__ rtp_s, const float* __restrict__ rw_s,
                                 const float* __restrict__ rho_pp, const float* __restrict__ rtpp,
                                 const float* __restrict__ rw_p, const float* __restrict__ ww_avg,
@@ -1213,7 +1221,7 @@ __global__ void HEX_VEC_BOUNDS kv_recover_cell(HexGeo g, int stage3, const float
   // the next stage's mass-flux divergence of ru_new (mass_flux_div4, the
   // same operands in the same order) accumulates in the same edge loop
   V4 hd = v4zero();
-  HEX_GATHER
+  HEX_UNROLL_N(HEX_U_recover_cell)
   for (int s = 0; s < n; ++s) {
     const int sl = __ldg(&g.slot[c * g.maxE + s].x), eo = slot_edge(sl);
     const float sign = slot_sign(sl), sd = __ldg(g.sdv + c * g.maxE + s);
@@ -1284,7 +1292,7 @@ __global__ void HEX_VEC_BOUNDS kv_recover_cell(HexGeo g, int stage3, const float
 #ifndef HEX_TR_GROUP
 #define HEX_TR_GROUP 3
 #endif
-__global__ void __launch_bounds__(256, HEX_TR_EDGE_MIN_BLOCKS) kv_tr_edge(HexGeo g, int nT, int mono, const float* __restrict__ q, const float* __restrict__ hv,
+__global__ void __launch_bounds__(256, HEX_B_tr_edge) kv_tr_edge(HexGeo g, int nT, int mono, const float* __restrict__ q, const float* __restrict__ hv,
                            float* __restrict__ out) {
   HEX_VEC_TRACER(g.nE, (nT + HEX_TR_GROUP - 1) / HEX_TR_GROUP)
   constexpr int TG = HEX_TR_GROUP;
@@ -1317,7 +1325,7 @@ __global__ void __launch_bounds__(256, HEX_TR_EDGE_MIN_BLOCKS) kv_tr_edge(HexGeo
           for (int j = 0; j < 4; ++j) res[t].a[j] = w[j] * qv.a[j];
         }
     }
-    HEX_UNROLL_N(HEX_TR_EDGE_UNROLL)
+    HEX_UNROLL_N(HEX_U_tr_edge)
     for (int s = 1; s < 10; ++s) {
       HEX_TR_WEIGHTS(s)
 #pragma unroll
@@ -1335,7 +1343,7 @@ __global__ void __launch_bounds__(256, HEX_TR_EDGE_MIN_BLOCKS) kv_tr_edge(HexGeo
   } else {
 #pragma unroll
     for (int t = 0; t < TG; ++t) res[t] = v4zero();
-    HEX_UNROLL_N(HEX_TR_EDGE_UNROLL)
+    HEX_UNROLL_N(HEX_U_tr_edge)
     for (int s = 0; s < n; ++s) {
       HEX_TR_WEIGHTS(s)
 #pragma unroll
@@ -1364,7 +1372,7 @@ __device__ __forceinline__ void tr_vflux_chunk(const HexGeo& g, const Win& q, co
 }
 
 // hexcore/transport.py:1649 advance_scalars (RK1/RK2 of split transport).
-__global__ void __launch_bounds__(256, HEX_TR_STD_MIN_BLOCKS) kv_tr_std(HexGeo g, int nT, float step, float wn, const float* __restrict__ q_old,
+__global__ void __launch_bounds__(256, HEX_B_tr_std) kv_tr_std(HexGeo g, int nT, float step, float wn, const float* __restrict__ q_old,
                           const float* __restrict__ q_stage, const float* __restrict__ rho_old,
                           const float* __restrict__ rho_new, const float* __restrict__ hv,
                           const float* __restrict__ ww, const float* __restrict__ edge_q,
@@ -1376,7 +1384,7 @@ __global__ void __launch_bounds__(256, HEX_TR_STD_MIN_BLOCKS) kv_tr_std(HexGeo g
   const float* ev = edge_q + (size_t)tr * g.nE * S;
   const int n = g.deg[c];
   V4 t = v4zero();
-  HEX_GATHER
+  HEX_UNROLL_N(HEX_U_tr_std)
   for (int s = 0; s < n; ++s) {
     const int sl = __ldg(&g.slot[c * g.maxE + s].x), eo = slot_edge(sl);
     const float ts = -slot_sign(sl);
@@ -1403,7 +1411,7 @@ __global__ void __launch_bounds__(256, HEX_TR_STD_MIN_BLOCKS) kv_tr_std(HexGeo g
 }
 
 // hexcore/transport.py:1887-1906 split-transport target density.
-__global__ void HEX_VEC_BOUNDS kv_fct_target(HexGeo g, float step, const float* __restrict__ rho_old,
+__global__ void __launch_bounds__(256, HEX_B_fct_target) kv_fct_target(HexGeo g, float step, const float* __restrict__ rho_old,
                               const float* __restrict__ hv, const float* __restrict__ ww,
                               float* __restrict__ target, int* flag) {
   HEX_VEC_PARALLEL(g.nC)
@@ -1412,7 +1420,7 @@ __global__ void HEX_VEC_BOUNDS kv_fct_target(HexGeo g, float step, const float* 
   const int n = g.deg[c];
   const float ia = g.inv_area[c];
   V4 hd = v4zero();
-  HEX_GATHER
+  HEX_UNROLL_N(HEX_U_fct_target)
   for (int s = 0; s < n; ++s) {
     const float tdv = -__ldg(g.sdv + c * g.maxE + s);  // (ts h) dv = h (ts dv), ts = -csign exact
     const V4 h = ld4(hv + k0 + __ldg(g.eslot + c * g.maxE + s).x);
@@ -1445,7 +1453,7 @@ __device__ __forceinline__ float fct_fcol_win(float step, const Win& o, const Wi
 // the bounds already load; the min/max over neighbours and the mass sums
 // still run in slot order, so the words are those of the two-loop form.
 template <bool ACROSS>
-__global__ void HEX_VEC_BOUNDS kv_fct_cell1(HexGeo g, int nT, float step, const float* __restrict__ q_old,
+__global__ void __launch_bounds__(256, HEX_B_fct_cell1) kv_fct_cell1(HexGeo g, int nT, float step, const float* __restrict__ q_old,
                              const float* __restrict__ q_stage, const float* __restrict__ rho_old,
                              const float* __restrict__ hv, const float* __restrict__ ww,
                              const float* __restrict__ high_e, const float* __restrict__ target,
@@ -1471,7 +1479,7 @@ __global__ void HEX_VEC_BOUNDS kv_fct_cell1(HexGeo g, int nT, float step, const 
   }
   const int n = g.deg[c];
   if (!ACROSS) {
-    HEX_GATHER
+    HEX_UNROLL_N(HEX_U_fct_cell1)
     for (int s = 0; s < n; ++s) {
       const V4 on = ld4(ot + g.coc[c * g.maxE + s] * S + k0);
 #pragma unroll
@@ -1506,7 +1514,7 @@ __global__ void HEX_VEC_BOUNDS kv_fct_cell1(HexGeo g, int nT, float step, const 
     s_out[j] = -rz.a[j] * (pos0(vr[j + 1]) - neg0(vr[j]));
   }
   const float ia = g.inv_area[c];
-  HEX_GATHER
+  HEX_UNROLL_N(HEX_U_fct_cell1)
   for (int s = 0; s < n; ++s) {
     const int2 sl = __ldg(g.slot + c * g.maxE + s);
     const int eo = slot_edge(sl.x);
@@ -1555,7 +1563,7 @@ __global__ void HEX_VEC_BOUNDS kv_fct_cell1(HexGeo g, int nT, float step, const 
 }
 
 // hexcore/transport.py:1919-2118: the limited antidiffusive edge flux.
-__global__ void __launch_bounds__(256, HEX_FCT_EDGE_MIN_BLOCKS) kv_fct_edge(HexGeo g, int nT, float step, const float* __restrict__ q_old, const float* __restrict__ hv,
+__global__ void __launch_bounds__(256, HEX_B_fct_edge) kv_fct_edge(HexGeo g, int nT, float step, const float* __restrict__ q_old, const float* __restrict__ hv,
                             const float* __restrict__ high_e, const float* __restrict__ scale_in,
                             const float* __restrict__ scale_out, float* __restrict__ hres_lim) {
   HEX_VEC_TRACER(g.nE, nT)
@@ -1581,7 +1589,7 @@ __global__ void __launch_bounds__(256, HEX_FCT_EDGE_MIN_BLOCKS) kv_fct_edge(HexG
 
 // hexcore/transport.py:1919-2118: limited update of the monotonic stage.
 // The vertical residual fluxes are those kv_fct_cell1 formed (vres).
-__global__ void HEX_VEC_BOUNDS kv_fct_cell2(HexGeo g, int nT, const float* __restrict__ vres,
+__global__ void __launch_bounds__(256, HEX_B_fct_cell2) kv_fct_cell2(HexGeo g, int nT, const float* __restrict__ vres,
                              const float* __restrict__ scale_in, const float* __restrict__ scale_out,
                              const float* __restrict__ mass_in, const float* __restrict__ hres_lim,
                              const float* __restrict__ target, float* __restrict__ q_out) {
@@ -1593,7 +1601,7 @@ __global__ void HEX_VEC_BOUNDS kv_fct_cell2(HexGeo g, int nT, const float* __res
   V4 mass = ld4(mass_in + toff + ii);
   const int n = g.deg[c];
   const float ia = g.inv_area[c];
-  HEX_GATHER
+  HEX_UNROLL_N(HEX_U_fct_cell2)
   for (int s = 0; s < n; ++s) {
     const int sl = __ldg(&g.slot[c * g.maxE + s].x);
     const float ts = -slot_sign(sl);
@@ -1695,7 +1703,7 @@ __device__ __forceinline__ float from_above(float a0) { return __shfl_down_sync(
 
 // hexcore/acoustic_v841.py:81 compute_vertical_implicit_coefficients_v841.
 #define HEX_VCOEFV_SMEM_ARRAYS 3
-__global__ void HEX_VEC_BOUNDS kv_vcoef(HexGeo g, float dts2, const float* __restrict__ exner, const float* __restrict__ theta,
+__global__ void __launch_bounds__(256, HEX_B_vcoef) kv_vcoef(HexGeo g, float dts2, const float* __restrict__ exner, const float* __restrict__ theta,
                          const float* __restrict__ rtp, const float* __restrict__ cqw,
                          const float* __restrict__ qtot, float* __restrict__ cofwr, float* __restrict__ cofwz,
                          float* __restrict__ coftz, float* __restrict__ cofwt, float* __restrict__ a_tri,
@@ -1821,7 +1829,7 @@ __global__ void HEX_VEC_BOUNDS kv_vcoef(HexGeo g, float dts2, const float* __res
 #ifndef HEX_AC_DSS_ZERO_SKIP
 #define HEX_AC_DSS_ZERO_SKIP 1
 #endif
-__global__ void HEX_VEC_BOUNDS kv_ac_cell(HexGeo g, int first, float dts, float dts2, const float* __restrict__ ru_p,
+__global__ void __launch_bounds__(256, HEX_B_ac_cell) kv_ac_cell(HexGeo g, int first, float dts, float dts2, const float* __restrict__ ru_p,
                            const float* __restrict__ theta_s, const float* __restrict__ tend_rho,
                            const float* __restrict__ tend_rt, const float* __restrict__ tend_rw,
                            const float* __restrict__ cofwr, const float* __restrict__ cofwz,
@@ -1873,7 +1881,7 @@ __global__ void HEX_VEC_BOUNDS kv_ac_cell(HexGeo g, int first, float dts, float 
     const int n = g.deg[c];
     const float ia = g.inv_area[c];
     const V4 tc = ld4(theta_s + ii);
-    HEX_GATHER
+    HEX_UNROLL_N(HEX_U_ac_cell)
     for (int s = 0; s < n; ++s) {
       const int2 sl = __ldg(g.slot + c * g.maxE + s);
       const float sdd = __ldg(g.sdv + c * g.maxE + s) * dts;  // (csign dts) dv

@@ -63,8 +63,8 @@ struct Launcher {
     signal(ctx.side_stream, st);
   }
   // entities per block for tpe threads per entity under the label's block size
-  int epb(const char* name, int tpe) const {
-    const int threads = ctx.threads_for(name);
+  int epb(const char* name, int tpe, long long n) const {
+    const int threads = ctx.threads_for(name, n * tpe);
     return tpe >= threads ? 1 : threads / tpe;
   }
   template <class K, class... A>
@@ -100,7 +100,7 @@ struct Launcher {
   void launch_impl(const char* name, int tpe, int n, int nz, size_t smem_per_entity, bool fold, K kernel,
                    A... args) {
     if (err != cudaSuccess || n <= 0 || nz <= 0) return;
-    const int e = epb(name, tpe);
+    const int e = epb(name, tpe, (long long)n * nz);
     const unsigned nb = (unsigned)((n + e - 1) / e);
     dim3 block(tpe, e), grid(fold ? nb * (unsigned)nz : nb, 1, fold ? 1 : nz);
     run(name, grid, block, smem_per_entity * e, kernel, args...);

@@ -354,7 +354,7 @@ int hexdyn_bind_state(HexDynHandle* h, const HexDynFields* fields, void* stream)
  * call's contents: each call clears the words it uses before the step, and
  * calls that overlap on the GPU (different streams, or concurrent host
  * threads) race on it, so issue them on one stream.  Kernels run on `stream`
- * alone (no second stream) at 256 threads per block (the handle's autotuned
+ * alone (no second stream) at the default block sizes (the handle's autotuned
  * block sizes are not used).  Reads the flag at the end like hexdyn_step
  * (synchronises `stream`). */
 int hexdyn_step_noalloc(HexDynHandle* h, const HexDynFields* in, const HexDynFields* out, void* stream,
