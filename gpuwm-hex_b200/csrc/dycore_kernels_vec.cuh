@@ -74,19 +74,31 @@
 #define HEX_B_mix_cell4 4
 #define HEX_U_mix_cell4 2
 
+// The chunk's first level.  Past this point the kernel's predecessor on the
+// stream is complete (a launch that may start early waits here, any other does
+// not), and the kernel's own successor may start its blocks, which then wait
+// for this one the same way.  Everything read before is the mesh's: every
+// address of a field is formed from the value returned here.
+__device__ __forceinline__ int chunk_level() {
+  int k0 = threadIdx.x * 4;
+  asm volatile("griddepcontrol.wait;\n\tgriddepcontrol.launch_dependents;" : "+r"(k0)::"memory");
+  __builtin_assume(k0 >= 0 && k0 < 1024);
+  return k0;
+}
+
 #define HEX_VEC_PARALLEL(n)                                \
-  const int k0 = threadIdx.x * 4;                          \
   const int ent = blockIdx.x * blockDim.y + threadIdx.y;   \
-  if (ent >= (n)) return;
+  if (ent >= (n)) return;                                  \
+  const int k0 = chunk_level();
 
 // Transport kernels over nT tracers: block b serves tracer b % nT of entity
 // block b / nT, so the nT tracers of an entity block run back to back and
 // share the reads of the velocities and stencil tables through L2.
 #define HEX_VEC_TRACER(n, nT)                                     \
-  const int k0 = threadIdx.x * 4;                                 \
   const int tr = blockIdx.x % (nT);                               \
   const int ent = (blockIdx.x / (nT)) * blockDim.y + threadIdx.y; \
-  if (ent >= (n)) return;
+  if (ent >= (n)) return;                                         \
+  const int k0 = chunk_level();
 
 #define HEX_PRAGMA(x) _Pragma(#x)
 #define HEX_UNROLL_N(n) HEX_PRAGMA(unroll n)
@@ -179,6 +191,46 @@ __device__ __forceinline__ Win win(const float* __restrict__ col, int k0, int S)
   return w;
 }
 
+// Neighbour loops.  What a loop reads of neighbour s is `load(s)`, what it does
+// with it `use(load(s), s)`, in slot order.  B = 0: a loop unrolled by U, for
+// grids of many waves, where resident warps hide the loads.  B > 0, for grids
+// that are resident at once, where the chain of dependent loads is the time:
+// `preload` issues the loads of the first B slots before any is used, those
+// past the entity's count too (their records are zero padding, and point at
+// the fields' first words; W is the records' slots per entity, at least 1).
+template <int B, class T>
+struct Pre {
+  T d[B > 0 ? B : 1];
+};
+template <int B, class Load>
+__device__ __forceinline__ auto preload(int W, Load load) -> Pre<B, decltype(load(0))> {
+  Pre<B, decltype(load(0))> p;
+  if constexpr (B > 0) {
+#pragma unroll
+    for (int i = 0; i < B; ++i) p.d[i] = load(i < W ? i : W - 1);
+  }
+  return p;
+}
+// the uses of the slots S0 .. n-1
+template <int B, int U, int S0 = 0, class T, class Load, class Use>
+__device__ __forceinline__ void gather(const Pre<B, T>& p, int n, Load load, Use use) {
+  if constexpr (B > 0) {
+#pragma unroll
+    for (int i = S0; i < B; ++i)
+      if (i < n) use(p.d[i], i);
+  }
+  constexpr int first = B > S0 ? B : S0;
+  if constexpr (B > 0) {
+#pragma unroll 1
+    for (int s = first; s < n; ++s) use(load(s), s);
+  } else {
+#pragma unroll U
+    for (int s = first; s < n; ++s) use(load(s), s);
+  }
+}
+// resident 256-thread blocks of a kernel: its own target when B = 0
+#define HEX_BOUNDS(B, target) __launch_bounds__(256, (B) ? 1 : (target))
+
 // End-of-step clamp of negative mixing ratios (hexcore/cuda_driver.py:5311,
 // `putmask(scalars, scalars < 0, 0)`): -0 and NaN compare false and stay.
 // blockIdx.z selects the scalar.
@@ -197,7 +249,8 @@ __global__ void __launch_bounds__(256, HEX_B_clamp_scalars) kv_clamp_scalars(Hex
 // qtot = sum of the scalars in scalar order, cqw = 1/(1 + (qtot(k) +
 // qtot(k-1))/2) above the surface, cqu = 1/(1 + sum of the two-cell means).
 // Scalars are stored [scalar][cell][S].
-__global__ void __launch_bounds__(256, HEX_B_moist_cell) kv_moist_cell(HexGeo g, const float* __restrict__ q, int nT,
+template <int B>
+__global__ void HEX_BOUNDS(B, HEX_B_moist_cell) kv_moist_cell(HexGeo g, const float* __restrict__ q, int nT,
                                              float* __restrict__ qtot, float* __restrict__ cqw) {
   HEX_VEC_PARALLEL(g.nC)
   const int c = ent, S = g.S;
@@ -205,13 +258,16 @@ __global__ void __launch_bounds__(256, HEX_B_moist_cell) kv_moist_cell(HexGeo g,
   const float* qc = q + c * S + k0;
   V4 acc = v4zero();
   float below = 0.0f;  // qtot at level k0 - 1
-  HEX_UNROLL_N(HEX_U_moist_cell)
-  for (int t = 0; t < nT; ++t) {
-    const V4 v = ld4(qc + t * tstride);
+  struct In {
+    V4 v;
+    float below;
+  };
+  const auto load = [&](int t) { return In{ld4(qc + t * tstride), k0 > 0 ? (qc - 1)[t * tstride] : 0.0f}; };
+  gather<B, HEX_U_moist_cell>(preload<B>(nT, load), nT, load, [&](const In& d, int) {
 #pragma unroll
-    for (int j = 0; j < 4; ++j) acc.a[j] = acc.a[j] + v.a[j];
-    if (k0 > 0) below = below + (qc - 1)[t * tstride];
-  }
+    for (int j = 0; j < 4; ++j) acc.a[j] = acc.a[j] + d.v.a[j];
+    if (k0 > 0) below = below + d.below;
+  });
   V4 cw;
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
@@ -222,7 +278,8 @@ __global__ void __launch_bounds__(256, HEX_B_moist_cell) kv_moist_cell(HexGeo g,
   st4m(cqw + c * S + k0, cw, k0, 0, g.L);
 }
 
-__global__ void __launch_bounds__(256, HEX_B_moist_edge) kv_moist_edge(HexGeo g, const float* __restrict__ q, int nT,
+template <int B>
+__global__ void HEX_BOUNDS(B, HEX_B_moist_edge) kv_moist_edge(HexGeo g, const float* __restrict__ q, int nT,
                                              float* __restrict__ cqu) {
   HEX_VEC_PARALLEL(g.nE)
   const int e = ent, S = g.S;
@@ -231,12 +288,14 @@ __global__ void __launch_bounds__(256, HEX_B_moist_edge) kv_moist_edge(HexGeo g,
   const float* q0 = q + ends.x + k0;
   const float* q1 = q + ends.y + k0;
   V4 acc = v4zero();
-  HEX_UNROLL_N(HEX_U_moist_edge)
-  for (int t = 0; t < nT; ++t) {
-    const V4 a = ld4(q0 + t * tstride), b = ld4(q1 + t * tstride);
+  struct In {
+    V4 a, b;
+  };
+  const auto load = [&](int t) { return In{ld4(q0 + t * tstride), ld4(q1 + t * tstride)}; };
+  gather<B, HEX_U_moist_edge>(preload<B>(nT, load), nT, load, [&](const In& d, int) {
 #pragma unroll
-    for (int j = 0; j < 4; ++j) acc.a[j] = acc.a[j] + 0.5f * (a.a[j] + b.a[j]);
-  }
+    for (int j = 0; j < 4; ++j) acc.a[j] = acc.a[j] + 0.5f * (d.a.a[j] + d.b.a[j]);
+  });
   V4 out;
 #pragma unroll
   for (int j = 0; j < 4; ++j) out.a[j] = 1.0f / (1.0f + acc.a[j]);
@@ -277,8 +336,8 @@ __global__ void __launch_bounds__(256, HEX_B_diag_vertex) kv_diag_vertex(HexGeo 
 
 // Cell kinetic energy (v8.4.1 kite blend 0.625) and, with APVM, cell PV;
 // DIV: also the divergence of u (the horizontal mixing's input).
-template <bool DIV>
-__global__ void __launch_bounds__(256, HEX_B_diag_cell) kv_diag_cell(HexGeo g, const float* __restrict__ u, const float* __restrict__ pv_vertex,
+template <bool DIV, int B>
+__global__ void HEX_BOUNDS(B, HEX_B_diag_cell) kv_diag_cell(HexGeo g, const float* __restrict__ u, const float* __restrict__ pv_vertex,
                              const float* __restrict__ ke_vertex, float* __restrict__ ke_out,
                              float* __restrict__ pv_cell, float* __restrict__ divergence) {
   HEX_VEC_PARALLEL(g.nC)
@@ -288,19 +347,32 @@ __global__ void __launch_bounds__(256, HEX_B_diag_cell) kv_diag_cell(HexGeo g, c
   const int2* slots = g.vslot + c * g.maxE;
   const int2* eslots = g.eslot + c * g.maxE;
   V4 ke = v4zero(), dv = v4zero();
-  HEX_UNROLL_N(HEX_U_diag_cell)
-  for (int s = 0; s < n; ++s) {
+  struct Edge {
+    float dd, sd;
+    V4 u;
+  };
+  struct Vertex {
+    float kite;
+    V4 ke, pv;
+  };
+  const auto edge = [&](int s) {
     const int2 r = __ldg(eslots + s);
-    const float dd = fbits(r.y);
-    const V4 ue = ld4(u + k0 + r.x);
+    return Edge{fbits(r.y), DIV ? __ldg(g.sdv + c * g.maxE + s) : 0.0f, ld4(u + k0 + r.x)};
+  };
+  const auto vertex = [&](int s) {
+    const int2 r = __ldg(slots + s);
+    return Vertex{fbits(r.y), ld4(ke_vertex + k0 + r.x), g.apvm_on ? ld4(pv_vertex + k0 + r.x) : v4zero()};
+  };
+  const auto edges = preload<B>(g.maxE, edge);
+  const auto vertices = preload<B>(g.maxE, vertex);
+  gather<B, HEX_U_diag_cell>(edges, n, edge, [&](const Edge& d, int) {
 #pragma unroll
-    for (int j = 0; j < 4; ++j) ke.a[j] = ke.a[j] + 0.25f * (dd * (ue.a[j] * ue.a[j]));
+    for (int j = 0; j < 4; ++j) ke.a[j] = ke.a[j] + 0.25f * (d.dd * (d.u.a[j] * d.u.a[j]));
     if (DIV) {
-      const float sd = __ldg(g.sdv + c * g.maxE + s);
 #pragma unroll
-      for (int j = 0; j < 4; ++j) dv.a[j] = dv.a[j] + sd * ue.a[j];
+      for (int j = 0; j < 4; ++j) dv.a[j] = dv.a[j] + d.sd * d.u.a[j];
     }
-  }
+  });
   if (DIV) {
 #pragma unroll
     for (int j = 0; j < 4; ++j) dv.a[j] = dv.a[j] * ia;
@@ -309,26 +381,22 @@ __global__ void __launch_bounds__(256, HEX_B_diag_cell) kv_diag_cell(HexGeo g, c
 #pragma unroll
   for (int j = 0; j < 4; ++j) ke.a[j] = ke.a[j] * ia * 0.625f;
   V4 pvc = v4zero();
-  HEX_UNROLL_N(HEX_U_diag_cell)
-  for (int s = 0; s < n; ++s) {
-    const int2 r = __ldg(slots + s);
-    const float kite = fbits(r.y);
-    const float kt = (1.0f - 0.625f) * kite;
-    const V4 kv = ld4(ke_vertex + k0 + r.x);
+  gather<B, HEX_U_diag_cell>(vertices, n, vertex, [&](const Vertex& d, int) {
+    const float kt = (1.0f - 0.625f) * d.kite;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) ke.a[j] = ke.a[j] + kt * kv.a[j] * ia;
+    for (int j = 0; j < 4; ++j) ke.a[j] = ke.a[j] + kt * d.ke.a[j] * ia;
     if (g.apvm_on) {
-      const V4 pv = ld4(pv_vertex + k0 + r.x);
 #pragma unroll
-      for (int j = 0; j < 4; ++j) pvc.a[j] = pvc.a[j] + kite * pv.a[j] * ia;
+      for (int j = 0; j < 4; ++j) pvc.a[j] = pvc.a[j] + d.kite * d.pv.a[j] * ia;
     }
-  }
+  });
   st4m(ke_out + c * S + k0, ke, k0, 0, g.L);
   if (g.apvm_on) st4m(pv_cell + c * S + k0, pvc, k0, 0, g.L);
 }
 
 // Tangential velocity (TRiSK weights) and edge PV with APVM upwinding.
-__global__ void __launch_bounds__(256, HEX_B_diag_edge) kv_diag_edge(HexGeo g, const float* __restrict__ u, const float* __restrict__ pv_vertex,
+template <int B>
+__global__ void HEX_BOUNDS(B, HEX_B_diag_edge) kv_diag_edge(HexGeo g, const float* __restrict__ u, const float* __restrict__ pv_vertex,
                              const float* __restrict__ pv_cell, float* __restrict__ v, float* __restrict__ pv_edge,
                              int recompute_v) {
   HEX_VEC_PARALLEL(g.nE)
@@ -338,20 +406,26 @@ __global__ void __launch_bounds__(256, HEX_B_diag_edge) kv_diag_edge(HexGeo g, c
     vt = v4zero();
     const int n = g.neoe[e];
     const int4* nbr = g.nbr + (size_t)e * g.nbrW;
-    HEX_UNROLL_N(HEX_U_diag_edge)
-    for (int s = 0; s + 1 < n; s += 2) {
-      const int4 r = __ldg(nbr + (s >> 1));
-      const V4 ua = ld4(u + k0 + r.x), ub = ld4(u + k0 + r.z);
+    struct Pair {
+      float wa, wb;
+      V4 a, b;
+    };
+    const auto load = [&](int i) {
+      const int4 r = __ldg(nbr + i);
+      return Pair{fbits(r.y), fbits(r.w), ld4(u + k0 + r.x), ld4(u + k0 + r.z)};
+    };
+    const auto add = [&](float w, const V4& x) {
 #pragma unroll
-      for (int j = 0; j < 4; ++j) vt.a[j] = vt.a[j] + fbits(r.y) * ua.a[j];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) vt.a[j] = vt.a[j] + fbits(r.w) * ub.a[j];
-    }
-    if (n & 1) {
+      for (int j = 0; j < 4; ++j) vt.a[j] = vt.a[j] + w * x.a[j];
+    };
+    // the last of an odd count is a pair's first half
+    gather<B, HEX_U_diag_edge>(preload<B>(g.nbrW, load), B ? (n + 1) >> 1 : n >> 1, load, [&](const Pair& d, int i) {
+      add(d.wa, d.a);
+      if (!B || 2 * i + 1 < n) add(d.wb, d.b);
+    });
+    if (!B && (n & 1)) {
       const int4 r = __ldg(nbr + (n >> 1));
-      const V4 un = ld4(u + k0 + r.x);
-#pragma unroll
-      for (int j = 0; j < 4; ++j) vt.a[j] = vt.a[j] + fbits(r.y) * un.a[j];
+      add(fbits(r.y), ld4(u + k0 + r.x));
     }
     st4m(v + e * S + k0, vt, k0, 0, g.L);
   } else {
@@ -411,16 +485,21 @@ __global__ void __launch_bounds__(256, HEX_B_euler_edge) kv_euler_edge(HexGeo g,
 }
 
 // hexcore/dynamics.py:86 mass_flux_divergence (stored inverse area), 4 levels.
+template <int B>
 __device__ __forceinline__ V4 mass_flux_div4(const HexGeo& g, const float* __restrict__ ru, int c, int k0) {
   V4 acc = v4zero();
   const int n = g.deg[c];
-  HEX_UNROLL_N(HEX_U_mass_flux)
-  for (int s = 0; s < n; ++s) {
-    const float sd = __ldg(g.sdv + c * g.maxE + s);
-    const V4 r = ld4(ru + k0 + __ldg(g.eslot + c * g.maxE + s).x);
+  struct In {
+    float sd;
+    V4 r;
+  };
+  const auto load = [&](int s) {
+    return In{__ldg(g.sdv + c * g.maxE + s), ld4(ru + k0 + __ldg(g.eslot + c * g.maxE + s).x)};
+  };
+  gather<B, HEX_U_mass_flux>(preload<B>(g.maxE, load), n, load, [&](const In& d, int) {
 #pragma unroll
-    for (int j = 0; j < 4; ++j) acc.a[j] = acc.a[j] + sd * r.a[j];
-  }
+    for (int j = 0; j < 4; ++j) acc.a[j] = acc.a[j] + d.sd * d.r.a[j];
+  });
   const float ia = g.inv_area[c];
 #pragma unroll
   for (int j = 0; j < 4; ++j) acc.a[j] = acc.a[j] * ia;
@@ -428,14 +507,15 @@ __device__ __forceinline__ V4 mass_flux_div4(const HexGeo& g, const float* __res
 }
 
 // hexcore/dynamics.py:122 density_tendency and hexcore/driver.py:2804 Euler w.
-__global__ void __launch_bounds__(256, HEX_B_euler_cell) kv_euler_cell(HexGeo g, const float* __restrict__ ru, const float* __restrict__ rw,
+template <int B>
+__global__ void HEX_BOUNDS(B, HEX_B_euler_cell) kv_euler_cell(HexGeo g, const float* __restrict__ ru, const float* __restrict__ rw,
                               const float* __restrict__ pp, const float* __restrict__ rp,
                               const float* __restrict__ qtot, const float* __restrict__ cqw,
                               float* __restrict__ tend_rho, float* __restrict__ euler_rw,
                               const float* __restrict__ phys_rho, float* __restrict__ tend_rho_dyn) {
   HEX_VEC_PARALLEL(g.nC)
   const int c = ent, S = g.S, L = g.L;
-  const V4 hd = mass_flux_div4(g, ru, c, k0);
+  const V4 hd = mass_flux_div4<B>(g, ru, c, k0);
   const Win rww = win<0, 1>(rw + c * S, k0, S);
   const Win ppw = win<1, 0>(pp + c * S, k0, S), rpw = win<1, 0>(rp + c * S, k0, S);
   const bool m = g.moist;
@@ -472,14 +552,16 @@ __global__ void __launch_bounds__(256, HEX_B_euler_cell) kv_euler_cell(HexGeo g,
 
 // ------------------------------------------------- stage tendencies
 // hexcore/dynamics.py:86 mass_flux_divergence of the stage rho*u.
-__global__ void __launch_bounds__(256, HEX_B_hdiv) kv_hdiv(HexGeo g, const float* __restrict__ ru, float* __restrict__ hdiv) {
+template <int B>
+__global__ void HEX_BOUNDS(B, HEX_B_hdiv) kv_hdiv(HexGeo g, const float* __restrict__ ru, float* __restrict__ hdiv) {
   HEX_VEC_PARALLEL(g.nC)
-  st4m(hdiv + ent * g.S + k0, mass_flux_div4(g, ru, ent, k0), k0, 0, g.L);
+  st4m(hdiv + ent * g.S + k0, mass_flux_div4<B>(g, ru, ent, k0), k0, 0, g.L);
 }
 
 // Third-order edge values of theta_m (levels) and w (interfaces):
 // hexcore/driver.py:1023-1034 and :1159-1172.
-__global__ void __launch_bounds__(256, HEX_B_edge_adv) kv_edge_adv(HexGeo g, const float* __restrict__ ru, const float* __restrict__ theta,
+template <int B>
+__global__ void HEX_BOUNDS(B, HEX_B_edge_adv) kv_edge_adv(HexGeo g, const float* __restrict__ ru, const float* __restrict__ theta,
                             const float* __restrict__ w, float* __restrict__ edge_theta,
                             float* __restrict__ edge_w) {
   HEX_VEC_PARALLEL(g.nE)
@@ -487,6 +569,15 @@ __global__ void __launch_bounds__(256, HEX_B_edge_adv) kv_edge_adv(HexGeo g, con
   const int n = g.n_adv[e];
   const int* off = g.adv_off + (size_t)e * g.advW;
   const float2* pm = g.adv_pm + (size_t)e * g.advW;
+  struct In {
+    float2 c;
+    V4 th, w;
+  };
+  const auto load = [&](int s) {
+    const int o = __ldg(off + s);
+    return In{__ldg(pm + s), ld4(theta + k0 + o), ld4(w + k0 + o)};
+  };
+  const auto cells = preload<B>(g.advW, load);
   const V4 r = ld4(ru + e * S + k0);
   const float rm = k0 > 0 ? ru[e * S + k0 - 1] : 0.0f;
   const V4 fm = ld4(g.fzm + k0), fp = ld4(g.fzp + k0);
@@ -500,17 +591,13 @@ __global__ void __launch_bounds__(256, HEX_B_edge_adv) kv_edge_adv(HexGeo g, con
     nw[j] = signbit(fm.a[j] * r.a[j] + fp.a[j] * rprev);
   }
   V4 at = v4zero(), aw = v4zero();
-  HEX_UNROLL_N(HEX_U_edge_adv)
-  for (int s = 0; s < n; ++s) {
-    const int o = __ldg(off + s);
-    const float2 c = __ldg(pm + s);
-    const V4 th = ld4(theta + k0 + o), wv = ld4(w + k0 + o);
+  gather<B, HEX_U_edge_adv>(cells, n, load, [&](const In& d, int) {
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      at.a[j] = at.a[j] + (nt[j] ? c.y : c.x) * th.a[j];
-      aw.a[j] = aw.a[j] + (nw[j] ? c.y : c.x) * wv.a[j];
+      at.a[j] = at.a[j] + (nt[j] ? d.c.y : d.c.x) * d.th.a[j];
+      aw.a[j] = aw.a[j] + (nw[j] ? d.c.y : d.c.x) * d.w.a[j];
     }
-  }
+  });
   st4m(edge_theta + e * S + k0, at, k0, 0, g.L);
   st4m(edge_w + e * S + k0, aw, k0, 1, g.L);
 }
@@ -550,8 +637,8 @@ __device__ __forceinline__ void column_ends(int k0, int L, float (&f)[5], F edge
 // tend_ru: vertical transport + hexcore/dynamics_v841.py:121 momentum + saved Euler.
 // RAYLEIGH: the upper Rayleigh damping of u is compiled in (an instance
 // without it keeps the common path's registers).
-template <bool RAYLEIGH>
-__global__ void __launch_bounds__(256, HEX_B_tend_u) kv_tend_u(HexGeo g, const float* __restrict__ u, const float* __restrict__ rw,
+template <bool RAYLEIGH, int B>
+__global__ void HEX_BOUNDS(B, HEX_B_tend_u) kv_tend_u(HexGeo g, const float* __restrict__ u, const float* __restrict__ rw,
                           const float* __restrict__ rho, const float* __restrict__ pv_edge,
                           const float* __restrict__ ke, const float* __restrict__ hdiv,
                           const float* __restrict__ euler_ru, float* __restrict__ tend_ru,
@@ -571,15 +658,21 @@ __global__ void __launch_bounds__(256, HEX_B_tend_u) kv_tend_u(HexGeo g, const f
       q.a[j] = q.a[j] + w * un.a[j] * work_pv;
     }
   };
-  HEX_UNROLL_N(HEX_U_tend_u)
-  for (int s = 0; s + 1 < n; s += 2) {
-    const int4 r = __ldg(nbr + (s >> 1));
-    const V4 ua = ld4(u + k0 + r.x), pa = ld4(pv_edge + k0 + r.x);
-    const V4 ub = ld4(u + k0 + r.z), pb = ld4(pv_edge + k0 + r.z);
-    coriolis(ua, pa, fbits(r.y));
-    coriolis(ub, pb, fbits(r.w));
-  }
-  if (n & 1) {
+  struct Pair {
+    float wa, wb;
+    V4 ua, pa, ub, pb;
+  };
+  const auto load = [&](int i) {
+    const int4 r = __ldg(nbr + i);
+    return Pair{fbits(r.y),          fbits(r.w),          ld4(u + k0 + r.x), ld4(pv_edge + k0 + r.x),
+                ld4(u + k0 + r.z), ld4(pv_edge + k0 + r.z)};
+  };
+  // the last of an odd count is a pair's first half
+  gather<B, HEX_U_tend_u>(preload<B>(g.nbrW, load), B ? (n + 1) >> 1 : n >> 1, load, [&](const Pair& d, int i) {
+    coriolis(d.ua, d.pa, d.wa);
+    if (!B || 2 * i + 1 < n) coriolis(d.ub, d.pb, d.wb);
+  });
+  if (!B && (n & 1)) {
     const int4 r = __ldg(nbr + (n >> 1));
     coriolis(ld4(u + k0 + r.x), ld4(pv_edge + k0 + r.x), fbits(r.y));
   }
@@ -657,7 +750,8 @@ __global__ void __launch_bounds__(256, HEX_B_tend_u) kv_tend_u(HexGeo g, const f
 
 // tend_rt (hexcore/driver.py:933), tend_rw (:1081) + Euler w, then
 // hexcore/acoustic.py:246 convert_w_tendency_to_omega.
-__global__ void __launch_bounds__(256, HEX_B_tend_cell) kv_tend_cell(HexGeo g, const float* __restrict__ ru, const float* __restrict__ ru_s,
+template <int B>
+__global__ void HEX_BOUNDS(B, HEX_B_tend_cell) kv_tend_cell(HexGeo g, const float* __restrict__ ru, const float* __restrict__ ru_s,
                              const float* __restrict__ rw, const float* __restrict__ rws,
                              const float* __restrict__ theta, const float* __restrict__ theta_s,
                              const float* __restrict__ w, const float* __restrict__ edge_theta,
@@ -673,40 +767,60 @@ __global__ void __launch_bounds__(256, HEX_B_tend_cell) kv_tend_cell(HexGeo g, c
   const V4 fm = ld4(g.fzm + k0), fp = ld4(g.fzp + k0);
   // horizontal parts: rho-theta flux divergence, RK>1 correction, w flux
   V4 res = v4zero(), hres = v4zero();
-  HEX_UNROLL_N(HEX_U_tend_cell)
-  for (int s = 0; s < n; ++s) {
+  struct Flux {
+    float sg, rm;
+    V4 r, et, ew;
+  };
+  const auto flux = [&](int s) {
     const int sl = __ldg(&slots[s].x), eo = slot_edge(sl);
-    const float sg = slot_sign(sl);
-    const V4 r = ld4(ru + k0 + eo), et = ld4(edge_theta + k0 + eo), ew = ld4(edge_w + k0 + eo);
-    const float rm = k0 > 0 ? (ru + k0 - 1)[eo] : 0.0f;
+    return Flux{slot_sign(sl), k0 > 0 ? (ru + k0 - 1)[eo] : 0.0f, ld4(ru + k0 + eo), ld4(edge_theta + k0 + eo),
+                ld4(edge_w + k0 + eo)};
+  };
+  struct Corr {
+    float dvs;
+    V4 r, rs, tn;
+  };
+  const auto corr = [&](int s) {
+    const int2 sl = __ldg(slots + s);
+    const int eo = slot_edge(sl.x);
+    return Corr{__ldg(g.sdv + c * g.maxE + s), ld4(ru + k0 + eo), ld4(ru_s + k0 + eo), ld4(theta_s + k0 + sl.y)};
+  };
+  const auto fluxes = preload<B>(g.maxE, flux);
+  const auto corrs = preload<B>(g.maxE, corr);
+  gather<B, HEX_U_tend_cell>(fluxes, n, flux, [&](const Flux& d, int) {
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       // sg is +-1: sg x y rounds once, and adding or subtracting it in one
       // fused operation rounds as the separate sum does
-      res.a[j] = fma_sign(-sg, r.a[j] * et.a[j], res.a[j]);
-      const float rprev = j == 0 ? rm : r.a[j - 1];
-      const float rui = fm.a[j] * r.a[j] + fp.a[j] * rprev;
-      hres.a[j] = fma_sign(-sg, rui * ew.a[j], hres.a[j]);
+      res.a[j] = fma_sign(-d.sg, d.r.a[j] * d.et.a[j], res.a[j]);
+      const float rprev = j == 0 ? d.rm : d.r.a[j - 1];
+      const float rui = fm.a[j] * d.r.a[j] + fp.a[j] * rprev;
+      hres.a[j] = fma_sign(-d.sg, rui * d.ew.a[j], hres.a[j]);
     }
-  }
+  });
   if (rk_step > 1) {
     const V4 tc = ld4(theta_s + c * S + k0);
-    HEX_UNROLL_N(HEX_U_tend_cell)
-    for (int s = 0; s < n; ++s) {
-      const int2 sl = __ldg(slots + s);
-      const int eo = slot_edge(sl.x);
-      const float dvs = __ldg(g.sdv + c * g.maxE + s);
-      const V4 r = ld4(ru + k0 + eo), rs = ld4(ru_s + k0 + eo);
-      const V4 tn = ld4(theta_s + k0 + sl.y);
+    gather<B, HEX_U_tend_cell>(corrs, n, corr, [&](const Corr& d, int) {
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         // theta_s[e1] + theta_s[e0] with this cell as one operand (IEEE
         // addition commutes, so the operand order changes no bit)
-        const float corr = dvs * (rs.a[j] - r.a[j]) * 0.5f * (tn.a[j] + tc.a[j]);
-        res.a[j] = res.a[j] - corr;
+        const float x = d.dvs * (d.rs.a[j] - d.r.a[j]) * 0.5f * (d.tn.a[j] + tc.a[j]);
+        res.a[j] = res.a[j] - x;
       }
-    }
+    });
   }
+  struct Omega {
+    float sg, tm;
+    V4 t, zb, zb3;
+  };
+  const auto omega = [&](int s) {
+    const int sl = __ldg(&slots[s].x), eo = slot_edge(sl);
+    const int zi = (c * g.maxE + s) * S + k0;
+    return Omega{slot_sign(sl), k0 > 0 ? (tend_ru + k0 - 1)[eo] : 0.0f, ld4(tend_ru + k0 + eo), ld4(g.zb + zi),
+                 ld4(g.zb3 + zi)};
+  };
+  const auto omegas = preload<B>(g.maxE, omega);
   const Win th = win<2, 2>(theta + c * S, k0, S), ths = win<1, 1>(theta_s + c * S, k0, S);
   const Win rww = win<1, 1>(rw + c * S, k0, S), rwsw = win<0, 1>(rws + c * S, k0, S);
   const Win ww = win<2, 2>(w + c * S, k0, S), zzw = win<1, 0>(g.zz + c * S, k0, S);
@@ -740,22 +854,15 @@ __global__ void __launch_bounds__(256, HEX_B_tend_cell) kv_tend_cell(HexGeo g, c
     trw.a[j] = rsw + er.a[j];
   }
   // omega conversion (interfaces 1..L-1)
-  HEX_UNROLL_N(HEX_U_tend_cell)
-  for (int s = 0; s < n; ++s) {
-    const int sl = __ldg(&slots[s].x), eo = slot_edge(sl);
-    const float sg = slot_sign(sl);
-    const V4 t = ld4(tend_ru + k0 + eo);
-    const float tm = k0 > 0 ? (tend_ru + k0 - 1)[eo] : 0.0f;
-    const int zi = (c * g.maxE + s) * S + k0;
-    const V4 zb = ld4(g.zb + zi), zb3 = ld4(g.zb3 + zi);
+  gather<B, HEX_U_tend_cell>(omegas, n, omega, [&](const Omega& d, int) {
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      const float tprev = j == 0 ? tm : t.a[j - 1];
-      const float flux = fm.a[j] * t.a[j] + fp.a[j] * tprev;
-      const float zt = fma_sign(copysignf(1.0f, t.a[j]), zb3.a[j], zb.a[j]);
-      trw.a[j] = fma_sign(-sg, zt * flux, trw.a[j]);
+      const float tprev = j == 0 ? d.tm : d.t.a[j - 1];
+      const float f = fm.a[j] * d.t.a[j] + fp.a[j] * tprev;
+      const float zt = fma_sign(copysignf(1.0f, d.t.a[j]), d.zb3.a[j], d.zb.a[j]);
+      trw.a[j] = fma_sign(-d.sg, zt * f, trw.a[j]);
     }
-  }
+  });
   // levels 0 and L hold 0 + the saved Euler term (every level ran the sums
   // above: no branch splits a warp between its columns' ends and insides)
 #pragma unroll
@@ -1140,7 +1247,8 @@ __global__ void __launch_bounds__(256, HEX_B_recover_edge) kv_recover_edge(HexGe
 // hexcore/driver.py:3166-3292 stage recovery, cell part: candidate state,
 // rw end conditions, theta_m, Exner and p' at stage 3, w from
 // hexcore/terrain.py:491 recover_velocities, and the split w-flux average.
-__global__ void __launch_bounds__(256, HEX_B_recover_cell) kv_recover_cell(HexGeo g, int stage3, const float* __restrict__ rp_s,
+template <int B>
+__global__ void HEX_BOUNDS(B, HEX_B_recover_cell) kv_recover_cell(HexGeo g, int stage3, const float* __restrict__ rp_s,
                                 const float* __restrict__ rtp_s, const float* __restrict__ rw_s,
                                 const float* __restrict__ rho_pp, const float* __restrict__ rtpp,
                                 const float* __restrict__ rw_p, const float* __restrict__ ww_avg,
@@ -1150,6 +1258,17 @@ __global__ void __launch_bounds__(256, HEX_B_recover_cell) kv_recover_cell(HexGe
   HEX_VEC_PARALLEL(g.nC)
   const int c = ent, S = g.S, L = g.L;
   const int ii = c * S + k0;
+  struct In {
+    float sign, sd, rm;
+    V4 r, zb, zb3;
+  };
+  const auto load = [&](int s) {
+    const int sl = __ldg(&g.slot[c * g.maxE + s].x), eo = slot_edge(sl);
+    const int zi = (c * g.maxE + s) * S + k0;
+    return In{slot_sign(sl),       __ldg(g.sdv + c * g.maxE + s), k0 > 0 ? (ru_new + k0 - 1)[eo] : 0.0f,
+              ld4(ru_new + k0 + eo), ld4(g.zb + zi),              ld4(g.zb3 + zi)};
+  };
+  const auto edges = preload<B>(g.maxE, load);
   // candidate density at the levels k0-1 .. k0+3 (recomputed, not read back)
   const Win rpw = win<1, 0>(rp_s + c * S, k0, S), ppw = win<1, 0>(rho_pp + c * S, k0, S);
   const Win rbw = win<1, 0>(g.rho_base + c * S, k0, S);
@@ -1221,28 +1340,21 @@ __global__ void __launch_bounds__(256, HEX_B_recover_cell) kv_recover_cell(HexGe
   // the next stage's mass-flux divergence of ru_new (mass_flux_div4, the
   // same operands in the same order) accumulates in the same edge loop
   V4 hd = v4zero();
-  HEX_UNROLL_N(HEX_U_recover_cell)
-  for (int s = 0; s < n; ++s) {
-    const int sl = __ldg(&g.slot[c * g.maxE + s].x), eo = slot_edge(sl);
-    const float sign = slot_sign(sl), sd = __ldg(g.sdv + c * g.maxE + s);
-    const V4 r = ld4(ru_new + k0 + eo);
+  gather<B, HEX_U_recover_cell>(edges, n, load, [&](const In& d, int) {
 #pragma unroll
-    for (int j = 0; j < 4; ++j) hd.a[j] = hd.a[j] + sd * r.a[j];
-    const float rm = k0 > 0 ? (ru_new + k0 - 1)[eo] : 0.0f;
-    const int zi = (c * g.maxE + s) * S + k0;
-    const V4 zb = ld4(g.zb + zi), zb3 = ld4(g.zb3 + zi);
+    for (int j = 0; j < 4; ++j) hd.a[j] = hd.a[j] + d.sd * d.r.a[j];
     if (bottom) {
-      const float flux = g.cf1 * r.a[0] + g.cf2 * r.a[1] + g.cf3 * r.a[2];
-      bacc = bacc + sign * (zb.a[0] + copysignf(1.0f, flux) * zb3.a[0]) * flux;
+      const float flux = g.cf1 * d.r.a[0] + g.cf2 * d.r.a[1] + g.cf3 * d.r.a[2];
+      bacc = bacc + d.sign * (d.zb.a[0] + copysignf(1.0f, flux) * d.zb3.a[0]) * flux;
     }
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      const float rprev = j == 0 ? rm : r.a[j - 1];
-      const float flux = fm.a[j] * r.a[j] + fp.a[j] * rprev;
-      const float zt = fma_sign(copysignf(1.0f, flux), zb3.a[j], zb.a[j]);
-      acc[j] = fma_sign(sign, zt * flux, acc[j]);
+      const float rprev = j == 0 ? d.rm : d.r.a[j - 1];
+      const float flux = fm.a[j] * d.r.a[j] + fp.a[j] * rprev;
+      const float zt = fma_sign(copysignf(1.0f, flux), d.zb3.a[j], d.zb.a[j]);
+      acc[j] = fma_sign(d.sign, zt * flux, acc[j]);
     }
-  }
+  });
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
     const int k = k0 + j;
@@ -1292,7 +1404,8 @@ __global__ void __launch_bounds__(256, HEX_B_recover_cell) kv_recover_cell(HexGe
 #ifndef HEX_TR_GROUP
 #define HEX_TR_GROUP 3
 #endif
-__global__ void __launch_bounds__(256, HEX_B_tr_edge) kv_tr_edge(HexGeo g, int nT, int mono, const float* __restrict__ q, const float* __restrict__ hv,
+template <int B>
+__global__ void HEX_BOUNDS(B, HEX_B_tr_edge) kv_tr_edge(HexGeo g, int nT, int mono, const float* __restrict__ q, const float* __restrict__ hv,
                            float* __restrict__ out) {
   HEX_VEC_TRACER(g.nE, (nT + HEX_TR_GROUP - 1) / HEX_TR_GROUP)
   constexpr int TG = HEX_TR_GROUP;
@@ -1303,39 +1416,47 @@ __global__ void __launch_bounds__(256, HEX_B_tr_edge) kv_tr_edge(HexGeo g, int n
   const int n = g.n_adv[e];
   const int* off = g.adv_off + (size_t)e * g.advW;
   const float2* pm = g.adv_pm + (size_t)e * g.advW;
+  struct In {
+    float2 c;
+    V4 q[TG];
+  };
+  const auto load = [&](int s) {
+    In d;
+    const float* qc = qg + __ldg(off + s);
+    d.c = __ldg(pm + s);
+#pragma unroll
+    for (int t = 0; t < TG; ++t)
+      if (t0 + t < nT) d.q[t] = ld4(qc + t * tstride);
+    return d;
+  };
+  const auto cells = preload<B>(g.advW, load);
   const V4 vel = ld4(hv + e * S + k0);
   // A + (coef3 sign(vel)) B is one of the record's two sums (see kv_edge_adv)
   bool neg[4];
 #pragma unroll
   for (int j = 0; j < 4; ++j) neg[j] = signbit(vel.a[j]);
-#define HEX_TR_WEIGHTS(s_)                                   \
-  const float* qc = qg + __ldg(off + (s_));                  \
-  const float2 c = __ldg(pm + (s_));                         \
-  float w[4];                                                \
-  _Pragma("unroll") for (int j = 0; j < 4; ++j) w[j] = neg[j] ? c.y : c.x;
   V4 res[TG];
   if (mono && n == 10) {
-    {
-      HEX_TR_WEIGHTS(0)
+    const auto first = [&](const In& d) {
 #pragma unroll
       for (int t = 0; t < TG; ++t)
         if (t0 + t < nT) {
-          const V4 qv = ld4(qc + t * tstride);
 #pragma unroll
-          for (int j = 0; j < 4; ++j) res[t].a[j] = w[j] * qv.a[j];
+          for (int j = 0; j < 4; ++j) res[t].a[j] = (neg[j] ? d.c.y : d.c.x) * d.q[t].a[j];
         }
-    }
-    HEX_UNROLL_N(HEX_U_tr_edge)
-    for (int s = 1; s < 10; ++s) {
-      HEX_TR_WEIGHTS(s)
+    };
+    if constexpr (B > 0)
+      first(cells.d[0]);
+    else
+      first(load(0));
+    gather<B, HEX_U_tr_edge, 1>(cells, 10, load, [&](const In& d, int) {
 #pragma unroll
       for (int t = 0; t < TG; ++t)
         if (t0 + t < nT) {
-          const V4 qv = ld4(qc + t * tstride);
 #pragma unroll
-          for (int j = 0; j < 4; ++j) res[t].a[j] = res[t].a[j] + w[j] * qv.a[j];
+          for (int j = 0; j < 4; ++j) res[t].a[j] = res[t].a[j] + (neg[j] ? d.c.y : d.c.x) * d.q[t].a[j];
         }
-    }
+    });
 #pragma unroll
     for (int t = 0; t < TG; ++t)
 #pragma unroll
@@ -1343,25 +1464,24 @@ __global__ void __launch_bounds__(256, HEX_B_tr_edge) kv_tr_edge(HexGeo g, int n
   } else {
 #pragma unroll
     for (int t = 0; t < TG; ++t) res[t] = v4zero();
-    HEX_UNROLL_N(HEX_U_tr_edge)
-    for (int s = 0; s < n; ++s) {
-      HEX_TR_WEIGHTS(s)
+    gather<B, HEX_U_tr_edge>(cells, n, load, [&](const In& d, int) {
+      float w[4];
 #pragma unroll
-      for (int j = 0; j < 4; ++j)
+      for (int j = 0; j < 4; ++j) {
+        w[j] = neg[j] ? d.c.y : d.c.x;
         if (mono) w[j] = vel.a[j] * w[j];
+      }
 #pragma unroll
       for (int t = 0; t < TG; ++t)
         if (t0 + t < nT) {
-          const V4 qv = ld4(qc + t * tstride);
 #pragma unroll
-          for (int j = 0; j < 4; ++j) res[t].a[j] = res[t].a[j] + w[j] * qv.a[j];
+          for (int j = 0; j < 4; ++j) res[t].a[j] = res[t].a[j] + w[j] * d.q[t].a[j];
         }
-    }
+    });
   }
 #pragma unroll
   for (int t = 0; t < TG; ++t)
     if (t0 + t < nT) st4m(out + (size_t)(t0 + t) * g.nE * S + e * S + k0, res[t], k0, 0, g.L);
-#undef HEX_TR_WEIGHTS
 }
 
 // transport vertical fluxes at the interfaces k0 .. k0+4 (hexcore/transport.py:1389).
@@ -1372,7 +1492,8 @@ __device__ __forceinline__ void tr_vflux_chunk(const HexGeo& g, const Win& q, co
 }
 
 // hexcore/transport.py:1649 advance_scalars (RK1/RK2 of split transport).
-__global__ void __launch_bounds__(256, HEX_B_tr_std) kv_tr_std(HexGeo g, int nT, float step, float wn, const float* __restrict__ q_old,
+template <int B>
+__global__ void HEX_BOUNDS(B, HEX_B_tr_std) kv_tr_std(HexGeo g, int nT, float step, float wn, const float* __restrict__ q_old,
                           const float* __restrict__ q_stage, const float* __restrict__ rho_old,
                           const float* __restrict__ rho_new, const float* __restrict__ hv,
                           const float* __restrict__ ww, const float* __restrict__ edge_q,
@@ -1384,14 +1505,18 @@ __global__ void __launch_bounds__(256, HEX_B_tr_std) kv_tr_std(HexGeo g, int nT,
   const float* ev = edge_q + (size_t)tr * g.nE * S;
   const int n = g.deg[c];
   V4 t = v4zero();
-  HEX_UNROLL_N(HEX_U_tr_std)
-  for (int s = 0; s < n; ++s) {
+  struct In {
+    float ts;
+    V4 h, x;
+  };
+  const auto load = [&](int s) {
     const int sl = __ldg(&g.slot[c * g.maxE + s].x), eo = slot_edge(sl);
-    const float ts = -slot_sign(sl);
-    const V4 h = ld4(hv + k0 + eo), x = ld4(ev + k0 + eo);
+    return In{-slot_sign(sl), ld4(hv + k0 + eo), ld4(ev + k0 + eo)};
+  };
+  gather<B, HEX_U_tr_std>(preload<B>(g.maxE, load), n, load, [&](const In& d, int) {
 #pragma unroll
-    for (int j = 0; j < 4; ++j) t.a[j] = fma_sign(ts, h.a[j] * x.a[j], t.a[j]);
-  }
+    for (int j = 0; j < 4; ++j) t.a[j] = fma_sign(d.ts, d.h.a[j] * d.x.a[j], t.a[j]);
+  });
   const float ia = g.inv_area[c];
   const Win qw = win<2, 2>(q_stage + toff + c * S, k0, S), www = win<0, 1>(ww + c * S, k0, S);
   const V4 ro = ld4(rho_old + ii), rn = ld4(rho_new + ii), qo = ld4(q_old + toff + ii);
@@ -1411,7 +1536,8 @@ __global__ void __launch_bounds__(256, HEX_B_tr_std) kv_tr_std(HexGeo g, int nT,
 }
 
 // hexcore/transport.py:1887-1906 split-transport target density.
-__global__ void __launch_bounds__(256, HEX_B_fct_target) kv_fct_target(HexGeo g, float step, const float* __restrict__ rho_old,
+template <int B>
+__global__ void HEX_BOUNDS(B, HEX_B_fct_target) kv_fct_target(HexGeo g, float step, const float* __restrict__ rho_old,
                               const float* __restrict__ hv, const float* __restrict__ ww,
                               float* __restrict__ target, int* flag) {
   HEX_VEC_PARALLEL(g.nC)
@@ -1420,13 +1546,18 @@ __global__ void __launch_bounds__(256, HEX_B_fct_target) kv_fct_target(HexGeo g,
   const int n = g.deg[c];
   const float ia = g.inv_area[c];
   V4 hd = v4zero();
-  HEX_UNROLL_N(HEX_U_fct_target)
-  for (int s = 0; s < n; ++s) {
-    const float tdv = -__ldg(g.sdv + c * g.maxE + s);  // (ts h) dv = h (ts dv), ts = -csign exact
-    const V4 h = ld4(hv + k0 + __ldg(g.eslot + c * g.maxE + s).x);
+  struct In {
+    float tdv;
+    V4 h;
+  };
+  const auto load = [&](int s) {
+    return In{-__ldg(g.sdv + c * g.maxE + s),  // (ts h) dv = h (ts dv), ts = -csign exact
+              ld4(hv + k0 + __ldg(g.eslot + c * g.maxE + s).x)};
+  };
+  gather<B, HEX_U_fct_target>(preload<B>(g.maxE, load), n, load, [&](const In& d, int) {
 #pragma unroll
-    for (int j = 0; j < 4; ++j) hd.a[j] = hd.a[j] + h.a[j] * tdv * ia;
-  }
+    for (int j = 0; j < 4; ++j) hd.a[j] = hd.a[j] + d.h.a[j] * d.tdv * ia;
+  });
   const Win www = win<0, 1>(ww + c * S, k0, S);
   const V4 ro = ld4(rho_old + ii);
   V4 td;
@@ -1452,8 +1583,8 @@ __device__ __forceinline__ float fct_fcol_win(float step, const Win& o, const Wi
 // slot s takes its two cell values from this column and the neighbour column
 // the bounds already load; the min/max over neighbours and the mass sums
 // still run in slot order, so the words are those of the two-loop form.
-template <bool ACROSS>
-__global__ void __launch_bounds__(256, HEX_B_fct_cell1) kv_fct_cell1(HexGeo g, int nT, float step, const float* __restrict__ q_old,
+template <bool ACROSS, int B>
+__global__ void HEX_BOUNDS(B, HEX_B_fct_cell1) kv_fct_cell1(HexGeo g, int nT, float step, const float* __restrict__ q_old,
                              const float* __restrict__ q_stage, const float* __restrict__ rho_old,
                              const float* __restrict__ hv, const float* __restrict__ ww,
                              const float* __restrict__ high_e, const float* __restrict__ target,
@@ -1465,6 +1596,24 @@ __global__ void __launch_bounds__(256, HEX_B_fct_cell1) kv_fct_cell1(HexGeo g, i
   const size_t toff = (size_t)tr * g.nC * S;
   const float* ot = q_old + toff;
   const float* he = high_e + (size_t)tr * g.nE * S;
+  struct In {
+    float cs, sd;
+    V4 vel, h, o0, o1;  // ACROSS: o0 is the cell across, o1 unused
+  };
+  const auto load = [&](int s) {
+    const int2 sl = __ldg(g.slot + c * g.maxE + s);
+    const int eo = slot_edge(sl.x);
+    In d{slot_sign(sl.x), __ldg(g.sdv + c * g.maxE + s), ld4(hv + k0 + eo), ld4(he + k0 + eo)};
+    if (ACROSS) {
+      d.o0 = ld4(ot + k0 + sl.y);
+    } else {
+      const int2 ends = __ldg(g.ends + g.eoc[c * g.maxE + s]);
+      d.o0 = ld4(ot + k0 + ends.x);
+      d.o1 = ld4(ot + k0 + ends.y);
+    }
+    return d;
+  };
+  const auto edges = preload<B>(g.maxE, load);
   const Win ow = win<1, 1>(ot + c * S, k0, S), qw = win<2, 2>(q_stage + toff + c * S, k0, S);
   const Win www = win<0, 1>(ww + c * S, k0, S);
   float mn[4], mx[4];
@@ -1514,18 +1663,14 @@ __global__ void __launch_bounds__(256, HEX_B_fct_cell1) kv_fct_cell1(HexGeo g, i
     s_out[j] = -rz.a[j] * (pos0(vr[j + 1]) - neg0(vr[j]));
   }
   const float ia = g.inv_area[c];
-  HEX_UNROLL_N(HEX_U_fct_cell1)
-  for (int s = 0; s < n; ++s) {
-    const int2 sl = __ldg(g.slot + c * g.maxE + s);
-    const int eo = slot_edge(sl.x);
-    const float cs = slot_sign(sl.x);
+  gather<B, HEX_U_fct_cell1>(edges, n, load, [&](const In& d, int) {
+    const float cs = d.cs;
     const float ts = -cs;
-    const float dvs = cs * __ldg(g.sdv + c * g.maxE + s) * step;  // dv step
-    const V4 vel = ld4(hv + k0 + eo), h = ld4(he + k0 + eo);
-    V4 o0, o1;
+    const float dvs = cs * d.sd * step;  // dv step
+    V4 o0 = d.o0, o1 = d.o1;
     if (ACROSS) {
       // csign > 0: this cell is the edge's first cell
-      const V4 on = ld4(ot + k0 + sl.y);
+      const V4 on = d.o0;
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         mn[j] = pymin(mn[j], on.a[j] + 0.0f);
@@ -1533,21 +1678,17 @@ __global__ void __launch_bounds__(256, HEX_B_fct_cell1) kv_fct_cell1(HexGeo g, i
         o0.a[j] = cs > 0.0f ? ow(j) : on.a[j];
         o1.a[j] = cs > 0.0f ? on.a[j] : ow(j);
       }
-    } else {
-      const int2 ends = __ldg(g.ends + g.eoc[c * g.maxE + s]);
-      o0 = ld4(ot + k0 + ends.x);
-      o1 = ld4(ot + k0 + ends.y);
     }
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      const float upw = dvs * (pos0(vel.a[j]) * (o0.a[j] + 0.0f) + neg0(vel.a[j]) * (o1.a[j] + 0.0f));
+      const float upw = dvs * (pos0(d.vel.a[j]) * (o0.a[j] + 0.0f) + neg0(d.vel.a[j]) * (o1.a[j] + 0.0f));
       mass[j] = fma_sign(ts, upw * ia, mass[j]);
-      const float hres = step * h.a[j] - upw;
+      const float hres = step * d.h.a[j] - upw;
       const float sr = -ts * hres;
       s_out[j] = s_out[j] - pos0(sr) * ia;
       s_in[j] = s_in[j] - neg0(sr) * ia;
     }
-  }
+  });
   V4 si, so, ms;
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
@@ -1589,7 +1730,8 @@ __global__ void __launch_bounds__(256, HEX_B_fct_edge) kv_fct_edge(HexGeo g, int
 
 // hexcore/transport.py:1919-2118: limited update of the monotonic stage.
 // The vertical residual fluxes are those kv_fct_cell1 formed (vres).
-__global__ void __launch_bounds__(256, HEX_B_fct_cell2) kv_fct_cell2(HexGeo g, int nT, const float* __restrict__ vres,
+template <int B>
+__global__ void HEX_BOUNDS(B, HEX_B_fct_cell2) kv_fct_cell2(HexGeo g, int nT, const float* __restrict__ vres,
                              const float* __restrict__ scale_in, const float* __restrict__ scale_out,
                              const float* __restrict__ mass_in, const float* __restrict__ hres_lim,
                              const float* __restrict__ target, float* __restrict__ q_out) {
@@ -1601,14 +1743,18 @@ __global__ void __launch_bounds__(256, HEX_B_fct_cell2) kv_fct_cell2(HexGeo g, i
   V4 mass = ld4(mass_in + toff + ii);
   const int n = g.deg[c];
   const float ia = g.inv_area[c];
-  HEX_UNROLL_N(HEX_U_fct_cell2)
-  for (int s = 0; s < n; ++s) {
+  struct In {
+    float ts;
+    V4 h;
+  };
+  const auto load = [&](int s) {
     const int sl = __ldg(&g.slot[c * g.maxE + s].x);
-    const float ts = -slot_sign(sl);
-    const V4 h = ld4(hl + k0 + slot_edge(sl));
+    return In{-slot_sign(sl), ld4(hl + k0 + slot_edge(sl))};
+  };
+  gather<B, HEX_U_fct_cell2>(preload<B>(g.maxE, load), n, load, [&](const In& d, int) {
 #pragma unroll
-    for (int j = 0; j < 4; ++j) mass.a[j] = fma_sign(ts, h.a[j] * ia, mass.a[j]);
-  }
+    for (int j = 0; j < 4; ++j) mass.a[j] = fma_sign(d.ts, d.h.a[j] * ia, mass.a[j]);
+  });
   const Win siw = win<1, 1>(scale_in + toff + c * S, k0, S), sow = win<1, 1>(scale_out + toff + c * S, k0, S);
   // interface k0 + 4 belongs to the next chunk; past the column's last chunk
   // it only feeds a padding level, never stored
@@ -1710,7 +1856,7 @@ __global__ void __launch_bounds__(256, HEX_B_vcoef) kv_vcoef(HexGeo g, float dts
                          float* __restrict__ alpha_tri, float* __restrict__ gamma_tri, int* flag) {
   extern __shared__ float sm[];
   const int S = g.S, L = g.L;
-  const int k0 = threadIdx.x * 4;
+  const int k0 = chunk_level();
   const int c = blockIdx.x * blockDim.y + threadIdx.y;
   const bool live = c < g.nC && k0 < S;
   float* s_a = sweep_row(sm, 0, S);
@@ -1829,7 +1975,8 @@ __global__ void __launch_bounds__(256, HEX_B_vcoef) kv_vcoef(HexGeo g, float dts
 #ifndef HEX_AC_DSS_ZERO_SKIP
 #define HEX_AC_DSS_ZERO_SKIP 1
 #endif
-__global__ void __launch_bounds__(256, HEX_B_ac_cell) kv_ac_cell(HexGeo g, int first, float dts, float dts2, const float* __restrict__ ru_p,
+template <int B>
+__global__ void HEX_BOUNDS(B, HEX_B_ac_cell) kv_ac_cell(HexGeo g, int first, float dts, float dts2, const float* __restrict__ ru_p,
                            const float* __restrict__ theta_s, const float* __restrict__ tend_rho,
                            const float* __restrict__ tend_rt, const float* __restrict__ tend_rw,
                            const float* __restrict__ cofwr, const float* __restrict__ cofwz,
@@ -1842,7 +1989,7 @@ __global__ void __launch_bounds__(256, HEX_B_ac_cell) kv_ac_cell(HexGeo g, int f
                            float* __restrict__ ww_avg) {
   extern __shared__ float sm[];
   const int S = g.S, L = g.L;
-  const int k0 = threadIdx.x * 4;
+  const int k0 = chunk_level();
   const int c = blockIdx.x * blockDim.y + threadIdx.y;
   const bool live = c < g.nC && k0 < S;
   float* s_r = sweep_row(sm, 0, S);
@@ -1881,20 +2028,25 @@ __global__ void __launch_bounds__(256, HEX_B_ac_cell) kv_ac_cell(HexGeo g, int f
     const int n = g.deg[c];
     const float ia = g.inv_area[c];
     const V4 tc = ld4(theta_s + ii);
-    HEX_UNROLL_N(HEX_U_ac_cell)
-    for (int s = 0; s < n; ++s) {
+    struct In {
+      float sdd;
+      V4 r, tn;
+    };
+    const auto load = [&](int s) {
       const int2 sl = __ldg(g.slot + c * g.maxE + s);
-      const float sdd = __ldg(g.sdv + c * g.maxE + s) * dts;  // (csign dts) dv
-      const V4 r = ld4(ru_p + k0 + slot_edge(sl.x)), tn = ld4(theta_s + k0 + sl.y);
+      return In{__ldg(g.sdv + c * g.maxE + s) * dts,  // (csign dts) dv
+                ld4(ru_p + k0 + slot_edge(sl.x)), ld4(theta_s + k0 + sl.y)};
+    };
+    gather<B, HEX_U_ac_cell>(preload<B>(g.maxE, load), n, load, [&](const In& d, int) {
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        const float flux = sdd * r.a[j] * ia;
+        const float flux = d.sdd * d.r.a[j] * ia;
         rs.a[j] = rs.a[j] - flux;
         // theta_s[e1] + theta_s[e0], one of the two being this cell (IEEE
         // addition commutes, so the order of the operands changes no bit)
-        ts.a[j] = ts.a[j] - flux * 0.5f * (tn.a[j] + tc.a[j]);
+        ts.a[j] = ts.a[j] - flux * 0.5f * (d.tn.a[j] + tc.a[j]);
       }
-    }
+    });
     const V4 trho = ld4(tend_rho + ii), trt = ld4(tend_rt + ii);
     const V4 wav = first ? v4zero() : ld4rw(ww_avg + ii);
 #pragma unroll

@@ -26,6 +26,9 @@ struct Launcher {
   cudaStream_t main_st = nullptr;  // the caller's stream while launches go to the side stream
   bool on_side = false;            // (the caller's stream may be the legacy stream, handle 0)
   int next_event = 0;
+  // Whether the last operation of this launcher on the caller's / the side
+  // stream was a kernel launch (then the next may start early, see run()).
+  bool chained[2] = {false, false};
   // Independent kernels: fork() makes the side stream wait for everything
   // launched so far, side() sends the following launches there, and
   // join() makes the caller's stream wait for them.  Serial (no-ops) when
@@ -39,6 +42,7 @@ struct Launcher {
     cudaEvent_t ev = ctx.fork_events[next_event++ & 3];
     err = cudaEventRecord(ev, from);
     if (err == cudaSuccess) err = cudaStreamWaitEvent(to, ev, 0);
+    chained[to == ctx.side_stream] = false;
   }
   void fork() {
     if (concurrent()) signal(st, ctx.side_stream);
@@ -62,9 +66,21 @@ struct Launcher {
     main();
     signal(ctx.side_stream, st);
   }
+  // Whether a level-vector launch over n entities (x nz) takes the kernel that
+  // preloads its neighbours (B > 0 in dycore_kernels_vec.cuh): up to two
+  // 128-thread blocks per SM, which those kernels' registers leave resident at
+  // once, the chain of dependent loads is a launch's time.  Two steps of 162
+  // cells x 12: 811 -> 696 us, of 642 x 41: 1154 -> 1032; above, resident warps
+  // count for more (2562 x 55, 36 k chunks of cells and 107 k of edges: none
+  // 1185 us, cells 1088, both 1111 us; 10242 x 55 with cells at 143 k: 3937 ->
+  // 4135).
+  static constexpr long long PRELOAD_CHUNKS = 40000;
+  bool pre(long long n, int nz = 1) const {
+    return ctx.geo.nbrW >= 1 && n * nz * (ctx.geo.S / 4) <= PRELOAD_CHUNKS;
+  }
   // entities per block for tpe threads per entity under the label's block size
-  int epb(const char* name, int tpe, long long n) const {
-    const int threads = ctx.threads_for(name, n * tpe);
+  int epb(const char* name, int tpe) const {
+    const int threads = ctx.threads_for(name);
     return tpe >= threads ? 1 : threads / tpe;
   }
   template <class K, class... A>
@@ -100,22 +116,47 @@ struct Launcher {
   void launch_impl(const char* name, int tpe, int n, int nz, size_t smem_per_entity, bool fold, K kernel,
                    A... args) {
     if (err != cudaSuccess || n <= 0 || nz <= 0) return;
-    const int e = epb(name, tpe, (long long)n * nz);
+    const int e = epb(name, tpe);
     const unsigned nb = (unsigned)((n + e - 1) / e);
     dim3 block(tpe, e), grid(fold ? nb * (unsigned)nz : nb, 1, fold ? 1 : nz);
-    run(name, grid, block, smem_per_entity * e, kernel, args...);
+    run(name, grid, block, smem_per_entity * e, fold || tpe < ctx.geo.S, kernel, args...);
   }
   template <class K, class... A>
-  void run(const char* name, dim3 grid, dim3 block, size_t smem, K kernel, A... args) {
+  void run(const char* name, dim3 grid, dim3 block, size_t smem, bool vec, K kernel, A... args) {
     HexProfEvent ev{name, nullptr, nullptr};
     if (prof) {
       cudaEventCreate(&ev.start);
       cudaEventCreate(&ev.stop);
       cudaEventRecord(ev.start, st);
     }
-    kernel<<<grid, block, smem, st>>>(args...);
+    // A level-vector kernel waits for its predecessor itself (chunk_level), so
+    // its blocks may be set up while that runs (programmatic stream
+    // serialisation; only after a kernel of this step on the same stream, and a
+    // programmatic edge of the captured graph).  Two steps of 162 x 12: 674 ->
+    // 634 us, 642 x 41: 976 -> 952, 10242 x 55 with mixing: 3960 -> 3875,
+    // x1.40962 x 55: 11051 -> 11020.  Not for grids between PRELOAD_CHUNKS and
+    // four 256-thread blocks per SM, which share the SMs with the other stream's
+    // kernel at once: waiting blocks take its slots (2562 x 55: 1086 -> 1134).
+    const long long chunks = (long long)grid.x * grid.z * block.x * block.y;
+    bool& ch = chained[on_side];
+    if (vec && ch && !prof && (chunks <= PRELOAD_CHUNKS || chunks > 256LL * 4 * 148)) {
+      cudaLaunchAttribute at{};
+      at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+      at.val.programmaticStreamSerializationAllowed = 1;
+      cudaLaunchConfig_t cfg{};
+      cfg.gridDim = grid;
+      cfg.blockDim = block;
+      cfg.dynamicSmemBytes = smem;
+      cfg.stream = st;
+      cfg.attrs = &at;
+      cfg.numAttrs = 1;
+      err = cudaLaunchKernelEx(&cfg, kernel, args...);
+    } else {
+      kernel<<<grid, block, smem, st>>>(args...);
+      err = cudaGetLastError();
+    }
+    ch = true;
     ++count;
-    err = cudaGetLastError();
     if (prof) {
       cudaEventRecord(ev.stop, st);
       prof->push_back(ev);
@@ -128,16 +169,17 @@ struct Launcher {
 #define LPSN(L, label, n, nz, name, ...) (L).lpv(label, n, nz, kv_##name, __VA_ARGS__)
 // Transport kernel kv_<name> over nT tracers (tracer folded into the block index).
 #define LPST(L, n, nT, name, g, ...) (L).lpvt("k_" #name, n, nT, kv_##name, g, nT, __VA_ARGS__)
-// Column-sweep kernel: the column-group form kv_<name> when a column fits in
-// one warp (S/4 <= 32), else the one-level form k_<name> (shared memory per
-// column: smem_v and smem respectively).
-#define LPG(L, label, n, smem, smem_v, name, ...)                      \
+// Column-sweep kernel: the column-group form (kernel_v, kv_<name>) when a
+// column fits in one warp (S/4 <= 32), else the one-level form (kernel,
+// k_<name>); shared memory per column: smem_v and smem respectively.
+#define LPGK(L, label, n, smem, smem_v, kernel, kernel_v, ...)         \
   do {                                                                 \
     if ((L).group())                                                   \
-      (L).lpg(label, n, smem_v, kv_##name, __VA_ARGS__);               \
+      (L).lpg(label, n, smem_v, kernel_v, __VA_ARGS__);                \
     else                                                               \
-      (L).lp(label, n, 1, smem, k_##name, __VA_ARGS__);                \
+      (L).lp(label, n, 1, smem, kernel, __VA_ARGS__);                  \
   } while (0)
+#define LPG(L, label, n, smem, smem_v, name, ...) LPGK(L, label, n, smem, smem_v, k_##name, kv_##name, __VA_ARGS__)
 
 static void diagnostics(Launcher& L, const float* u, int recompute_v) {
   HexCtx& c = L.ctx;
@@ -145,10 +187,12 @@ static void diagnostics(Launcher& L, const float* u, int recompute_v) {
   HexWork& w = c.w;
   // (vorticity and divergence are kept only for the horizontal mixing)
   LPS(L, g.nV, 1, diag_vertex, g, u, w.pv_vertex, w.ke_vertex, w.vorticity);
-  L.lpv("k_diag_cell", g.nC, 1, w.divergence ? kv_diag_cell<true> : kv_diag_cell<false>, g, u,
+  const auto cell = w.divergence ? (L.pre(g.nC) ? kv_diag_cell<true, 6> : kv_diag_cell<true, 0>)
+                                 : (L.pre(g.nC) ? kv_diag_cell<false, 6> : kv_diag_cell<false, 0>);
+  L.lpv("k_diag_cell", g.nC, 1, cell, g, u,
         (const float*)w.pv_vertex, (const float*)w.ke_vertex, w.ke, w.pv_cell, w.divergence);
-  LPSN(L, recompute_v ? "k_diag_edge_v" : "k_diag_edge", g.nE, 1, diag_edge, g, u, (const float*)w.pv_vertex,
-       (const float*)w.pv_cell, w.v, w.pv_edge, recompute_v);
+  L.lpv(recompute_v ? "k_diag_edge_v" : "k_diag_edge", g.nE, 1, L.pre(g.nE) ? kv_diag_edge<5> : kv_diag_edge<0>,
+        g, u, (const float*)w.pv_vertex, (const float*)w.pv_cell, w.v, w.pv_edge, recompute_v);
 }
 
 cudaError_t diagnostics_only(HexCtx& ctx, const HexState& s, const HexSide& side, cudaStream_t stream) {
@@ -188,6 +232,7 @@ cudaError_t run_step(HexCtx& ctx, const HexState& in, const HexSide& side_in, co
         bufs[n] = const_cast<float*>(b.first);
         kinds[n++] = b.second;
       }
+    L.chained[0] = L.chained[1] = false;
     if (ctx.exchange_hook(ctx.exchange_user, point, n, bufs, kinds) < 0) {
       ctx.phys_failed = 1;
       L.err = cudaErrorLaunchFailure;
@@ -202,8 +247,11 @@ cudaError_t run_step(HexCtx& ctx, const HexState& in, const HexSide& side_in, co
   const size_t sm_ac_v = sizeof(float) * (g.S + HEX_SWEEP_PAD) * HEX_ACV_SMEM_ARRAYS;
 
   if (g.moist) {
-    L.lpv("k_moist_cell", g.nC, 1, kv_moist_cell, g, (const float*)in.scalars, nT, w.qtot, w.cqw);
-    L.lpv("k_moist_edge", g.nE, 1, kv_moist_edge, g, (const float*)in.scalars, nT, w.cqu);
+    // (no scalar: nothing to preload)
+    L.lpv("k_moist_cell", g.nC, 1, nT && L.pre(g.nC) ? kv_moist_cell<6> : kv_moist_cell<0>,
+          g, (const float*)in.scalars, nT, w.qtot, w.cqw);
+    L.lpv("k_moist_edge", g.nE, 1, nT && L.pre(g.nE) ? kv_moist_edge<6> : kv_moist_edge<0>,
+          g, (const float*)in.scalars, nT, w.cqu);
   }
   // initial solve diagnostics with v reconstructed (rk_step=3)
   diagnostics(L, side_in.u, 1);
@@ -231,7 +279,8 @@ cudaError_t run_step(HexCtx& ctx, const HexState& in, const HexSide& side_in, co
     L.side();
     LPS(L, g.nE, 1, euler_edge, g, (const float*)s_in->pressure_p, (const float*)s_in->rho_p,
          (const float*)w.qtot, (const float*)w.cqu, w.euler_ru);
-    LPS(L, g.nC, 1, euler_cell, g, (const float*)saved->rho_u, (const float*)saved->rho_w,
+    L.lpv("k_euler_cell", g.nC, 1, L.pre(g.nC) ? kv_euler_cell<6> : kv_euler_cell<0>,
+          g, (const float*)saved->rho_u, (const float*)saved->rho_w,
          (const float*)s_in->pressure_p, (const float*)s_in->rho_p, (const float*)w.qtot, (const float*)w.cqw,
          w.tend_rho, w.euler_rw, (const float*)(hooked && ctx.phys_held_rho ? ctx.phys_rho : nullptr),
          hooked ? ctx.tend_rho_dyn : nullptr);
@@ -271,6 +320,7 @@ cudaError_t run_step(HexCtx& ctx, const HexState& in, const HexSide& side_in, co
                                              cs->theta_m, cs->exner, cs->rho_p, cs->rtheta_p, cs->pressure_p,
                                              cs->u, cs->w};
         for (int i = 0; i < HEXDYN_NUM_FIELDS; ++i) cur_fields.field[i] = const_cast<float*>(f[i]);
+        L.chained[0] = L.chained[1] = false;
         phys = ctx.stage_hook(ctx.stage_user, sub + 1, stg.stage, &cur_fields);
         if (phys < 0) {
           ctx.phys_failed = 1;
@@ -280,15 +330,19 @@ cudaError_t run_step(HexCtx& ctx, const HexState& in, const HexSide& side_in, co
       }
       // the mass-flux divergence of cur->rho_u: computed by the previous
       // stage's recovery, except for the first stage of the step
-      if (sub == 0 && si == 0) LPS(L, g.nC, 1, hdiv, g, (const float*)cur->rho_u, w.hdiv);
+      if (sub == 0 && si == 0)
+        L.lpv("k_hdiv", g.nC, 1, L.pre(g.nC) ? kv_hdiv<6> : kv_hdiv<0>, g, (const float*)cur->rho_u, w.hdiv);
       // edge values, the momentum tendency and (stage 2) the coefficients
       // are independent: the first on this stream, the others on the side
       L.region = 2;
       L.fork();
-      LPS(L, g.nE, 1, edge_adv, g, (const float*)cur->rho_u, (const float*)cs->theta_m, (const float*)cs->w,
+      L.lpv("k_edge_adv", g.nE, 1, L.pre(g.nE) ? kv_edge_adv<10> : kv_edge_adv<0>,
+            g, (const float*)cur->rho_u, (const float*)cs->theta_m, (const float*)cs->w,
            w.edge_theta, w.edge_w);
       L.side();
-      L.lpv("k_tend_u", g.nE, 1, g.rayleigh_levels ? kv_tend_u<true> : kv_tend_u<false>, g, (const float*)cs->u,
+      const auto tend_u = g.rayleigh_levels ? (L.pre(g.nE) ? kv_tend_u<true, 5> : kv_tend_u<true, 0>)
+                                            : (L.pre(g.nE) ? kv_tend_u<false, 5> : kv_tend_u<false, 0>);
+      L.lpv("k_tend_u", g.nE, 1, tend_u, g, (const float*)cs->u,
             (const float*)cur->rho_w, (const float*)cur->rho, (const float*)w.pv_edge, (const float*)w.ke,
             (const float*)w.hdiv, saved_ru, w.tend_ru,
             (const float*)((phys & HEXDYN_PHYS_RHO_U) ? ctx.phys_ru : nullptr), dts,
@@ -299,7 +353,8 @@ cudaError_t run_step(HexCtx& ctx, const HexState& in, const HexSide& side_in, co
              w.cofwt, w.a_tri, w.alpha_tri, w.gamma_tri, w.flag);
       }
       L.join();
-      LPS(L, g.nC, 1, tend_cell, g, (const float*)cur->rho_u, (const float*)saved->rho_u,
+      L.lpv("k_tend_cell", g.nC, 1, L.pre(g.nC) ? kv_tend_cell<6> : kv_tend_cell<0>,
+            g, (const float*)cur->rho_u, (const float*)saved->rho_u,
            (const float*)cur->rho_w, (const float*)saved->rho_w, (const float*)cs->theta_m,
            (const float*)s_in->theta_m, (const float*)cs->w, (const float*)w.edge_theta, (const float*)w.edge_w,
            saved_rw, (const float*)w.tend_ru, w.tend_rt, w.tend_rw, stg.stage, saved_theta,
@@ -326,7 +381,8 @@ cudaError_t run_step(HexCtx& ctx, const HexState& in, const HexSide& side_in, co
                prev_old, (const float*)w.rho_pp, (const float*)s_in->theta_m, (const float*)s_in->exner,
                (const float*)w.cqu, w.ru_p, w.ru_avg);
         }
-        LPG(L, n == 1 ? "k_ac_cell_first" : "k_ac_cell", g.nC, sm_ac, sm_ac_v, ac_cell, g, n == 1 ? 1 : 0, dts, dts2, (const float*)w.ru_p,
+        LPGK(L, n == 1 ? "k_ac_cell_first" : "k_ac_cell", g.nC, sm_ac, sm_ac_v, k_ac_cell,
+             (L.pre(g.nC) ? kv_ac_cell<6> : kv_ac_cell<0>), g, n == 1 ? 1 : 0, dts, dts2, (const float*)w.ru_p,
              (const float*)s_in->theta_m, (const float*)w.tend_rho, (const float*)w.tend_rt,
              (const float*)w.tend_rw, (const float*)w.cofwr, (const float*)w.cofwz, (const float*)w.coftz,
              (const float*)w.cofwt, (const float*)w.a_tri, (const float*)w.alpha_tri, (const float*)w.gamma_tri,
@@ -354,7 +410,8 @@ cudaError_t run_step(HexCtx& ctx, const HexState& in, const HexSide& side_in, co
       // the cell recovery and the diagnostics of the new u share no array
       L.region = 4;
       L.fork();
-      LPS(L, g.nC, 1, recover_cell, g, stg.stage == 3 ? 1 : 0, (const float*)s_in->rho_p,
+      L.lpv("k_recover_cell", g.nC, 1, L.pre(g.nC) ? kv_recover_cell<6> : kv_recover_cell<0>,
+            g, stg.stage == 3 ? 1 : 0, (const float*)s_in->rho_p,
            (const float*)s_in->rtheta_p, (const float*)saved->rho_w, (const float*)w.rho_pp, rtpp_final,
            (const float*)w.rw_p, (const float*)w.ww_avg, (const float*)o.rho_u, o, so, w.flux_w, fm, inv_steps,
            inv_splits, w.flag, w.hdiv);
@@ -386,10 +443,12 @@ cudaError_t run_step(HexCtx& ctx, const HexState& in, const HexSide& side_in, co
       L.err = cap == cudaStreamCaptureStatusActive
                   ? cudaEventRecordWithFlags(ctx.dynamics_done, L.st, cudaEventRecordExternal)
                   : cudaEventRecord(ctx.dynamics_done, L.st);
+    L.chained[0] = false;
   }
   // split scalar transport: RK1, RK2 standard, RK3 monotonic FCT
   if (nT > 0) {
     const float* q_prev = in.scalars;
+    const int groups = (nT + HEX_TR_GROUP - 1) / HEX_TR_GROUP;
     for (int si = 0; si < 3; ++si) {
       const HexStage& stg = ctx.scal[si];
       const float step = (float)stg.large_dt;
@@ -401,22 +460,29 @@ cudaError_t run_step(HexCtx& ctx, const HexState& in, const HexSide& side_in, co
       if (si < 2 || !ctx.monotonic) {
         // hexcore/transport.py:1749-1755 time-interpolation weight of rho_new
         const float wn = si == 0 ? (ctx.order == 3 ? (float)(1.0 / 3.0) : 0.5f) : (si == 1 ? 0.5f : 1.0f);
-        L.lpvt("k_tr_edge", g.nE, (nT + HEX_TR_GROUP - 1) / HEX_TR_GROUP, kv_tr_edge, g, nT, 0, q_prev,
-               (const float*)w.flux_u, w.edge_q);
-        LPST(L, g.nC, nT, tr_std, g, step, wn, (const float*)in.scalars, q_prev, (const float*)in.rho,
+        L.lpvt("k_tr_edge", g.nE, groups, L.pre(g.nE, groups) ? kv_tr_edge<10> : kv_tr_edge<0>, g, nT, 0,
+               q_prev, (const float*)w.flux_u, w.edge_q);
+        L.lpvt("k_tr_std", g.nC, nT, L.pre(g.nC, nT) ? kv_tr_std<6> : kv_tr_std<0>,
+              g, nT, step, wn, (const float*)in.scalars, q_prev, (const float*)in.rho,
              (const float*)out.rho, (const float*)w.flux_u, (const float*)w.flux_w, (const float*)w.edge_q, q_next);
       } else {
-        LPS(L, g.nC, 1, fct_target, g, step, (const float*)in.rho, (const float*)w.flux_u,
+        L.lpv("k_fct_target", g.nC, 1, L.pre(g.nC) ? kv_fct_target<6> : kv_fct_target<0>,
+              g, step, (const float*)in.rho, (const float*)w.flux_u,
              (const float*)w.flux_w, w.target, w.flag);
-        L.lpvt("k_tr_edge", g.nE, (nT + HEX_TR_GROUP - 1) / HEX_TR_GROUP, kv_tr_edge, g, nT, 1, q_prev,
-               (const float*)w.flux_u, w.edge_q);
-        L.lpvt("k_fct_cell1", g.nC, nT, g.coc_across ? kv_fct_cell1<true> : kv_fct_cell1<false>, g, nT, step,
+        L.lpvt("k_tr_edge", g.nE, groups, L.pre(g.nE, groups) ? kv_tr_edge<10> : kv_tr_edge<0>, g, nT, 1,
+               q_prev, (const float*)w.flux_u, w.edge_q);
+        // (the slots' cellsOnCell need not be valid past a cell's degree)
+        const auto cell1 = !g.coc_across     ? kv_fct_cell1<false, 0>
+                           : L.pre(g.nC, nT) ? kv_fct_cell1<true, 6>
+                                             : kv_fct_cell1<true, 0>;
+        L.lpvt("k_fct_cell1", g.nC, nT, cell1, g, nT, step,
              (const float*)in.scalars, q_prev, (const float*)in.rho, (const float*)w.flux_u, (const float*)w.flux_w, (const float*)w.edge_q, (const float*)w.target,
              w.scale_in, w.scale_out, w.mass, w.vres);
         exchange(HEXDYN_XCH_FCT, {{w.scale_in, KT}, {w.scale_out, KT}});
         LPST(L, g.nE, nT, fct_edge, g, step, (const float*)in.scalars, (const float*)w.flux_u,
              (const float*)w.edge_q, (const float*)w.scale_in, (const float*)w.scale_out, w.hres_lim);
-        LPST(L, g.nC, nT, fct_cell2, g, (const float*)w.vres, (const float*)w.scale_in, (const float*)w.scale_out, (const float*)w.mass, (const float*)w.hres_lim,
+        L.lpvt("k_fct_cell2", g.nC, nT, L.pre(g.nC, nT) ? kv_fct_cell2<6> : kv_fct_cell2<0>,
+              g, nT, (const float*)w.vres, (const float*)w.scale_in, (const float*)w.scale_out, (const float*)w.mass, (const float*)w.hres_lim,
              (const float*)w.target, q_next);
       }
       q_prev = q_next;

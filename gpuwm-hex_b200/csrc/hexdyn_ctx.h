@@ -116,16 +116,15 @@ struct HexCtx {
   // Halo exchange hook of a partitioned instance (hexdyn_set_exchange_hook)
   HexDynExchangeHook exchange_hook = nullptr;
   void* exchange_user = nullptr;
-  // Block size of a launch of `chunks` four-level chunks (threads).  Untuned:
-  // 128 when blocks of 256 would not all be resident at once (4 per SM of
-  // 148), 256 below.  128 fits the registers of an SM more evenly and leaves
-  // shorter last waves (x1.40962 step: 6.30 vs 6.42 ms); a grid that is
-  // resident at once gains nothing from more blocks (2562 cells: 645 vs 638 us).
-  int threads_for(const char* label, long long chunks) const {
+  // Block size of a launch (threads).  Untuned: 128, which fits the registers
+  // of an SM more evenly than 256 and leaves shorter last waves (x1.40962
+  // step: 6.30 vs 6.42 ms), and spreads a small grid over more SMs (two steps
+  // of 162 cells 634 vs 673 us, of 2562 cells 1086 vs 1112).
+  int threads_for(const char* label) const {
     if (force_threads) return force_threads;
     for (const auto& t : tuned_threads)
       if (t.first == label) return t.second;
-    return chunks > 256LL * 4 * 148 ? 128 : 256;
+    return 128;
   }
 };
 
