@@ -182,6 +182,24 @@ struct Gemm {
   uint32_t mma_wait_polls;  // polls of the MMA issuer's wait for a loaded stage (WAIT_LIMIT normally)
 };
 
+// eight floats as bf16 (two per conversion)
+__device__ __forceinline__ uint4 pack8(const float* v) {
+  uint32_t r[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const __nv_bfloat162 t = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
+    r[i] = *reinterpret_cast<const uint32_t*>(&t);
+  }
+  return make_uint4(r[0], r[1], r[2], r[3]);
+}
+// eight bf16 to eight rows `ld` apart
+__device__ __forceinline__ void store_column8(bf16* dst, int ld, const uint4& v) {
+  const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+  unsigned short* d = reinterpret_cast<unsigned short*>(dst);
+#pragma unroll
+  for (int i = 0; i < 8; ++i) d[(size_t)i * ld] = (unsigned short)(w[i >> 1] >> (16 * (i & 1)));
+}
+
 // Epilogue of 8 accumulator columns of one row: bias, then the selected
 // epilogue, stores of C / C^T / Z / Cf (shared by both GEMM kernels).
 __device__ __forceinline__ void epilogue8(const Gemm& p, int row, int col, float* v, uint4* c_out = nullptr,
@@ -200,42 +218,30 @@ __device__ __forceinline__ void epilogue8(const Gemm& p, int row, int col, float
     v[7] += b1.w;
   }
   if (p.epilogue == HEXMLP_EPI_GELU) {
-    __nv_bfloat16 z[8], h[8];
+    float h[8];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      z[i] = __float2bfloat16_rn(v[i]);
-      h[i] = __float2bfloat16_rn(gelu(v[i]));
-    }
-    if (p.Z) *reinterpret_cast<uint4*>(p.Z + (size_t)row * p.N + col) = *reinterpret_cast<uint4*>(z);
+    for (int i = 0; i < 8; ++i) h[i] = gelu(v[i]);
+    if (p.Z) *reinterpret_cast<uint4*>(p.Z + (size_t)row * p.N + col) = pack8(v);
+    const uint4 hb = pack8(h);
     if (c_out)
-      *c_out = *reinterpret_cast<uint4*>(h);  // the caller stores C
+      *c_out = hb;  // the caller stores C
     else if (p.C)
-      *reinterpret_cast<uint4*>(p.C + (size_t)row * p.N + col) = *reinterpret_cast<uint4*>(h);
-    if (p.Ct) {
-#pragma unroll
-      for (int i = 0; i < 8; ++i) p.Ct[(size_t)(col + i) * p.M + row] = h[i];
-    }
+      *reinterpret_cast<uint4*>(p.C + (size_t)row * p.N + col) = hb;
+    if (p.Ct) store_column8(p.Ct + (size_t)col * p.M + row, p.M, hb);
   } else if (p.epilogue == HEXMLP_EPI_GELU_GRAD) {
-    __nv_bfloat16 d[8];
+    float d[8];
     const uint4 zr = *reinterpret_cast<const uint4*>(p.Zin + (size_t)row * p.N + col);
     const __nv_bfloat16* zz = reinterpret_cast<const __nv_bfloat16*>(&zr);
 #pragma unroll
-    for (int i = 0; i < 8; ++i) d[i] = __float2bfloat16_rn(v[i] * gelu_grad(__bfloat162float(zz[i])));
-    if (p.C) *reinterpret_cast<uint4*>(p.C + (size_t)row * p.N + col) = *reinterpret_cast<uint4*>(d);
-    if (p.Ct) {
-#pragma unroll
-      for (int i = 0; i < 8; ++i) p.Ct[(size_t)(col + i) * p.M + row] = d[i];
-    }
+    for (int i = 0; i < 8; ++i) d[i] = v[i] * gelu_grad(__bfloat162float(zz[i]));
+    const uint4 db = pack8(d);
+    if (p.C) *reinterpret_cast<uint4*>(p.C + (size_t)row * p.N + col) = db;
+    if (p.Ct) store_column8(p.Ct + (size_t)col * p.M + row, p.M, db);
   } else {
     float4* dst = f_out ? f_out : reinterpret_cast<float4*>(p.Cf + (size_t)row * p.N + col);  // f_out: caller stores
     dst[0] = make_float4(v[0], v[1], v[2], v[3]);
     dst[1] = make_float4(v[4], v[5], v[6], v[7]);
-    if (p.C) {
-      __nv_bfloat16 b[8];
-#pragma unroll
-      for (int i = 0; i < 8; ++i) b[i] = __float2bfloat16_rn(v[i]);
-      *reinterpret_cast<uint4*>(p.C + (size_t)row * p.N + col) = *reinterpret_cast<uint4*>(b);
-    }
+    if (p.C) *reinterpret_cast<uint4*>(p.C + (size_t)row * p.N + col) = pack8(v);
   }
 }
 
@@ -367,9 +373,17 @@ __global__ void __launch_bounds__(THREADS, 2) k_gemm_bf16(Gemm p) {
 // producer waits for every TMA load it issued to land and the MMA issuer
 // commits a drain barrier and waits for every MMA it issued, so no
 // asynchronous copy or MMA is in flight at exit on either path.
-constexpr int WS_THREADS = 320;
+constexpr int WS_EPI_WARPS = 8;  // two per lane quarter, each half of the tile's columns
+constexpr int WS_THREADS = 64 + 32 * WS_EPI_WARPS;
 constexpr int WS_STAGES = 4;
-constexpr int STAGE_ROW = 80;  // bytes between rows of an epilogue warp's staging tile
+// An epilogue warp's staging tiles: 32 rows of 64 bytes each, the 16-byte
+// pieces of a row permuted as the 64-byte TMA swizzle has them (which spreads
+// a column of pieces over the banks).  Two, so that one fills while the TMA
+// store reads the other.
+constexpr int STAGE_TILE = 32 * 64;
+constexpr int STAGE_TILES = 2;
+constexpr int WS_BARRIERS = 512;  // mbarriers; the staging tiles after them start on the swizzle's 512 bytes
+__device__ __forceinline__ int stage_at(int row, int piece) { return row * 64 + 16 * (piece ^ ((row >> 1) & 3)); }
 
 __device__ __forceinline__ void mbar_expect_tx(uint32_t mbar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(mbar), "r"(bytes) : "memory");
@@ -396,9 +410,34 @@ __device__ __forceinline__ uint64_t umma_desc_sw128(uint32_t addr) {
   return d;
 }
 
-template <int BN>
-__global__ void __launch_bounds__(WS_THREADS, 1)
-    k_gemm_ws(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, Gemm p) {
+__device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, int x, int y, uint32_t src) {
+  asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group [%0, {%1, %2}], [%3];" ::"l"(
+                   reinterpret_cast<uint64_t>(map)),
+               "r"(x), "r"(y), "r"(src)
+               : "memory");
+}
+
+// Products of one launch: their tiles in one sequence, product i's from
+// first[i] on.  `out` maps C (bf16) or Cf where the epilogue stores through it.
+template <int G>
+struct GemmGroup {
+  CUtensorMap a[G], b[G], out[G];
+  Gemm p[G];
+  int first[G + 1];
+  int tiles;
+};
+// (index of the product, output tile) of the launch's tile t; `i` only grows
+template <int BN, int G>
+__device__ __forceinline__ void group_tile(const GemmGroup<G>& g, int t, int& i, int& m0, int& n0) {
+  if (G > 1)
+    while (t >= g.first[i + 1]) ++i;
+  const int local = t - g.first[i], n_n = g.p[i].N / BN;
+  m0 = (local / n_n) * BM;
+  n0 = (local % n_n) * BN;
+}
+
+template <int BN, int G>
+__global__ void __launch_bounds__(WS_THREADS, 1) k_gemm_ws(const __grid_constant__ GemmGroup<G> grp) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   // stage buffers on a 1024-byte boundary (the swizzle atom)
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -411,7 +450,7 @@ __global__ void __launch_bounds__(WS_THREADS, 1)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drain + 1);
   volatile int* abort_word = reinterpret_cast<volatile int*>(tmem_slot + 1);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int n_n = p.N / BN, tiles = (p.M / BM) * n_n, nk = p.K / BK;
+  const int tiles = grp.tiles;
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < WS_STAGES; ++i) {
@@ -420,7 +459,7 @@ __global__ void __launch_bounds__(WS_THREADS, 1)
     }
     for (int i = 0; i < 2; ++i) {
       mbar_init(smem_u32(&acc_full[i]), 1);
-      mbar_init(smem_u32(&acc_empty[i]), 8);  // one arrival per epilogue warp
+      mbar_init(smem_u32(&acc_empty[i]), WS_EPI_WARPS);  // one arrival per epilogue warp
     }
     mbar_init(smem_u32(drain), 1);
     *abort_word = 0;
@@ -443,8 +482,11 @@ __global__ void __launch_bounds__(WS_THREADS, 1)
       int last_it[WS_STAGES];  // last iteration whose loads went to each stage
 #pragma unroll
       for (int s = 0; s < WS_STAGES; ++s) last_it[s] = -1;
+      int gi = 0;
       for (int t = blockIdx.x; t < tiles && !*abort_word; t += gridDim.x) {
-        const int m0 = (t / n_n) * BM, n0 = (t % n_n) * BN;
+        int m0, n0;
+        group_tile<BN, G>(grp, t, gi, m0, n0);
+        const int nk = grp.p[gi].K / BK;
         for (int kt = 0; kt < nk; ++kt, ++it) {
           const int s = it % WS_STAGES;
           if (!mbar_wait_or_abort(smem_u32(&empty[s]), ((it / WS_STAGES) & 1) ^ 1, abort_word, WAIT_LIMIT)) {
@@ -453,8 +495,8 @@ __global__ void __launch_bounds__(WS_THREADS, 1)
           }
           uint8_t* a = smem + s * STAGE;
           mbar_expect_tx(smem_u32(&full[s]), STAGE);
-          tma_load_2d(smem_u32(a), &tmA, kt * BK, m0, smem_u32(&full[s]));
-          tma_load_2d(smem_u32(a + A_BYTES), &tmB, kt * BK, n0, smem_u32(&full[s]));
+          tma_load_2d(smem_u32(a), &grp.a[gi], kt * BK, m0, smem_u32(&full[s]));
+          tma_load_2d(smem_u32(a + A_BYTES), &grp.b[gi], kt * BK, n0, smem_u32(&full[s]));
           last_it[s] = it;
         }
       }
@@ -469,8 +511,11 @@ __global__ void __launch_bounds__(WS_THREADS, 1)
     // MMA issuer
     if (lane == 0) {
       const uint32_t idesc = umma_idesc(BM, BN);
-      int it = 0, tc = 0;
+      int it = 0, tc = 0, gi = 0;
       for (int t = blockIdx.x; t < tiles && !*abort_word; t += gridDim.x, ++tc) {
+        int m0, n0;
+        group_tile<BN, G>(grp, t, gi, m0, n0);
+        const int nk = grp.p[gi].K / BK;
         const int b = tc & 1;
         if (!mbar_wait_or_abort(smem_u32(&acc_empty[b]), ((tc >> 1) & 1) ^ 1, abort_word, WAIT_LIMIT)) {
           *abort_word = 1;
@@ -480,7 +525,7 @@ __global__ void __launch_bounds__(WS_THREADS, 1)
         const uint32_t acc = tmem + (uint32_t)(b * BN);
         for (int kt = 0; kt < nk; ++kt, ++it) {
           const int s = it % WS_STAGES;
-          if (!mbar_wait_or_abort(smem_u32(&full[s]), (it / WS_STAGES) & 1, abort_word, p.mma_wait_polls)) {
+          if (!mbar_wait_or_abort(smem_u32(&full[s]), (it / WS_STAGES) & 1, abort_word, grp.p[gi].mma_wait_polls)) {
             *abort_word = 1;
             break;
           }
@@ -502,15 +547,20 @@ __global__ void __launch_bounds__(WS_THREADS, 1)
     }
   } else {
     // epilogue warps 2..9: lane quarter warp % 4, column half (warp - 2) / 4
-    const int quarter = warp & 3, half = (warp - 2) >> 2;
-    // bf16 activations leave through a per-warp staging tile (32 rows of 64
-    // bytes, rows 80 bytes apart) so that the global stores are row-contiguous
-    const bool staged = p.epilogue == HEXMLP_EPI_GELU && p.C != nullptr;
-    const bool staged_f32 = p.epilogue == HEXMLP_EPI_F32 && p.C == nullptr;
-    uint8_t* stage_tile = smem + WS_STAGES * STAGE + 256 + (warp - 2) * 32 * STAGE_ROW;
-    int tc = 0;
+    constexpr int PART = BN / (WS_EPI_WARPS / 4);
+    const int quarter = warp & 3, part = (warp - 2) >> 2;
+    // activations and FP32 results leave through the staging tiles by TMA
+    // stores (a warp's 32 rows x 64 bytes each): the stores need neither
+    // shared-memory reads nor address arithmetic of the warps that set the pace
+    uint8_t* stage_tile = smem + WS_STAGES * STAGE + WS_BARRIERS + (warp - 2) * STAGE_TILES * STAGE_TILE;
+    int tc = 0, gi = 0, buf = 0;
     for (int t = blockIdx.x; t < tiles; t += gridDim.x, ++tc) {
       const int b = tc & 1;
+      int m0, n0;
+      group_tile<BN, G>(grp, t, gi, m0, n0);
+      const Gemm& p = grp.p[gi];
+      const bool staged = p.epilogue == HEXMLP_EPI_GELU && p.C != nullptr;
+      const bool staged_f32 = p.epilogue == HEXMLP_EPI_F32 && p.C == nullptr;
       bool ok = true;
       if (lane == 0) ok = mbar_wait_or_abort(smem_u32(&acc_full[b]), (tc >> 1) & 1, abort_word, WAIT_LIMIT);
       ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
@@ -520,48 +570,53 @@ __global__ void __launch_bounds__(WS_THREADS, 1)
       }
       if (*abort_word) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const int m0 = (t / n_n) * BM, n0 = (t % n_n) * BN;
-      const int row = m0 + quarter * 32 + lane;
+      const int row0 = m0 + quarter * 32, row = row0 + lane;
       const uint32_t base = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(b * BN);
-      for (int c32 = half * (BN / 2); c32 < (half + 1) * (BN / 2); c32 += 32) {
+      // a staging tile that no TMA store is still reading: at most the other
+      // tile's store may be in flight
+      const auto tile_ready = [&]() {
+        if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+        __syncwarp();
+      };
+      // the staged tile out to columns x.. of this warp's rows
+      const auto tile_store = [&](uint8_t* tile, int x) {
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) {
+          tma_store_2d(&grp.out[gi], x, row0, smem_u32(tile));
+          asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+        }
+        buf ^= 1;
+      };
+      for (int c32 = part * PART; c32 < (part + 1) * PART; c32 += 32) {
         float v32[32];
         tmem_ld32(base + (uint32_t)c32, v32);
         if (staged) {
-          // this lane's row of 32 activations into the warp's staging tile,
-          // then out row by row: 4 lanes write a row's 64 contiguous bytes
+          // this lane's row of 32 activations
+          uint8_t* tile = stage_tile + buf * STAGE_TILE;
+          tile_ready();
 #pragma unroll
           for (int g8 = 0; g8 < 4; ++g8) {
             uint4 h;
             epilogue8(p, row, n0 + c32 + 8 * g8, v32 + 8 * g8, &h);
-            *reinterpret_cast<uint4*>(stage_tile + lane * STAGE_ROW + 16 * g8) = h;
+            *reinterpret_cast<uint4*>(tile + stage_at(lane, g8)) = h;
           }
-          __syncwarp();
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const int r = 8 * j + (lane >> 2), piece = lane & 3;
-            const uint4 h = *reinterpret_cast<const uint4*>(stage_tile + r * STAGE_ROW + 16 * piece);
-            *reinterpret_cast<uint4*>(p.C + (size_t)(m0 + quarter * 32 + r) * p.N + n0 + c32 + 8 * piece) = h;
-          }
-          __syncwarp();
+          tile_store(tile, n0 + c32);
         } else if (staged_f32) {
-          // FP32 out: two halves of 16 columns (64 bytes a row) through the tile
+          // FP32 out: two halves of 16 columns (64 bytes a row)
 #pragma unroll
           for (int hh = 0; hh < 2; ++hh) {
+            uint8_t* tile = stage_tile + buf * STAGE_TILE;
+            tile_ready();
 #pragma unroll
             for (int g = 0; g < 2; ++g) {
               const int g8 = 2 * hh + g;
-              epilogue8(p, row, n0 + c32 + 8 * g8, v32 + 8 * g8, nullptr,
-                        reinterpret_cast<float4*>(stage_tile + lane * STAGE_ROW + 32 * g));
+              float4 f[2];
+              epilogue8(p, row, n0 + c32 + 8 * g8, v32 + 8 * g8, nullptr, f);
+              *reinterpret_cast<float4*>(tile + stage_at(lane, 2 * g)) = f[0];
+              *reinterpret_cast<float4*>(tile + stage_at(lane, 2 * g + 1)) = f[1];
             }
-            __syncwarp();
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              const int r = 8 * j + (lane >> 2), piece = lane & 3;
-              const float4 f = *reinterpret_cast<const float4*>(stage_tile + r * STAGE_ROW + 16 * piece);
-              *reinterpret_cast<float4*>(p.Cf + (size_t)(m0 + quarter * 32 + r) * p.N + n0 + c32 + 16 * hh +
-                                         4 * piece) = f;
-            }
-            __syncwarp();
+            tile_store(tile, n0 + c32 + 16 * hh);
           }
         } else {
 #pragma unroll
@@ -572,9 +627,12 @@ __global__ void __launch_bounds__(WS_THREADS, 1)
       __syncwarp();
       if (lane == 0) mbar_arrive(smem_u32(&acc_empty[b]));
     }
+    // the stores have read their tiles and are written before the CTA exits
+    if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+    __syncwarp();
   }
   __syncthreads();
-  if (*abort_word && threadIdx.x == 0) atomicOr(p.err, 1);
+  if (*abort_word && threadIdx.x < G) atomicOr(grp.p[threadIdx.x].err, 1);
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   if (warp == 0) {
@@ -583,32 +641,77 @@ __global__ void __launch_bounds__(WS_THREADS, 1)
   }
 }
 
+// The elementwise kernels of training work on 32 x 32 tiles (256 threads, four
+// rows each), so that a transposed copy leaves through shared memory in rows
+// of 64 bytes like the plain one.  (One element per thread, transposed 2-byte
+// stores a row apart and an atomic per warp: 28 us for the loss gradient of
+// 2048 x 256 and 6 us for Adam on 512 x 512.)
+constexpr int ET = 32;
+struct TileT {
+  __nv_bfloat16 v[ET][ET + 2];
+};
+// the transposed tile (r0, c0) of a [rows][cols] array into its [cols][rows] copy
+__device__ __forceinline__ void store_transposed(const TileT& tile, bf16* out, int rows, int cols, int r0, int c0) {
+  __syncthreads();
+  const int x = threadIdx.x & 31;
+#pragma unroll
+  for (int y = threadIdx.x >> 5; y < ET; y += 8)
+    if (c0 + y < cols && r0 + x < rows) out[(size_t)(c0 + y) * rows + r0 + x] = tile.v[x][y];
+}
+
 // dY = 2 (Y - T) / count over the valid rows and columns (zero elsewhere),
 // in bf16 and transposed bf16; the squared error summed into *loss.
-__global__ void k_mse_grad(const float* __restrict__ Y, const float* __restrict__ T, int M, int N, int m_valid,
-                           int n_valid, float scale, __nv_bfloat16* __restrict__ dY,
-                           __nv_bfloat16* __restrict__ dYt, float* loss) {
-  const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(256) k_mse_grad(const float* __restrict__ Y, const float* __restrict__ T, int M,
+                                                  int N, int m_valid, int n_valid, float scale, bf16* __restrict__ dY,
+                                                  bf16* __restrict__ dYt, float* loss) {
+  __shared__ TileT tile;
+  __shared__ float red[8];
+  const int tiles_n = (N + ET - 1) / ET;
+  const int r0 = (int)(blockIdx.x / tiles_n) * ET, c0 = (int)(blockIdx.x % tiles_n) * ET;
+  const int x = threadIdx.x & 31, n = c0 + x;
   float sq = 0.0f;
-  if (i < (size_t)M * N) {
-    const int m = (int)(i / N), n = (int)(i % N);
+#pragma unroll
+  for (int y = threadIdx.x >> 5; y < ET; y += 8) {
+    const int m = r0 + y;
+    if (m >= M || n >= N) continue;
+    const size_t i = (size_t)m * N + n;
     float g = 0.0f;
     if (m < m_valid && n < n_valid) {
       const float d = Y[i] - T[i];
-      sq = d * d;
+      sq += d * d;
       g = 2.0f * d * scale;
     }
-    const __nv_bfloat16 b = __float2bfloat16_rn(g);
+    const bf16 b = __float2bfloat16_rn(g);
     dY[i] = b;
-    if (dYt) dYt[(size_t)n * M + m] = b;
+    tile.v[y][x] = b;
   }
+  if (dYt) store_transposed(tile, dYt, M, N, r0, c0);
+  if (!loss) return;
   for (int o = 16; o > 0; o >>= 1) sq += __shfl_down_sync(0xffffffffu, sq, o);
-  if ((threadIdx.x & 31) == 0 && loss) atomicAdd(loss, sq);
+  if (x == 0) red[threadIdx.x >> 5] = sq;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    sq = red[0];
+    for (int w = 1; w < 8; ++w) sq += red[w];
+    atomicAdd(loss, sq);
+  }
 }
 
-// db[n] = sum over m of dZ^T[n][m]
-__global__ void k_bias_grad(const __nv_bfloat16* __restrict__ dZt, int N, int M, float* __restrict__ db) {
-  const int n = blockIdx.x;
+// Segments of one launch: a block finds its own by the segments' first blocks.
+constexpr int SEGMENTS = 16;
+
+// db[n] = sum over m of dZ^T[n][m], a block per row
+struct BiasSegments {
+  const bf16* dZt[SEGMENTS];
+  float* db[SEGMENTS];
+  int first[SEGMENTS + 1];
+  int M;
+};
+__global__ void k_bias_grad(const __grid_constant__ BiasSegments g) {
+  int k = 0;
+  while ((int)blockIdx.x >= g.first[k + 1]) ++k;
+  const int n = blockIdx.x - g.first[k], M = g.M;
+  const bf16* dZt = g.dZt[k];
   float acc = 0.0f;
   for (int m = threadIdx.x; m < M; m += blockDim.x) acc += __bfloat162float(dZt[(size_t)n * M + m]);
   __shared__ float red[32];
@@ -618,30 +721,52 @@ __global__ void k_bias_grad(const __nv_bfloat16* __restrict__ dZt, int N, int M,
   if (threadIdx.x < 32) {
     acc = threadIdx.x < (blockDim.x >> 5) ? red[threadIdx.x] : 0.0f;
     for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
-    if (threadIdx.x == 0) db[n] = acc;
+    if (threadIdx.x == 0) g.db[k][n] = acc;
   }
 }
 
 // Adam on FP32 master weights [rows][cols] (bias when rows == 1); refreshes
-// the bf16 copy and, when given, its transpose.
-__global__ void k_adam(float* __restrict__ w, float* __restrict__ m1, float* __restrict__ m2,
-                       const float* __restrict__ g, int rows, int cols, float lr, float b1, float b2, float eps,
-                       float c1, float c2, float decay, __nv_bfloat16* __restrict__ wb, __nv_bfloat16* __restrict__ wbt) {
-  const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-  if (i >= (size_t)rows * cols) return;
-  const float gi = g[i] + decay * w[i];
-  const float a = b1 * m1[i] + (1.0f - b1) * gi;
-  const float b = b2 * m2[i] + (1.0f - b2) * gi * gi;
-  m1[i] = a;
-  m2[i] = b;
-  const float wi = w[i] - lr * (a / c1) / (sqrtf(b / c2) + eps);
-  w[i] = wi;
-  const __nv_bfloat16 h = __float2bfloat16_rn(wi);
-  if (wb) wb[i] = h;
-  if (wbt) {
-    const int r = (int)(i / cols), c = (int)(i % cols);
-    wbt[(size_t)c * rows + r] = h;
+// the bf16 copy and, when given, its transpose.  A block per 32 x 32 tile of
+// one of the segments.
+struct AdamSegment {
+  float *w, *m1, *m2;
+  const float* g;
+  bf16 *wb, *wbt;
+  int rows, cols;
+  float decay;
+};
+struct AdamSegments {
+  AdamSegment s[SEGMENTS];
+  int first[SEGMENTS + 1];
+  float lr, b1, b2, eps, c1, c2;
+};
+__global__ void __launch_bounds__(256) k_adam(const __grid_constant__ AdamSegments a) {
+  __shared__ TileT tile;
+  int k = 0;
+  while ((int)blockIdx.x >= a.first[k + 1]) ++k;
+  const AdamSegment& s = a.s[k];
+  const int local = blockIdx.x - a.first[k], tiles_c = (s.cols + ET - 1) / ET;
+  const int r0 = (local / tiles_c) * ET, c0 = (local % tiles_c) * ET;
+  const int x = threadIdx.x & 31, c = c0 + x;
+#pragma unroll
+  for (int y = threadIdx.x >> 5; y < ET; y += 8) {
+    const int r = r0 + y;
+    if (r >= s.rows || c >= s.cols) continue;
+    const size_t i = (size_t)r * s.cols + c;
+    const float gi = s.g[i] + s.decay * s.w[i];
+    // (the contractions written out, so that the weights of a training run do
+    // not depend on how the compiler schedules this loop)
+    const float m = __fmaf_rn(a.b1, s.m1[i], __fmul_rn(1.0f - a.b1, gi));
+    const float v = __fmaf_rn(a.b2, s.m2[i], __fmul_rn(__fmul_rn(1.0f - a.b2, gi), gi));
+    s.m1[i] = m;
+    s.m2[i] = v;
+    const float wi = s.w[i] - a.lr * (m / a.c1) / (sqrtf(v / a.c2) + a.eps);
+    s.w[i] = wi;
+    const bf16 h = __float2bfloat16_rn(wi);
+    if (s.wb) s.wb[i] = h;
+    tile.v[y][x] = h;
   }
+  if (s.wbt) store_transposed(tile, s.wbt, s.rows, s.cols, r0, c0);
 }
 
 // out[r][f] = bf16((raw[r][f] - mean[f]) * inv_std[f]) for r < rows and
@@ -714,20 +839,45 @@ bool make_map(CUtensorMap* m, const void* base, int rows, int K, int box_rows) {
 
 template <int BN>
 size_t ws_smem_bytes() {
-  return (size_t)WS_STAGES * (BM + BN) * BK * 2 + 1024 + 256 + 8 * 32 * STAGE_ROW;
+  return (size_t)WS_STAGES * (BM + BN) * BK * 2 + 1024 + WS_BARRIERS + WS_EPI_WARPS * STAGE_TILES * STAGE_TILE;
 }
 
-template <int BN>
-int launch_ws(const Gemm& g, cudaStream_t st) {
-  CUtensorMap ta, tb;
-  if (!make_map(&ta, g.A, g.M, g.K, BM) || !make_map(&tb, g.B, g.N, g.K, BN)) return HEXMLP_E_ARG;
+// [rows][N] results, boxes of 32 rows x 64 bytes, 64-byte swizzle
+bool make_out_map(CUtensorMap* m, void* base, int rows, int N, bool f32) {
+  EncodeTiled fn = encode_fn();
+  if (!fn) return false;
+  const cuuint64_t size = f32 ? 4 : 2;
+  const cuuint64_t dims[2] = {(cuuint64_t)N, (cuuint64_t)rows};
+  const cuuint64_t strides[1] = {(cuuint64_t)N * size};
+  const cuuint32_t box[2] = {(cuuint32_t)(64 / size), 32};
+  const cuuint32_t es[2] = {1, 1};
+  return fn(m, f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, base, dims, strides, box,
+            es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_NONE,
+            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// The n <= G products g[0..n-1], which share the tile width BN, in one launch.
+template <int BN, int G>
+int launch_ws(const Gemm* g, int n, cudaStream_t st) {
+  GemmGroup<G> grp{};
+  for (int i = 0; i < G; ++i) {
+    const Gemm& q = g[i < n ? i : n - 1];
+    grp.p[i] = q;
+    grp.first[i] = grp.tiles;
+    if (i >= n) continue;
+    if (!make_map(&grp.a[i], q.A, q.M, q.K, BM) || !make_map(&grp.b[i], q.B, q.N, q.K, BN)) return HEXMLP_E_ARG;
+    const bool f32 = q.epilogue == HEXMLP_EPI_F32;
+    void* out = f32 ? (void*)q.Cf : (void*)q.C;
+    if (out && !make_out_map(&grp.out[i], out, q.M, q.N, f32)) return HEXMLP_E_ARG;
+    grp.tiles += (q.M / BM) * (q.N / BN);
+  }
+  grp.first[G] = grp.tiles;
   static int sms = 0;
   if (!sms) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, 0);
   const size_t smem = ws_smem_bytes<BN>();
-  cudaError_t e = cudaFuncSetAttribute(k_gemm_ws<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = cudaFuncSetAttribute(k_gemm_ws<BN, G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return (int)e;
-  const int tiles = (g.M / BM) * (g.N / BN);
-  k_gemm_ws<BN><<<tiles < sms ? tiles : sms, WS_THREADS, smem, st>>>(ta, tb, g);
+  k_gemm_ws<BN, G><<<grp.tiles < sms ? grp.tiles : sms, WS_THREADS, smem, st>>>(grp);
   return (int)cudaGetLastError();
 }
 
@@ -735,7 +885,7 @@ int launch_ws(const Gemm& g, cudaStream_t st) {
 
 namespace {
 
-int gemm_impl(const HexMlpGemm* p, uint32_t mma_wait_polls, void* stream) {
+int checked(const HexMlpGemm* p, uint32_t mma_wait_polls, Gemm* out) {
   if (!p || !p->A || !p->B || !p->err) return HEXMLP_E_ARG;
   if (p->M <= 0 || p->N <= 0 || p->K <= 0 || p->M % BM || p->K % BK) return HEXMLP_E_ARG;
   if (!(p->bn == 128 || p->bn == 256) || p->N % p->bn) return HEXMLP_E_ARG;
@@ -747,24 +897,52 @@ int gemm_impl(const HexMlpGemm* p, uint32_t mma_wait_polls, void* stream) {
   const void* ptrs[] = {p->A, p->B, p->C, p->Z, p->Zin, p->Cf, p->bias};
   for (const void* q : ptrs)
     if (q && ((uintptr_t)q & 15u)) return HEXMLP_E_ARG;
+  *out = Gemm{(const bf16*)p->A, (const bf16*)p->B, p->M, p->N, p->K, p->bn, p->epilogue, p->bias, (bf16*)p->C,
+              (bf16*)p->Ct, (bf16*)p->Z, (const bf16*)p->Zin, p->Cf, p->err, mma_wait_polls};
+  return 0;
+}
+
+int gemm_impl(const HexMlpGemm* p, uint32_t mma_wait_polls, void* stream) {
+  Gemm g;
+  const int rc = checked(p, mma_wait_polls, &g);
+  if (rc) return rc;
+  if (p->kernel == HEXMLP_GEMM_PERSISTENT)
+    return p->bn == 256 ? launch_ws<256, 1>(&g, 1, (cudaStream_t)stream)
+                        : launch_ws<128, 1>(&g, 1, (cudaStream_t)stream);
+  if (p->kernel != HEXMLP_GEMM_STAGED || mma_wait_polls != WAIT_LIMIT) return HEXMLP_E_ARG;
   const size_t smem = hexmlp_gemm_smem_bytes(p->bn);
   cudaError_t e = cudaFuncSetAttribute(k_gemm_bf16, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return (int)e;
-  const Gemm g{(const bf16*)p->A, (const bf16*)p->B, p->M, p->N, p->K, p->bn, p->epilogue, p->bias, (bf16*)p->C,
-               (bf16*)p->Ct, (bf16*)p->Z, (const bf16*)p->Zin, p->Cf, p->err, mma_wait_polls};
-  if (p->kernel == HEXMLP_GEMM_PERSISTENT)
-    return p->bn == 256 ? launch_ws<256>(g, (cudaStream_t)stream) : launch_ws<128>(g, (cudaStream_t)stream);
-  if (p->kernel != HEXMLP_GEMM_STAGED || mma_wait_polls != WAIT_LIMIT) return HEXMLP_E_ARG;
   dim3 grid(p->M / BM, p->N / p->bn);
   k_gemm_bf16<<<grid, THREADS, smem, (cudaStream_t)stream>>>(g);
   return (int)cudaGetLastError();
 }
+
+constexpr int GROUP = 8;  // products of one grouped launch
 
 }  // namespace
 
 extern "C" {
 
 int hexmlp_gemm(const HexMlpGemm* p, void* stream) { return gemm_impl(p, WAIT_LIMIT, stream); }
+
+int hexmlp_gemm_group(const HexMlpGemm* p, int n, void* stream) {
+  if (!p || n < 0) return HEXMLP_E_ARG;
+  Gemm g[GROUP];
+  for (int i = 0; i < n; ++i) {  // nothing is launched if any is refused
+    const int rc = checked(p + i, WAIT_LIMIT, g);
+    if (rc) return rc;
+    if (p[i].kernel != HEXMLP_GEMM_PERSISTENT || p[i].bn != p[0].bn) return HEXMLP_E_ARG;
+  }
+  for (int i = 0; i < n; i += GROUP) {
+    const int m = n - i < GROUP ? n - i : GROUP;
+    for (int q = 0; q < m; ++q) checked(p + i + q, WAIT_LIMIT, g + q);
+    const int rc = p[0].bn == 256 ? launch_ws<256, GROUP>(g, m, (cudaStream_t)stream)
+                                  : launch_ws<128, GROUP>(g, m, (cudaStream_t)stream);
+    if (rc) return rc;
+  }
+  return 0;
+}
 
 int hexmlp_gemm_wait_limit(const HexMlpGemm* p, uint32_t mma_wait_polls, void* stream) {
   if (!p || p->kernel != HEXMLP_GEMM_PERSISTENT) return HEXMLP_E_ARG;
@@ -776,29 +954,71 @@ int hexmlp_mse_grad(const float* Y, const float* T, int M, int N, int m_valid, i
   bf16* dY = (bf16*)dY_;
   bf16* dYt = (bf16*)dYt_;
   if (!Y || !T || !dY || M <= 0 || N <= 0) return HEXMLP_E_ARG;
-  const size_t n = (size_t)M * N;
-  k_mse_grad<<<(unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream>>>(Y, T, M, N, m_valid, n_valid, scale,
+  const size_t tiles = (size_t)((M + ET - 1) / ET) * ((N + ET - 1) / ET);
+  k_mse_grad<<<(unsigned)tiles, 256, 0, (cudaStream_t)stream>>>(Y, T, M, N, m_valid, n_valid, scale,
                                                                           dY, dYt, loss);
   return (int)cudaGetLastError();
 }
 
-int hexmlp_bias_grad(const void* dZt_, int N, int M, float* db, void* stream) {
-  const bf16* dZt = (const bf16*)dZt_;
-  if (!dZt || !db || N <= 0 || M <= 0) return HEXMLP_E_ARG;
-  k_bias_grad<<<N, 256, 0, (cudaStream_t)stream>>>(dZt, N, M, db);
-  return (int)cudaGetLastError();
+int hexmlp_bias_grad(const void* dZt, int N, int M, float* db, void* stream) {
+  return hexmlp_bias_grads(&dZt, &N, &db, 1, M, stream);
+}
+
+int hexmlp_bias_grads(const void* const* dZt, const int* N, float* const* db, int n, int M, void* stream) {
+  if (!dZt || !N || !db || n < 0 || M <= 0) return HEXMLP_E_ARG;
+  for (int i = 0; i < n; ++i)
+    if (!dZt[i] || !db[i] || N[i] <= 0) return HEXMLP_E_ARG;
+  for (int i = 0; i < n; i += SEGMENTS) {
+    BiasSegments g{};
+    int blocks = 0;
+    for (int k = 0; k < SEGMENTS; ++k) {
+      g.first[k] = blocks;
+      if (i + k >= n) continue;
+      g.dZt[k] = (const bf16*)dZt[i + k];
+      g.db[k] = db[i + k];
+      blocks += N[i + k];
+    }
+    g.first[SEGMENTS] = blocks;
+    g.M = M;
+    k_bias_grad<<<blocks, 256, 0, (cudaStream_t)stream>>>(g);
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return (int)e;
+  }
+  return 0;
 }
 
 int hexmlp_adam(float* w, float* m1, float* m2, const float* g, int rows, int cols, float lr, float b1, float b2,
-                float eps, int t, float decay, void* wb_, void* wbt_, void* stream) {
-  bf16* wb = (bf16*)wb_;
-  bf16* wbt = (bf16*)wbt_;
-  if (!w || !m1 || !m2 || !g || rows <= 0 || cols <= 0 || t < 1) return HEXMLP_E_ARG;
-  const float c1 = 1.0f - powf(b1, (float)t), c2 = 1.0f - powf(b2, (float)t);
-  const size_t n = (size_t)rows * cols;
-  k_adam<<<(unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream>>>(w, m1, m2, g, rows, cols, lr, b1, b2, eps,
-                                                                      c1, c2, decay, wb, wbt);
-  return (int)cudaGetLastError();
+                float eps, int t, float decay, void* wb, void* wbt, void* stream) {
+  const HexMlpAdam s{w, m1, m2, g, wb, wbt, rows, cols, decay};
+  return hexmlp_adam_layers(&s, 1, lr, b1, b2, eps, t, stream);
+}
+
+int hexmlp_adam_layers(const HexMlpAdam* p, int n, float lr, float b1, float b2, float eps, int t, void* stream) {
+  if (!p || n < 0 || t < 1) return HEXMLP_E_ARG;
+  for (int i = 0; i < n; ++i)
+    if (!p[i].w || !p[i].m1 || !p[i].m2 || !p[i].g || p[i].rows <= 0 || p[i].cols <= 0) return HEXMLP_E_ARG;
+  for (int i = 0; i < n; i += SEGMENTS) {
+    AdamSegments a{};
+    a.lr = lr;
+    a.b1 = b1;
+    a.b2 = b2;
+    a.eps = eps;
+    a.c1 = 1.0f - powf(b1, (float)t);
+    a.c2 = 1.0f - powf(b2, (float)t);
+    int blocks = 0;
+    for (int k = 0; k < SEGMENTS; ++k) {
+      a.first[k] = blocks;
+      if (i + k >= n) continue;
+      const HexMlpAdam& q = p[i + k];
+      a.s[k] = AdamSegment{q.w, q.m1, q.m2, q.g, (bf16*)q.wb, (bf16*)q.wbt, q.rows, q.cols, q.decay};
+      blocks += ((q.rows + ET - 1) / ET) * ((q.cols + ET - 1) / ET);
+    }
+    a.first[SEGMENTS] = blocks;
+    k_adam<<<blocks, 256, 0, (cudaStream_t)stream>>>(a);
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return (int)e;
+  }
+  return 0;
 }
 
 }  // extern "C"

@@ -31,11 +31,19 @@ class HexMlpGemm(C.Structure):
                 ("err", C.c_void_p), ("kernel", C.c_int32)]
 
 
+class HexMlpAdam(C.Structure):
+    _fields_ = [("w", C.c_void_p), ("m1", C.c_void_p), ("m2", C.c_void_p), ("g", C.c_void_p), ("wb", C.c_void_p),
+                ("wbt", C.c_void_p), ("rows", C.c_int32), ("cols", C.c_int32), ("decay", C.c_float)]
+
+
 GEMM_PERSISTENT, GEMM_STAGED = 0, 1
+# tiles of a launch below which 256 columns a tile leave SMs of the 148 idle
+FULL_GRID = 148
 
 
 MLP_EXPORTS = {
     "hexmlp_gemm": (C.c_int, [C.POINTER(HexMlpGemm), C.c_void_p]),
+    "hexmlp_gemm_group": (C.c_int, [C.POINTER(HexMlpGemm), C.c_int, C.c_void_p]),
     "hexmlp_gemm_wait_limit": (C.c_int, [C.POINTER(HexMlpGemm), C.c_uint32, C.c_void_p]),
     "hexmlp_gemm_smem_bytes": (C.c_size_t, [C.c_int]),
     "hexmlp_gemm_tile_rows": (C.c_int, []),
@@ -43,11 +51,15 @@ MLP_EXPORTS = {
     "hexmlp_mse_grad": (C.c_int, [C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_int, C.c_float,
                                   C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p]),
     "hexmlp_bias_grad": (C.c_int, [C.c_void_p, C.c_int, C.c_int, C.c_void_p, C.c_void_p]),
+    "hexmlp_bias_grads": (C.c_int, [C.POINTER(C.c_void_p), C.POINTER(C.c_int), C.POINTER(C.c_void_p), C.c_int,
+                                    C.c_int, C.c_void_p]),
     "hexmlp_pack": (C.c_int, [C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_void_p, C.c_void_p, C.c_int, C.c_int,
                               C.c_void_p, C.c_void_p, C.c_void_p]),
     "hexmlp_adam": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_float,
                               C.c_float, C.c_float, C.c_float, C.c_int, C.c_float, C.c_void_p, C.c_void_p,
                               C.c_void_p]),
+    "hexmlp_adam_layers": (C.c_int, [C.POINTER(HexMlpAdam), C.c_int, C.c_float, C.c_float, C.c_float, C.c_float,
+                                     C.c_int, C.c_void_p]),
 }
 
 
@@ -81,30 +93,40 @@ def round_up(x: int, m: int) -> int:
     return (x + m - 1) // m * m
 
 
-def gemm(A, B, *, epilogue: int = EPI_F32, bias=None, C_out=None, Ct=None, Z=None, Zin=None, Cf=None, err=None,
-         bn: int | None = None, kernel: int = GEMM_PERSISTENT, mma_wait_polls: int | None = None):
-    """C = A . B^T on the tensor cores (see include/hexmlp.h).  ``bn``: the
-    output tile width, 128 or 256 (default: 256 where N allows it for the
-    persistent kernel, 128 for the staged one).  ``mma_wait_polls`` bounds
-    the MMA issuer's wait for each loaded stage (``hexmlp_gemm_wait_limit``,
-    a check of the kernel's give-up path; None: the normal limit)."""
+def _problem(A, B, bn, epilogue, bias, C_out, Ct, Z, Zin, Cf, err, kernel) -> HexMlpGemm:
     import torch
 
     M, K = A.shape
     N = B.shape[0]
     assert B.shape[1] == K and A.dtype == torch.bfloat16 and B.dtype == torch.bfloat16
     assert A.is_contiguous() and B.is_contiguous()
+    if bn is None:
+        bn = 128
+        if kernel == GEMM_PERSISTENT and N % 256 == 0 and (M // TILE_M) * (N // 256) >= FULL_GRID:
+            bn = 256
+    return HexMlpGemm(_ptr(A), _ptr(B), M, N, K, bn, epilogue, _ptr(bias), _ptr(C_out), _ptr(Ct), _ptr(Z), _ptr(Zin),
+                      _ptr(Cf), _ptr(err), kernel)
+
+
+def gemm(A, B, *, epilogue: int = EPI_F32, bias=None, C_out=None, Ct=None, Z=None, Zin=None, Cf=None, err=None,
+         bn: int | None = None, kernel: int = GEMM_PERSISTENT, mma_wait_polls: int | None = None):
+    """C = A . B^T on the tensor cores (see include/hexmlp.h).  ``bn``: the
+    output tile width, 128 or 256 (default: 256 for the persistent kernel
+    where N allows it and those tiles fill the GPU, else 128: a training
+    batch of 2048 rows x 512 columns is 32 tiles of 256 or 64 of 128).  ``mma_wait_polls`` bounds
+    the MMA issuer's wait for each loaded stage (``hexmlp_gemm_wait_limit``,
+    a check of the kernel's give-up path; None: the normal limit)."""
+    import torch
+
     if err is None:
         err = torch.zeros(1, dtype=torch.int32, device=A.device)
-    if bn is None:
-        bn = 256 if (kernel == GEMM_PERSISTENT and N % 256 == 0) else 128
-    p = HexMlpGemm(_ptr(A), _ptr(B), M, N, K, bn, epilogue, _ptr(bias), _ptr(C_out), _ptr(Ct), _ptr(Z), _ptr(Zin),
-                   _ptr(Cf), _ptr(err), kernel)
+    p = _problem(A, B, bn, epilogue, bias, C_out, Ct, Z, Zin, Cf, err, kernel)
     if mma_wait_polls is None:
-        _check(load().hexmlp_gemm(C.byref(p), _stream()), f"hexmlp_gemm {M}x{N}x{K}")
+        rc = load().hexmlp_gemm(C.byref(p), _stream())
     else:
-        _check(load().hexmlp_gemm_wait_limit(C.byref(p), int(mma_wait_polls), _stream()),
-               f"hexmlp_gemm_wait_limit {M}x{N}x{K}")
+        rc = load().hexmlp_gemm_wait_limit(C.byref(p), int(mma_wait_polls), _stream())
+    if rc != 0:
+        _check(rc, f"hexmlp_gemm {p.M}x{p.N}x{p.K}")
     return err
 
 
@@ -164,18 +186,17 @@ class TensorCoreMLP:
         if ws is None:
             dev = self.layers[0].w.device
             bf = dict(dtype=torch.bfloat16, device=dev)
-            ws = {"H": [], "Ht": [], "Z": []}
+            ws = {"H": [], "Ht": [], "Z": [], "dZt": []}
             for _ in range(self.depth):
                 ws["H"].append(torch.empty(M, self.p_hidden, **bf))
                 ws["Ht"].append(torch.empty(self.p_hidden, M, **bf))
                 ws["Z"].append(torch.empty(M, self.p_hidden, **bf))
+                ws["dZt"].append(torch.empty(self.p_hidden, M, **bf))
             ws["Y"] = torch.empty(M, self.p_out, dtype=torch.float32, device=dev)
             ws["dY"] = torch.empty(M, self.p_out, **bf)
             ws["dYt"] = torch.empty(self.p_out, M, **bf)
             ws["dZ"] = torch.empty(M, self.p_hidden, **bf)
-            ws["dZt"] = torch.empty(self.p_hidden, M, **bf)
             ws["dZ2"] = torch.empty(M, self.p_hidden, **bf)
-            ws["dZt2"] = torch.empty(self.p_hidden, M, **bf)
             ws["Xt"] = torch.empty(self.p_in, M, **bf)
             ws["loss"] = torch.zeros(1, dtype=torch.float32, device=dev)
             self._ws[M] = ws
@@ -209,31 +230,38 @@ class TensorCoreMLP:
         scale = 1.0 / float(m_valid * self.n_out)
         _check(lib.hexmlp_mse_grad(_ptr(Y), _ptr(T), M, self.p_out, m_valid, self.n_out, scale, _ptr(ws["dY"]),
                                    _ptr(ws["dYt"]), _ptr(ws["loss"]), _stream()), "mse_grad")
-        d, dt = ws["dY"], ws["dYt"]
-        bufs = [(ws["dZ"], ws["dZt"]), (ws["dZ2"], ws["dZt2"])]
-        for i in range(self.depth, -1, -1):
-            lay = self.layers[i]
-            prev_t = ws["Ht"][i - 1] if i > 0 else Xt
-            # dW = dZ^T . A_prev (A_prev^T rows are the B operand), db = sum dZ
-            gemm(dt, prev_t, epilogue=EPI_F32, Cf=lay.gw, err=self.err)
-            _check(lib.hexmlp_bias_grad(_ptr(dt), dt.shape[0], M, _ptr(lay.gb), _stream()), "bias_grad")
-            if i > 0:
-                nd, ndt = bufs[i % 2]
-                # dA_prev = dZ . W, times GELU'(Z_prev)
-                gemm(d, lay.wbt, epilogue=EPI_GELU_GRAD, C_out=nd, Ct=ndt, Zin=ws["Z"][i - 1], err=self.err)
-                d, dt = nd, ndt
+        # dA_prev = dZ . W, times GELU'(Z_prev), from the last layer down
+        d = ws["dY"]
+        for i in range(self.depth, 0, -1):
+            nd = ws["dZ2" if i % 2 else "dZ"]
+            gemm(d, self.layers[i].wbt, epilogue=EPI_GELU_GRAD, C_out=nd, Ct=ws["dZt"][i - 1], Zin=ws["Z"][i - 1],
+                 err=self.err)
+            d = nd
+        # dW = dZ^T . A_prev (A_prev^T rows are the B operand) and db = sum dZ
+        # of every layer at once: a layer's gradient alone is 12 to 16 tiles
+        # for 148 SMs
+        n = self.depth + 1
+        dts = [*ws["dZt"], ws["dYt"]]
+        prevs = [Xt, *ws["Ht"]]
+        problems = (HexMlpGemm * n)(*[
+            _problem(dts[i], prevs[i], 128, EPI_F32, None, None, None, None, None, self.layers[i].gw, self.err,
+                     GEMM_PERSISTENT) for i in range(n)])
+        _check(lib.hexmlp_gemm_group(problems, n, _stream()), "hexmlp_gemm_group")
+        _check(lib.hexmlp_bias_grads((C.c_void_p * n)(*map(_ptr, dts)), (C.c_int * n)(*[t.shape[0] for t in dts]),
+                                     (C.c_void_p * n)(*[_ptr(lay.gb) for lay in self.layers]), n, M, _stream()),
+               "bias_grads")
         return ws["loss"]
 
     def adam(self, lr: float, *, b1: float = 0.9, b2: float = 0.999, eps: float = 1e-8, decay: float = 0.0):
-        lib = load()
         self.step_count += 1
-        st = _stream()
+        parts = []
         for lay in self.layers:
             rows, cols = lay.w.shape
-            _check(lib.hexmlp_adam(_ptr(lay.w), _ptr(lay.m1), _ptr(lay.m2), _ptr(lay.gw), rows, cols, lr, b1, b2,
-                                   eps, self.step_count, decay, _ptr(lay.wb), _ptr(lay.wbt), st), "adam")
-            _check(lib.hexmlp_adam(_ptr(lay.b), _ptr(lay.bm1), _ptr(lay.bm2), _ptr(lay.gb), 1, rows, lr, b1, b2,
-                                   eps, self.step_count, 0.0, None, None, st), "adam bias")
+            parts.append(HexMlpAdam(_ptr(lay.w), _ptr(lay.m1), _ptr(lay.m2), _ptr(lay.gw), _ptr(lay.wb),
+                                    _ptr(lay.wbt), rows, cols, decay))
+            parts.append(HexMlpAdam(_ptr(lay.b), _ptr(lay.bm1), _ptr(lay.bm2), _ptr(lay.gb), None, None, 1, rows, 0.0))
+        _check(load().hexmlp_adam_layers((HexMlpAdam * len(parts))(*parts), len(parts), lr, b1, b2, eps,
+                                         self.step_count, _stream()), "adam")
 
     def check(self) -> None:
         if int(self.err.item()) != 0:

@@ -54,6 +54,9 @@ typedef struct HexMlpGemm {
 #define HEXMLP_GEMM_STAGED 1
 
 int hexmlp_gemm(const HexMlpGemm* p, void* stream);
+/* n independent products of one tile width (HEXMLP_GEMM_PERSISTENT), up to
+ * eight to a launch: the tiles of all share the SMs. */
+int hexmlp_gemm_group(const HexMlpGemm* p, int n, void* stream);
 /* Check of the persistent GEMM's failure path: hexmlp_gemm with the MMA
  * issuer's wait for each loaded stage bounded by `mma_wait_polls` mbarrier
  * polls instead of 2^20.  With 0 that wait gives up before the first stage
@@ -73,12 +76,27 @@ int hexmlp_mse_grad(const float* Y, const float* T, int M, int N, int m_valid, i
 
 /* db[n] = sum over m of dZt[n][m] (bf16 [N][M]). */
 int hexmlp_bias_grad(const void* dZt, int N, int M, float* db, void* stream);
+/* The same for n arrays dZt[i] ([N[i]][M]) in one launch for every 16. */
+int hexmlp_bias_grads(const void* const* dZt, const int* N, float* const* db, int n, int M, void* stream);
 
 /* Adam step t (1-based) on FP32 weights w [rows][cols] with moments m1, m2
  * and gradient g (L2 decay `decay`); refreshes the bf16 copy wb and, if
  * given, its transpose wbt [cols][rows]. */
 int hexmlp_adam(float* w, float* m1, float* m2, const float* g, int rows, int cols, float lr, float b1, float b2,
                 float eps, int t, float decay, void* wb, void* wbt, void* stream);
+
+/* The same step on n arrays in one launch for every 16. */
+typedef struct HexMlpAdam {
+  float* w;
+  float* m1;
+  float* m2;
+  const float* g;
+  void* wb;   /* bf16 copy or NULL */
+  void* wbt;  /* its transpose or NULL */
+  int32_t rows, cols;
+  float decay;
+} HexMlpAdam;
+int hexmlp_adam_layers(const HexMlpAdam* p, int n, float lr, float b1, float b2, float eps, int t, void* stream);
 
 /* Normalise and pack network inputs: out[r][f] = bf16((raw[r][f] -
  * mean[f]) * inv_std[f]) for r < rows, f < n_feat; zero in the padding of
