@@ -34,9 +34,16 @@ struct Launcher {
   // join() makes the caller's stream wait for them.  Serial (no-ops) when
   // the context has no side stream or launches are being profiled.
   int region = 0;  // the forked region being launched (bit of ctx.concurrent_regions)
+  // (A step of a small mesh under a host hook is paced by its launches: the
+  // forks' events cost more there than the overlap gives, two steps of
+  // 2562 x 55 under a physics callback 3713 -> 3549 us.)
   bool concurrent() const {
-    return ctx.side_stream != nullptr && prof == nullptr && (ctx.concurrent_regions & region);
+    if (ctx.side_stream == nullptr || prof != nullptr || !(ctx.concurrent_regions & region)) return false;
+    const bool hooked = ctx.stage_hook != nullptr || ctx.exchange_hook != nullptr;
+    return !(hooked && (long long)ctx.geo.nE * (ctx.geo.S / 4) <= RESIDENT_CHUNKS);
   }
+  // chunks of a launch that four 256-thread blocks on each of 148 SMs hold at once
+  static constexpr long long RESIDENT_CHUNKS = 256LL * 4 * 148;
   void signal(cudaStream_t from, cudaStream_t to) {
     if (err != cudaSuccess) return;
     cudaEvent_t ev = ctx.fork_events[next_event++ & 3];
@@ -135,11 +142,10 @@ struct Launcher {
     // programmatic edge of the captured graph).  Two steps of 162 x 12: 674 ->
     // 634 us, 642 x 41: 976 -> 952, 10242 x 55 with mixing: 3960 -> 3875,
     // x1.40962 x 55: 11051 -> 11020.  Not for grids between PRELOAD_CHUNKS and
-    // four 256-thread blocks per SM, which share the SMs with the other stream's
-    // kernel at once: waiting blocks take its slots (2562 x 55: 1086 -> 1134).
+    // RESIDENT_CHUNKS, which share the SMs with the other stream's kernel at once: waiting blocks take its slots (2562 x 55: 1086 -> 1134).
     const long long chunks = (long long)grid.x * grid.z * block.x * block.y;
     bool& ch = chained[on_side];
-    if (vec && ch && !prof && (chunks <= PRELOAD_CHUNKS || chunks > 256LL * 4 * 148)) {
+    if (vec && ch && !prof && (chunks <= PRELOAD_CHUNKS || chunks > RESIDENT_CHUNKS)) {
       cudaLaunchAttribute at{};
       at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
       at.val.programmaticStreamSerializationAllowed = 1;

@@ -395,16 +395,21 @@ class HexDycoreDriver:
         t = torch.as_tensor(_CudaArray(ptr.value, (n, self.level_stride), self), device="cuda")
         return t[:, : self.sizes["n_levels"]].t()
 
-    def _field_view(self, ptr: int, name: str):
+    def _field_view(self, ptr: int, name: str, bases: dict):
+        """Logical view of the library's buffer of a field; ``bases`` holds the
+        buffers wrapped so far by address and field."""
         import torch
 
         n, blocks = self._entities(name)
         rows = self._rows(name)
-        if blocks > 1:
+        t = bases.get((ptr, name))
+        if t is None:
             t = torch.as_tensor(_CudaArray(ptr, (blocks * n, self.level_stride), self), device="cuda")
-            return t[:, :rows].reshape(blocks, n, rows).transpose(1, 2)
-        t = torch.as_tensor(_CudaArray(ptr, (n, self.level_stride), self), device="cuda")
-        return t[:, :rows].t()
+            bases[(ptr, name)] = t
+        S = self.level_stride
+        if blocks > 1:
+            return t.as_strided((blocks, rows, n), (n * S, 1, S))
+        return t.as_strided((rows, n), (1, S))
 
     def _step_with_stage_callback(self, callback) -> DeviceStepResult:
         """One eager step with ``callback`` run before every RK stage
@@ -419,11 +424,20 @@ class HexDycoreDriver:
                    (_lib.PHYS_DIABATIC_THETA, "diabatic_theta"))
         stream = torch.cuda.ExternalStream(self._stream_handle().value or 0) if self._stream is not None else None
         t0 = self.time_seconds
+        # The stages of a step pass four sets of the library's buffers among
+        # them: a buffer is wrapped once a step, and every stage takes views of
+        # its own from that.
+        bases: dict = {}
+
+        def physics_view(which):
+            if which not in bases:
+                bases[which] = self._physics_view(which)
+            return bases[which]
 
         def hook(user, substep, rk_step, fields):
             try:
                 f = fields.contents
-                views = {name: self._field_view(f.field[i], name) for name, i in _lib.FIELDS.items()
+                views = {name: self._field_view(f.field[i], name, bases) for name, i in _lib.FIELDS.items()
                          if f.field[i] and not (name == "scalars" and self.sizes["n_scalars"] == 0)}
                 state = SimpleNamespace(**{k: views[k] for k in _lib.STATE_FIELDS if k in views}, time_seconds=t0)
                 saved = SimpleNamespace(**{k: views[k] for k in _lib.SIDECAR_FIELDS})
@@ -437,7 +451,7 @@ class HexDycoreDriver:
                         value = getattr(tend, name, None)
                         if value is None:
                             continue
-                        dst = self._physics_view(bit)
+                        dst = physics_view(bit)
                         src = torch.as_tensor(value, device="cuda", dtype=torch.float32)
                         if tuple(src.shape) != tuple(dst.shape):
                             raise ValueError(f"physics {name} shape {tuple(src.shape)} != {tuple(dst.shape)}")
