@@ -364,8 +364,8 @@ __global__ void __launch_bounds__(THREADS, 2) k_gemm_bf16(Gemm p) {
 // mbarrier) into an NS-stage ring; warp 1 (one lane) issues four K=16
 // tcgen05.mma per slab into one of two tensor-memory accumulators and
 // commits each slab to the stage's "empty" mbarrier and each finished tile
-// to the accumulator's "full" mbarrier; warps 2..9 drain the other
-// accumulator (warp w reads lanes 32(w%4).. and one half of the columns),
+// to the accumulator's "full" mbarrier; warps 2..17 drain the other
+// accumulator (warp w reads lanes 32(w%4).. and one quarter of the columns),
 // apply the epilogue and store, then release the accumulator.  The
 // epilogue of tile i thus overlaps the loads and MMAs of tile i+1.  Every
 // wait is bounded; a role that gives up raises the CTA's abort word and
@@ -373,15 +373,18 @@ __global__ void __launch_bounds__(THREADS, 2) k_gemm_bf16(Gemm p) {
 // producer waits for every TMA load it issued to land and the MMA issuer
 // commits a drain barrier and waits for every MMA it issued, so no
 // asynchronous copy or MMA is in flight at exit on either path.
-constexpr int WS_EPI_WARPS = 8;  // two per lane quarter, each half of the tile's columns
+// Epilogue warps, four per lane quarter, each a quarter of the tile's columns.
+// With two per quarter a scheduler had two warps of dependent work (issue 34 %
+// busy, no pipe above 20 %) and the epilogue set the pace: 41088 x 512 x 512
+// with GELU 33.9 -> 29.7 us, 122880 x 256 x 256 41.0 -> 32.9, 41088 x 256 x 512
+// FP32 out 22.7 -> 20.6.
+constexpr int WS_EPI_WARPS = 16;
 constexpr int WS_THREADS = 64 + 32 * WS_EPI_WARPS;
 constexpr int WS_STAGES = 4;
-// An epilogue warp's staging tiles: 32 rows of 64 bytes each, the 16-byte
-// pieces of a row permuted as the 64-byte TMA swizzle has them (which spreads
-// a column of pieces over the banks).  Two, so that one fills while the TMA
-// store reads the other.
+// An epilogue warp's staging tile: 32 rows of 64 bytes, the 16-byte pieces of
+// a row permuted as the 64-byte TMA swizzle has them (which spreads a column
+// of pieces over the banks).
 constexpr int STAGE_TILE = 32 * 64;
-constexpr int STAGE_TILES = 2;
 constexpr int WS_BARRIERS = 512;  // mbarriers; the staging tiles after them start on the swizzle's 512 bytes
 __device__ __forceinline__ int stage_at(int row, int piece) { return row * 64 + 16 * (piece ^ ((row >> 1) & 3)); }
 
@@ -546,14 +549,14 @@ __global__ void __launch_bounds__(WS_THREADS, 1) k_gemm_ws(const __grid_constant
       if (!mbar_wait(smem_u32(drain), 0)) *abort_word = 1;
     }
   } else {
-    // epilogue warps 2..9: lane quarter warp % 4, column half (warp - 2) / 4
+    // epilogue warps 2..17: lane quarter warp % 4, columns part (warp - 2) / 4
     constexpr int PART = BN / (WS_EPI_WARPS / 4);
     const int quarter = warp & 3, part = (warp - 2) >> 2;
     // activations and FP32 results leave through the staging tiles by TMA
     // stores (a warp's 32 rows x 64 bytes each): the stores need neither
     // shared-memory reads nor address arithmetic of the warps that set the pace
-    uint8_t* stage_tile = smem + WS_STAGES * STAGE + WS_BARRIERS + (warp - 2) * STAGE_TILES * STAGE_TILE;
-    int tc = 0, gi = 0, buf = 0;
+    uint8_t* stage_tile = smem + WS_STAGES * STAGE + WS_BARRIERS + (warp - 2) * STAGE_TILE;
+    int tc = 0, gi = 0;
     for (int t = blockIdx.x; t < tiles; t += gridDim.x, ++tc) {
       const int b = tc & 1;
       int m0, n0;
@@ -572,51 +575,47 @@ __global__ void __launch_bounds__(WS_THREADS, 1) k_gemm_ws(const __grid_constant
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const int row0 = m0 + quarter * 32, row = row0 + lane;
       const uint32_t base = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(b * BN);
-      // a staging tile that no TMA store is still reading: at most the other
-      // tile's store may be in flight
+      // the staging tile, once no TMA store is reading it
       const auto tile_ready = [&]() {
-        if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+        if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
         __syncwarp();
       };
       // the staged tile out to columns x.. of this warp's rows
-      const auto tile_store = [&](uint8_t* tile, int x) {
+      const auto tile_store = [&](int x) {
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncwarp();
         if (lane == 0) {
-          tma_store_2d(&grp.out[gi], x, row0, smem_u32(tile));
+          tma_store_2d(&grp.out[gi], x, row0, smem_u32(stage_tile));
           asm volatile("cp.async.bulk.commit_group;" ::: "memory");
         }
-        buf ^= 1;
       };
       for (int c32 = part * PART; c32 < (part + 1) * PART; c32 += 32) {
         float v32[32];
         tmem_ld32(base + (uint32_t)c32, v32);
         if (staged) {
           // this lane's row of 32 activations
-          uint8_t* tile = stage_tile + buf * STAGE_TILE;
           tile_ready();
 #pragma unroll
           for (int g8 = 0; g8 < 4; ++g8) {
             uint4 h;
             epilogue8(p, row, n0 + c32 + 8 * g8, v32 + 8 * g8, &h);
-            *reinterpret_cast<uint4*>(tile + stage_at(lane, g8)) = h;
+            *reinterpret_cast<uint4*>(stage_tile + stage_at(lane, g8)) = h;
           }
-          tile_store(tile, n0 + c32);
+          tile_store(n0 + c32);
         } else if (staged_f32) {
           // FP32 out: two halves of 16 columns (64 bytes a row)
 #pragma unroll
           for (int hh = 0; hh < 2; ++hh) {
-            uint8_t* tile = stage_tile + buf * STAGE_TILE;
             tile_ready();
 #pragma unroll
             for (int g = 0; g < 2; ++g) {
               const int g8 = 2 * hh + g;
               float4 f[2];
               epilogue8(p, row, n0 + c32 + 8 * g8, v32 + 8 * g8, nullptr, f);
-              *reinterpret_cast<float4*>(tile + stage_at(lane, 2 * g)) = f[0];
-              *reinterpret_cast<float4*>(tile + stage_at(lane, 2 * g + 1)) = f[1];
+              *reinterpret_cast<float4*>(stage_tile + stage_at(lane, 2 * g)) = f[0];
+              *reinterpret_cast<float4*>(stage_tile + stage_at(lane, 2 * g + 1)) = f[1];
             }
-            tile_store(tile, n0 + c32 + 16 * hh);
+            tile_store(n0 + c32 + 16 * hh);
           }
         } else {
 #pragma unroll
@@ -839,7 +838,7 @@ bool make_map(CUtensorMap* m, const void* base, int rows, int K, int box_rows) {
 
 template <int BN>
 size_t ws_smem_bytes() {
-  return (size_t)WS_STAGES * (BM + BN) * BK * 2 + 1024 + WS_BARRIERS + WS_EPI_WARPS * STAGE_TILES * STAGE_TILE;
+  return (size_t)WS_STAGES * (BM + BN) * BK * 2 + 1024 + WS_BARRIERS + WS_EPI_WARPS * STAGE_TILE;
 }
 
 // [rows][N] results, boxes of 32 rows x 64 bytes, 64-byte swizzle
