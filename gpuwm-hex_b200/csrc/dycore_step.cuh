@@ -140,12 +140,18 @@ struct Launcher {
     // its blocks may be set up while that runs (programmatic stream
     // serialisation; only after a kernel of this step on the same stream, and a
     // programmatic edge of the captured graph).  Two steps of 162 x 12: 674 ->
-    // 634 us, 642 x 41: 976 -> 952, 10242 x 55 with mixing: 3960 -> 3875,
-    // x1.40962 x 55: 11051 -> 11020.  Not for grids between PRELOAD_CHUNKS and
-    // RESIDENT_CHUNKS, which share the SMs with the other stream's kernel at once: waiting blocks take its slots (2562 x 55: 1086 -> 1134).
+    // 634 us, 642 x 41: 976 -> 952, 10242 x 55 with mixing: 3960 -> 3875.
+    // Not for grids between PRELOAD_CHUNKS and RESIDENT_CHUNKS, which share the
+    // SMs with the other stream's kernel at once: waiting blocks take its slots
+    // (2562 x 55: 1086 -> 1134).
+    // Nor for grids of more than three such waves, where a launch's gap is small
+    // beside the launch (x1.40962 x 55: 11085 us with, 11050 without) and the
+    // waiting blocks take slots of another group's kernels in a batch (4 x 10242
+    // and 3 x 40962: 68.2 ms with, 66.7 without).
     const long long chunks = (long long)grid.x * grid.z * block.x * block.y;
     bool& ch = chained[on_side];
-    if (vec && ch && !prof && (chunks <= PRELOAD_CHUNKS || chunks > RESIDENT_CHUNKS)) {
+    const bool early = chunks <= PRELOAD_CHUNKS || (chunks > RESIDENT_CHUNKS && chunks <= 3 * RESIDENT_CHUNKS);
+    if (vec && ch && !prof && early) {
       cudaLaunchAttribute at{};
       at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
       at.val.programmaticStreamSerializationAllowed = 1;
