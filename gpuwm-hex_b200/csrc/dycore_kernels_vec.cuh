@@ -153,9 +153,40 @@ __device__ __forceinline__ void st4m(float* p, const V4& v, int k0, int lo, int 
 // c + s x with s = +-1: the product is exact, so the fused operation rounds
 // once, as c + (s x) does.
 __device__ __forceinline__ float fma_sign(float s, float x, float c) { return __fmaf_rn(s, x, c); }
+// c + (s x) y with s = +-1.  Strict: the product and the sum each round, two
+// operations.  Contracted: one fused operation of s x (exact) and y, as the
+// compiler contracts the expression itself; rounding x y first would be an
+// operation less precise and give a fast run other words.
+__device__ __forceinline__ float add_signed(float s, float x, float y, float c) {
+#if HEX_CONTRACT
+  return __fmaf_rn(s * x, y, c);
+#else
+  return fma_sign(s, x * y, c);
+#endif
+}
 __device__ __forceinline__ float fbits(int x) { return __int_as_float(x); }
 __device__ __forceinline__ int slot_edge(int x) { return x & ~1; }
 __device__ __forceinline__ float slot_sign(int x) { return __int_as_float(0x3f800000 | (x << 31)); }
+
+// Sums of two products, a b + c d and a b - c d, have two contracted forms,
+// and the compiler takes one by the code around them.  Where the two forms of
+// a kernel (B, below) or two versions of it took different ones, the choice is
+// written out, so that a fast run's words do not depend on it:
+// a b + c d with a b fused onto c d, and c - a b with a b fused onto c.
+__device__ __forceinline__ float sum_products(float a, float b, float c, float d) {
+#if HEX_CONTRACT
+  return __fmaf_rn(a, b, __fmul_rn(c, d));
+#else
+  return a * b + c * d;
+#endif
+}
+__device__ __forceinline__ float sub_product(float c, float a, float b) {
+#if HEX_CONTRACT
+  return __fmaf_rn(-a, b, c);
+#else
+  return c - a * b;
+#endif
+}
 
 // A divisor at level k: one in the padding levels, where the operands are
 // zero and 0 / 0 would take the division's slow path in every warp that
@@ -445,7 +476,7 @@ __global__ void HEX_BOUNDS(B, HEX_B_diag_edge) kv_diag_edge(HexGeo g, const floa
     for (int j = 0; j < 4; ++j) {
       const float gpt = (p1.a[j] - p0.a[j]) * idv;
       const float gpn = (q1.a[j] - q0.a[j]) * idc;
-      pve.a[j] = pve.a[j] - g.apvm_scale * (vt.a[j] * gpt + ue.a[j] * gpn);
+      pve.a[j] = sub_product(pve.a[j], g.apvm_scale, sum_products(vt.a[j], gpt, ue.a[j], gpn));
     }
   }
   st4m(pv_edge + e * S + k0, pve, k0, 0, g.L);
@@ -792,10 +823,10 @@ __global__ void HEX_BOUNDS(B, HEX_B_tend_cell) kv_tend_cell(HexGeo g, const floa
     for (int j = 0; j < 4; ++j) {
       // sg is +-1: sg x y rounds once, and adding or subtracting it in one
       // fused operation rounds as the separate sum does
-      res.a[j] = fma_sign(-d.sg, d.r.a[j] * d.et.a[j], res.a[j]);
+      res.a[j] = add_signed(-d.sg, d.r.a[j], d.et.a[j], res.a[j]);
       const float rprev = j == 0 ? d.rm : d.r.a[j - 1];
       const float rui = fm.a[j] * d.r.a[j] + fp.a[j] * rprev;
-      hres.a[j] = fma_sign(-d.sg, rui * d.ew.a[j], hres.a[j]);
+      hres.a[j] = add_signed(-d.sg, rui, d.ew.a[j], hres.a[j]);
     }
   });
   if (rk_step > 1) {
@@ -832,12 +863,13 @@ __global__ void HEX_BOUNDS(B, HEX_B_tend_cell) kv_tend_cell(HexGeo g, const floa
   flux3_chunk(th, vel, g.coef3, vt);
   const float fm5[5] = {fm.a[0], fm.a[1], fm.a[2], fm.a[3], k0 + 4 < S ? g.fzm[k0 + 4] : 0.0f};
   const float fp5[5] = {fp.a[0], fp.a[1], fp.a[2], fp.a[3], k0 + 4 < S ? g.fzp[k0 + 4] : 0.0f};
-  column_ends(k0, L, vt, [&](int d) {
-    return (k0 + d == 1 ? rww(d) : rwsw(d)) * (fm5[d] * th(d) + fp5[d] * th(d - 1));
-  });
+  // (interface 1 is formed below, from its flux and the correction at once)
+  column_ends(k0, L, vt, [&](int d) { return rwsw(d) * (fm5[d] * th(d) + fp5[d] * th(d - 1)); });
 #pragma unroll
   for (int d = 0; d < 5; ++d) {
-    const float with = vt[d] + (rwsw(d) - rww(d)) * (fm5[d] * ths(d) + fp5[d] * ths(d - 1));
+    const float drw = rwsw(d) - rww(d), te = fm5[d] * ths(d) + fp5[d] * ths(d - 1);
+    float with = vt[d] + drw * te;
+    if (d == 1 && k0 == 0) with = sum_products(rww(d), fm5[d] * th(d) + fp5[d] * th(d - 1), drw, te);
     vt[d] = k0 + d >= 1 && k0 + d < L - 1 ? with : vt[d];
   }
   // w flux (hexcore/driver.py:1176-1200)
@@ -860,7 +892,7 @@ __global__ void HEX_BOUNDS(B, HEX_B_tend_cell) kv_tend_cell(HexGeo g, const floa
       const float tprev = j == 0 ? d.tm : d.t.a[j - 1];
       const float f = fm.a[j] * d.t.a[j] + fp.a[j] * tprev;
       const float zt = fma_sign(copysignf(1.0f, d.t.a[j]), d.zb3.a[j], d.zb.a[j]);
-      trw.a[j] = fma_sign(-d.sg, zt * f, trw.a[j]);
+      trw.a[j] = add_signed(-d.sg, f, zt, trw.a[j]);
     }
   });
   // levels 0 and L hold 0 + the saved Euler term (every level ran the sums
@@ -1352,7 +1384,7 @@ __global__ void HEX_BOUNDS(B, HEX_B_recover_cell) kv_recover_cell(HexGeo g, int 
       const float rprev = j == 0 ? d.rm : d.r.a[j - 1];
       const float flux = fm.a[j] * d.r.a[j] + fp.a[j] * rprev;
       const float zt = fma_sign(copysignf(1.0f, flux), d.zb3.a[j], d.zb.a[j]);
-      acc[j] = fma_sign(d.sign, zt * flux, acc[j]);
+      acc[j] = add_signed(d.sign, zt, flux, acc[j]);
     }
   });
 #pragma unroll
@@ -1515,7 +1547,7 @@ __global__ void HEX_BOUNDS(B, HEX_B_tr_std) kv_tr_std(HexGeo g, int nT, float st
   };
   gather<B, HEX_U_tr_std>(preload<B>(g.maxE, load), n, load, [&](const In& d, int) {
 #pragma unroll
-    for (int j = 0; j < 4; ++j) t.a[j] = fma_sign(d.ts, d.h.a[j] * d.x.a[j], t.a[j]);
+    for (int j = 0; j < 4; ++j) t.a[j] = add_signed(d.ts, d.h.a[j], d.x.a[j], t.a[j]);
   });
   const float ia = g.inv_area[c];
   const Win qw = win<2, 2>(q_stage + toff + c * S, k0, S), www = win<0, 1>(ww + c * S, k0, S);
@@ -1572,9 +1604,10 @@ __global__ void HEX_BOUNDS(B, HEX_B_fct_target) kv_fct_target(HexGeo g, float st
   st4m(target + ii, td, k0, 0, g.L);
 }
 
-// low-order upwind vertical flux at interface j = k0 + d (old + 0 scalars)
-__device__ __forceinline__ float fct_fcol_win(float step, const Win& o, const Win& ww, int d) {
-  return step * (pos0(ww(d)) * (o(d - 1) + 0.0f) + neg0(ww(d)) * (o(d) + 0.0f));
+// low-order upwind vertical flux, before its factor step, at interface
+// j = k0 + d (old + 0 scalars)
+__device__ __forceinline__ float fct_fcol_win(const Win& o, const Win& ww, int d) {
+  return pos0(ww(d)) * (o(d - 1) + 0.0f) + neg0(ww(d)) * (o(d) + 0.0f);
 }
 // hexcore/transport.py:1919-2118 (v8.4.1 order): bounds, low-order mass,
 // incoming/outgoing antidiffusive totals and the scale factors.
@@ -1644,9 +1677,10 @@ __global__ void HEX_BOUNDS(B, HEX_B_fct_cell1) kv_fct_cell1(HexGeo g, int nT, fl
   tr_vflux_chunk(g, qw, www, k0, vr);
 #pragma unroll
   for (int d = 0; d < 5; ++d) {
-    fc[d] = fct_fcol_win(step, ow, www, d);
+    const float low = fct_fcol_win(ow, www, d);
+    fc[d] = step * low;
     const float h = step * vr[d];
-    vr[d] = k0 + d >= 1 && k0 + d < L ? h - fc[d] : h;
+    vr[d] = k0 + d >= 1 && k0 + d < L ? sub_product(h, step, low) : h;
   }
   // interfaces k0..k0+3 for the limited update (every interface of the
   // column is some thread's k0 + d, d < 4)
@@ -1682,7 +1716,7 @@ __global__ void HEX_BOUNDS(B, HEX_B_fct_cell1) kv_fct_cell1(HexGeo g, int nT, fl
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const float upw = dvs * (pos0(d.vel.a[j]) * (o0.a[j] + 0.0f) + neg0(d.vel.a[j]) * (o1.a[j] + 0.0f));
-      mass[j] = fma_sign(ts, upw * ia, mass[j]);
+      mass[j] = add_signed(ts, upw, ia, mass[j]);
       const float hres = step * d.h.a[j] - upw;
       const float sr = -ts * hres;
       s_out[j] = s_out[j] - pos0(sr) * ia;
@@ -1753,7 +1787,7 @@ __global__ void HEX_BOUNDS(B, HEX_B_fct_cell2) kv_fct_cell2(HexGeo g, int nT, co
   };
   gather<B, HEX_U_fct_cell2>(preload<B>(g.maxE, load), n, load, [&](const In& d, int) {
 #pragma unroll
-    for (int j = 0; j < 4; ++j) mass.a[j] = fma_sign(d.ts, d.h.a[j] * ia, mass.a[j]);
+    for (int j = 0; j < 4; ++j) mass.a[j] = add_signed(d.ts, d.h.a[j], ia, mass.a[j]);
   });
   const Win siw = win<1, 1>(scale_in + toff + c * S, k0, S), sow = win<1, 1>(scale_out + toff + c * S, k0, S);
   // interface k0 + 4 belongs to the next chunk; past the column's last chunk

@@ -4,6 +4,7 @@
 #include "hexdyn_ctx.h"
 #include "powf_gnu.cuh"
 
+#define HEX_CONTRACT 0  // -fmad as a constant
 namespace hexdyn_strict {
 #include "dycore_kernels.cuh"
 #include "dycore_kernels_vec.cuh"
