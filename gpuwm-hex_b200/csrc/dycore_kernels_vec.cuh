@@ -109,14 +109,20 @@ struct V4 {
 
 __device__ __forceinline__ V4 v4zero() { return V4{{0.0f, 0.0f, 0.0f, 0.0f}}; }
 
-// read-only (non-coherent) 128-bit load: the array is not written by the kernel
-__device__ __forceinline__ V4 ld4(const float* __restrict__ p) {
-  const float4 t = __ldg(reinterpret_cast<const float4*>(p));
+// Fields are read with ordinary (coherent) loads, whether the kernel writes
+// them or not: a kernel whose blocks are set up early is resident while its
+// predecessor still writes what it will read, and a read-only load is defined
+// only for words that do not change in a kernel's lifetime.  For the same
+// reason no kernel takes a field as `const float* __restrict__`, whose loads
+// the compiler may turn into read-only ones.
+__device__ __forceinline__ V4 ld4(const float* p) {
+  const float4 t = *reinterpret_cast<const float4*>(p);
   return V4{{t.x, t.y, t.z, t.w}};
 }
-// coherent 128-bit load for arrays the kernel also writes
-__device__ __forceinline__ V4 ld4rw(const float* p) {
-  const float4 t = *reinterpret_cast<const float4*>(p);
+// The mesh's arrays and records (HexGeo) are never written after the instance
+// is made: read-only loads.
+__device__ __forceinline__ V4 ldg4(const float* __restrict__ p) {
+  const float4 t = __ldg(reinterpret_cast<const float4*>(p));
   return V4{{t.x, t.y, t.z, t.w}};
 }
 __device__ __forceinline__ void st4(float* p, const V4& v) {
@@ -200,22 +206,30 @@ struct Win {
   float a[8];
   __device__ __forceinline__ float operator()(int d) const { return a[d + 2]; }
 };
-template <int LO, int HI>
-__device__ __forceinline__ Win win(const float* __restrict__ col, int k0, int S) {
+// MESH: a column of a mesh array.
+template <bool MESH, class T>
+__device__ __forceinline__ T ld(const T* p) {
+  if constexpr (MESH) return __ldg(p);
+  return *p;
+}
+template <int LO, int HI, bool MESH = false>
+__device__ __forceinline__ Win win(const float* col, int k0, int S) {
   Win w;
-  const V4 v = ld4(col + k0);
-#pragma unroll
-  for (int j = 0; j < 4; ++j) w.a[j + 2] = v.a[j];
+  const float4 v = ld<MESH>(reinterpret_cast<const float4*>(col + k0));
+  w.a[2] = v.x;
+  w.a[3] = v.y;
+  w.a[4] = v.z;
+  w.a[5] = v.w;
   w.a[0] = w.a[1] = w.a[6] = w.a[7] = 0.0f;
-  if (LO == 1 && k0 > 0) w.a[1] = __ldg(col + k0 - 1);
+  if (LO == 1 && k0 > 0) w.a[1] = ld<MESH>(col + k0 - 1);
   if (LO == 2 && k0 > 0) {
-    const float2 t = __ldg(reinterpret_cast<const float2*>(col + k0 - 2));
+    const float2 t = ld<MESH>(reinterpret_cast<const float2*>(col + k0 - 2));
     w.a[0] = t.x;
     w.a[1] = t.y;
   }
-  if (HI == 1 && k0 + 4 < S) w.a[6] = __ldg(col + k0 + 4);
+  if (HI == 1 && k0 + 4 < S) w.a[6] = ld<MESH>(col + k0 + 4);
   if (HI == 2 && k0 + 4 < S) {
-    const float2 t = __ldg(reinterpret_cast<const float2*>(col + k0 + 4));
+    const float2 t = ld<MESH>(reinterpret_cast<const float2*>(col + k0 + 4));
     w.a[6] = t.x;
     w.a[7] = t.y;
   }
@@ -268,7 +282,7 @@ __device__ __forceinline__ void gather(const Pre<B, T>& p, int n, Load load, Use
 __global__ void __launch_bounds__(256, HEX_B_clamp_scalars) kv_clamp_scalars(HexGeo g, float* __restrict__ q) {
   HEX_VEC_PARALLEL(g.nC)
   float* p = q + ((size_t)blockIdx.z * g.nC + ent) * g.S + k0;
-  V4 v = ld4rw(p);
+  V4 v = ld4(p);
 #pragma unroll
   for (int j = 0; j < 4; ++j)
     if (v.a[j] < 0.0f) v.a[j] = 0.0f;
@@ -281,7 +295,7 @@ __global__ void __launch_bounds__(256, HEX_B_clamp_scalars) kv_clamp_scalars(Hex
 // qtot(k-1))/2) above the surface, cqu = 1/(1 + sum of the two-cell means).
 // Scalars are stored [scalar][cell][S].
 template <int B>
-__global__ void HEX_BOUNDS(B, HEX_B_moist_cell) kv_moist_cell(HexGeo g, const float* __restrict__ q, int nT,
+__global__ void HEX_BOUNDS(B, HEX_B_moist_cell) kv_moist_cell(HexGeo g, const float* q, int nT,
                                              float* __restrict__ qtot, float* __restrict__ cqw) {
   HEX_VEC_PARALLEL(g.nC)
   const int c = ent, S = g.S;
@@ -310,7 +324,7 @@ __global__ void HEX_BOUNDS(B, HEX_B_moist_cell) kv_moist_cell(HexGeo g, const fl
 }
 
 template <int B>
-__global__ void HEX_BOUNDS(B, HEX_B_moist_edge) kv_moist_edge(HexGeo g, const float* __restrict__ q, int nT,
+__global__ void HEX_BOUNDS(B, HEX_B_moist_edge) kv_moist_edge(HexGeo g, const float* q, int nT,
                                              float* __restrict__ cqu) {
   HEX_VEC_PARALLEL(g.nE)
   const int e = ent, S = g.S;
@@ -336,7 +350,7 @@ __global__ void HEX_BOUNDS(B, HEX_B_moist_edge) kv_moist_edge(HexGeo g, const fl
 // ---------------------------------------------------------- diagnostics
 // hexcore/diagnostics.py:95 compute_solve_diagnostics, v8.4.1 stored inverses.
 
-__global__ void __launch_bounds__(256, HEX_B_diag_vertex) kv_diag_vertex(HexGeo g, const float* __restrict__ u, float* __restrict__ pv_vertex,
+__global__ void __launch_bounds__(256, HEX_B_diag_vertex) kv_diag_vertex(HexGeo g, const float* u, float* __restrict__ pv_vertex,
                                float* __restrict__ ke_vertex, float* __restrict__ vorticity) {
   HEX_VEC_PARALLEL(g.nV)
   const int v = ent, S = g.S;
@@ -368,8 +382,8 @@ __global__ void __launch_bounds__(256, HEX_B_diag_vertex) kv_diag_vertex(HexGeo 
 // Cell kinetic energy (v8.4.1 kite blend 0.625) and, with APVM, cell PV;
 // DIV: also the divergence of u (the horizontal mixing's input).
 template <bool DIV, int B>
-__global__ void HEX_BOUNDS(B, HEX_B_diag_cell) kv_diag_cell(HexGeo g, const float* __restrict__ u, const float* __restrict__ pv_vertex,
-                             const float* __restrict__ ke_vertex, float* __restrict__ ke_out,
+__global__ void HEX_BOUNDS(B, HEX_B_diag_cell) kv_diag_cell(HexGeo g, const float* u, const float* pv_vertex,
+                             const float* ke_vertex, float* __restrict__ ke_out,
                              float* __restrict__ pv_cell, float* __restrict__ divergence) {
   HEX_VEC_PARALLEL(g.nC)
   const int c = ent, S = g.S;
@@ -427,8 +441,8 @@ __global__ void HEX_BOUNDS(B, HEX_B_diag_cell) kv_diag_cell(HexGeo g, const floa
 
 // Tangential velocity (TRiSK weights) and edge PV with APVM upwinding.
 template <int B>
-__global__ void HEX_BOUNDS(B, HEX_B_diag_edge) kv_diag_edge(HexGeo g, const float* __restrict__ u, const float* __restrict__ pv_vertex,
-                             const float* __restrict__ pv_cell, float* __restrict__ v, float* __restrict__ pv_edge,
+__global__ void HEX_BOUNDS(B, HEX_B_diag_edge) kv_diag_edge(HexGeo g, const float* u, const float* pv_vertex,
+                             const float* pv_cell, float* __restrict__ v, float* __restrict__ pv_edge,
                              int recompute_v) {
   HEX_VEC_PARALLEL(g.nE)
   const int e = ent, S = g.S;
@@ -460,7 +474,7 @@ __global__ void HEX_BOUNDS(B, HEX_B_diag_edge) kv_diag_edge(HexGeo g, const floa
     }
     st4m(v + e * S + k0, vt, k0, 0, g.L);
   } else {
-    vt = ld4rw(v + e * S + k0);
+    vt = ld4(v + e * S + k0);
   }
   const int2 ve = __ldg(g.vends + e);
   const V4 p0 = ld4(pv_vertex + k0 + ve.x), p1 = ld4(pv_vertex + k0 + ve.y);
@@ -490,8 +504,8 @@ __device__ __forceinline__ float dpdz_of(const HexGeo& g, float rp, float qt, fl
 }
 
 // hexcore/dynamics.py:188 pressure_gradient_euler_tendency.
-__global__ void __launch_bounds__(256, HEX_B_euler_edge) kv_euler_edge(HexGeo g, const float* __restrict__ pp, const float* __restrict__ rp,
-                              const float* __restrict__ qtot, const float* __restrict__ cqu,
+__global__ void __launch_bounds__(256, HEX_B_euler_edge) kv_euler_edge(HexGeo g, const float* pp, const float* rp,
+                              const float* qtot, const float* cqu,
                               float* __restrict__ euler_ru) {
   HEX_VEC_PARALLEL(g.nE)
   const int e = ent, S = g.S;
@@ -501,9 +515,9 @@ __global__ void __launch_bounds__(256, HEX_B_euler_edge) kv_euler_edge(HexGeo g,
   // moisture terms of dpdz are read only with native moist coefficients
   const bool m = g.moist;
   const V4 q0 = m ? ld4(qtot + i0) : v4zero(), q1 = m ? ld4(qtot + i1) : v4zero();
-  const V4 b0 = m ? ld4(g.rho_base + i0) : v4zero(), b1 = m ? ld4(g.rho_base + i1) : v4zero();
-  const V4 z0 = ld4(g.zz + i0), z1 = ld4(g.zz + i1);
-  const V4 cq = ld4(cqu + e * S + k0), zx = ld4(g.zxu + e * S + k0);
+  const V4 b0 = m ? ldg4(g.rho_base + i0) : v4zero(), b1 = m ? ldg4(g.rho_base + i1) : v4zero();
+  const V4 z0 = ldg4(g.zz + i0), z1 = ldg4(g.zz + i1);
+  const V4 cq = ld4(cqu + e * S + k0), zx = ldg4(g.zxu + e * S + k0);
   const float idc = g.inv_dc[e];
   V4 out;
 #pragma unroll
@@ -517,7 +531,7 @@ __global__ void __launch_bounds__(256, HEX_B_euler_edge) kv_euler_edge(HexGeo g,
 
 // hexcore/dynamics.py:86 mass_flux_divergence (stored inverse area), 4 levels.
 template <int B>
-__device__ __forceinline__ V4 mass_flux_div4(const HexGeo& g, const float* __restrict__ ru, int c, int k0) {
+__device__ __forceinline__ V4 mass_flux_div4(const HexGeo& g, const float* ru, int c, int k0) {
   V4 acc = v4zero();
   const int n = g.deg[c];
   struct In {
@@ -539,18 +553,18 @@ __device__ __forceinline__ V4 mass_flux_div4(const HexGeo& g, const float* __res
 
 // hexcore/dynamics.py:122 density_tendency and hexcore/driver.py:2804 Euler w.
 template <int B>
-__global__ void HEX_BOUNDS(B, HEX_B_euler_cell) kv_euler_cell(HexGeo g, const float* __restrict__ ru, const float* __restrict__ rw,
-                              const float* __restrict__ pp, const float* __restrict__ rp,
-                              const float* __restrict__ qtot, const float* __restrict__ cqw,
+__global__ void HEX_BOUNDS(B, HEX_B_euler_cell) kv_euler_cell(HexGeo g, const float* ru, const float* rw,
+                              const float* pp, const float* rp,
+                              const float* qtot, const float* cqw,
                               float* __restrict__ tend_rho, float* __restrict__ euler_rw,
-                              const float* __restrict__ phys_rho, float* __restrict__ tend_rho_dyn) {
+                              const float* phys_rho, float* __restrict__ tend_rho_dyn) {
   HEX_VEC_PARALLEL(g.nC)
   const int c = ent, S = g.S, L = g.L;
   const V4 hd = mass_flux_div4<B>(g, ru, c, k0);
   const Win rww = win<0, 1>(rw + c * S, k0, S);
   const Win ppw = win<1, 0>(pp + c * S, k0, S), rpw = win<1, 0>(rp + c * S, k0, S);
   const bool m = g.moist;
-  const Win qtw = m ? win<1, 0>(qtot + c * S, k0, S) : Win{}, rbw = m ? win<1, 0>(g.rho_base + c * S, k0, S) : Win{};
+  const Win qtw = m ? win<1, 0>(qtot + c * S, k0, S) : Win{}, rbw = m ? win<1, 0, true>(g.rho_base + c * S, k0, S) : Win{};
   const V4 cq = m ? ld4(cqw + c * S + k0) : v4zero();
   V4 tr, er;
 #pragma unroll
@@ -584,7 +598,7 @@ __global__ void HEX_BOUNDS(B, HEX_B_euler_cell) kv_euler_cell(HexGeo g, const fl
 // ------------------------------------------------- stage tendencies
 // hexcore/dynamics.py:86 mass_flux_divergence of the stage rho*u.
 template <int B>
-__global__ void HEX_BOUNDS(B, HEX_B_hdiv) kv_hdiv(HexGeo g, const float* __restrict__ ru, float* __restrict__ hdiv) {
+__global__ void HEX_BOUNDS(B, HEX_B_hdiv) kv_hdiv(HexGeo g, const float* ru, float* __restrict__ hdiv) {
   HEX_VEC_PARALLEL(g.nC)
   st4m(hdiv + ent * g.S + k0, mass_flux_div4<B>(g, ru, ent, k0), k0, 0, g.L);
 }
@@ -592,8 +606,8 @@ __global__ void HEX_BOUNDS(B, HEX_B_hdiv) kv_hdiv(HexGeo g, const float* __restr
 // Third-order edge values of theta_m (levels) and w (interfaces):
 // hexcore/driver.py:1023-1034 and :1159-1172.
 template <int B>
-__global__ void HEX_BOUNDS(B, HEX_B_edge_adv) kv_edge_adv(HexGeo g, const float* __restrict__ ru, const float* __restrict__ theta,
-                            const float* __restrict__ w, float* __restrict__ edge_theta,
+__global__ void HEX_BOUNDS(B, HEX_B_edge_adv) kv_edge_adv(HexGeo g, const float* ru, const float* theta,
+                            const float* w, float* __restrict__ edge_theta,
                             float* __restrict__ edge_w) {
   HEX_VEC_PARALLEL(g.nE)
   const int e = ent, S = g.S;
@@ -611,7 +625,7 @@ __global__ void HEX_BOUNDS(B, HEX_B_edge_adv) kv_edge_adv(HexGeo g, const float*
   const auto cells = preload<B>(g.advW, load);
   const V4 r = ld4(ru + e * S + k0);
   const float rm = k0 > 0 ? ru[e * S + k0 - 1] : 0.0f;
-  const V4 fm = ld4(g.fzm + k0), fp = ld4(g.fzp + k0);
+  const V4 fm = ldg4(g.fzm + k0), fp = ldg4(g.fzp + k0);
   // The stencil weight A + (coef3 sign(v)) B is one of the record's two
   // sums, by the sign bit of the level's velocity.
   bool nt[4], nw[4];
@@ -669,11 +683,11 @@ __device__ __forceinline__ void column_ends(int k0, int L, float (&f)[5], F edge
 // RAYLEIGH: the upper Rayleigh damping of u is compiled in (an instance
 // without it keeps the common path's registers).
 template <bool RAYLEIGH, int B>
-__global__ void HEX_BOUNDS(B, HEX_B_tend_u) kv_tend_u(HexGeo g, const float* __restrict__ u, const float* __restrict__ rw,
-                          const float* __restrict__ rho, const float* __restrict__ pv_edge,
-                          const float* __restrict__ ke, const float* __restrict__ hdiv,
-                          const float* __restrict__ euler_ru, float* __restrict__ tend_ru,
-                          const float* __restrict__ phys_ru, float first_dts, float* __restrict__ ru_p0,
+__global__ void HEX_BOUNDS(B, HEX_B_tend_u) kv_tend_u(HexGeo g, const float* u, const float* rw,
+                          const float* rho, const float* pv_edge,
+                          const float* ke, const float* hdiv,
+                          const float* euler_ru, float* __restrict__ tend_ru,
+                          const float* phys_ru, float first_dts, float* __restrict__ ru_p0,
                           float* __restrict__ ru_avg0) {
   HEX_VEC_PARALLEL(g.nE)
   const int e = ent, S = g.S;
@@ -741,7 +755,7 @@ __global__ void HEX_BOUNDS(B, HEX_B_tend_u) kv_tend_u(HexGeo g, const float* __r
   const V4 rh0 = ld4(rho + i0), rh1 = ld4(rho + i1);
   const V4 ke0 = ld4(ke + i0), ke1 = ld4(ke + i1);
   const V4 hd0 = ld4(hdiv + i0), hd1 = ld4(hdiv + i1);
-  const V4 rz = ld4(g.rdzw + k0);
+  const V4 rz = ldg4(g.rdzw + k0);
   const V4 eu = ld4(euler_ru + e * S + k0);
   const float idc = g.inv_dc[e];
   V4 out;
@@ -782,20 +796,20 @@ __global__ void HEX_BOUNDS(B, HEX_B_tend_u) kv_tend_u(HexGeo g, const float* __r
 // tend_rt (hexcore/driver.py:933), tend_rw (:1081) + Euler w, then
 // hexcore/acoustic.py:246 convert_w_tendency_to_omega.
 template <int B>
-__global__ void HEX_BOUNDS(B, HEX_B_tend_cell) kv_tend_cell(HexGeo g, const float* __restrict__ ru, const float* __restrict__ ru_s,
-                             const float* __restrict__ rw, const float* __restrict__ rws,
-                             const float* __restrict__ theta, const float* __restrict__ theta_s,
-                             const float* __restrict__ w, const float* __restrict__ edge_theta,
-                             const float* __restrict__ edge_w, const float* __restrict__ euler_rw,
-                             const float* __restrict__ tend_ru, float* __restrict__ tend_rt,
-                             float* __restrict__ tend_rw, int rk_step, const float* __restrict__ mix_theta,
+__global__ void HEX_BOUNDS(B, HEX_B_tend_cell) kv_tend_cell(HexGeo g, const float* ru, const float* ru_s,
+                             const float* rw, const float* rws,
+                             const float* theta, const float* theta_s,
+                             const float* w, const float* edge_theta,
+                             const float* edge_w, const float* euler_rw,
+                             const float* tend_ru, float* __restrict__ tend_rt,
+                             float* __restrict__ tend_rw, int rk_step, const float* mix_theta,
                              HexPhysCell phys) {
   HEX_VEC_PARALLEL(g.nC)
   const int c = ent, S = g.S, L = g.L;
   const int n = g.deg[c];
   const float ia = g.inv_area[c];
   const int2* slots = g.slot + c * g.maxE;
-  const V4 fm = ld4(g.fzm + k0), fp = ld4(g.fzp + k0);
+  const V4 fm = ldg4(g.fzm + k0), fp = ldg4(g.fzp + k0);
   // horizontal parts: rho-theta flux divergence, RK>1 correction, w flux
   V4 res = v4zero(), hres = v4zero();
   struct Flux {
@@ -848,13 +862,13 @@ __global__ void HEX_BOUNDS(B, HEX_B_tend_cell) kv_tend_cell(HexGeo g, const floa
   const auto omega = [&](int s) {
     const int sl = __ldg(&slots[s].x), eo = slot_edge(sl);
     const int zi = (c * g.maxE + s) * S + k0;
-    return Omega{slot_sign(sl), k0 > 0 ? (tend_ru + k0 - 1)[eo] : 0.0f, ld4(tend_ru + k0 + eo), ld4(g.zb + zi),
-                 ld4(g.zb3 + zi)};
+    return Omega{slot_sign(sl), k0 > 0 ? (tend_ru + k0 - 1)[eo] : 0.0f, ld4(tend_ru + k0 + eo), ldg4(g.zb + zi),
+                 ldg4(g.zb3 + zi)};
   };
   const auto omegas = preload<B>(g.maxE, omega);
   const Win th = win<2, 2>(theta + c * S, k0, S), ths = win<1, 1>(theta_s + c * S, k0, S);
   const Win rww = win<1, 1>(rw + c * S, k0, S), rwsw = win<0, 1>(rws + c * S, k0, S);
-  const Win ww = win<2, 2>(w + c * S, k0, S), zzw = win<1, 0>(g.zz + c * S, k0, S);
+  const Win ww = win<2, 2>(w + c * S, k0, S), zzw = win<1, 0, true>(g.zz + c * S, k0, S);
   const V4 er = ld4(euler_rw + c * S + k0);
   // theta flux at the interfaces (hexcore/driver.py:1048-1076)
   float vt[5], vw[5], vel[5];
@@ -877,7 +891,7 @@ __global__ void HEX_BOUNDS(B, HEX_B_tend_cell) kv_tend_cell(HexGeo g, const floa
   for (int d = 0; d < 5; ++d) vel[d] = 0.5f * (rww(d) + rww(d - 1));
   flux3_chunk(ww, vel, 1.0f, vw);
   column_ends(k0, L, vw, [&](int d) { return 0.25f * (rww(d) + rww(d - 1)) * (ww(d) + ww(d - 1)); });
-  const V4 rz = ld4(g.rdzw + k0), rzu = ld4(g.rdzu + k0);
+  const V4 rz = ldg4(g.rdzw + k0), rzu = ldg4(g.rdzu + k0);
   V4 trt, trw;
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
@@ -945,7 +959,7 @@ __device__ __forceinline__ float np_min(float a, float b) { return a != a ? a : 
 
 // hexcore/mixing_v841.py:615 smagorinsky_2d: kdiff of every cell level from
 // the deformation of the edge normal (u) and tangential (v) velocities.
-__global__ void __launch_bounds__(256, HEX_B_smag_kdiff) kv_smag_kdiff(HexGeo g, const float* __restrict__ u, const float* __restrict__ v,
+__global__ void __launch_bounds__(256, HEX_B_smag_kdiff) kv_smag_kdiff(HexGeo g, const float* u, const float* v,
                               float* __restrict__ kdiff) {
   HEX_VEC_PARALLEL(g.nC)
   const int c = ent, S = g.S;
@@ -986,9 +1000,9 @@ __global__ void __launch_bounds__(256, HEX_B_smag_kdiff) kv_smag_kdiff(HexGeo g,
 // hexcore/mixing.py:391-474 second-order momentum filter: delsq_u and the
 // Euler u term plus rho_edge kdiff delsq_u meshScalingDel2 (rho_edge the
 // diagnostics' h_edge of the subcycle's start density).
-__global__ void __launch_bounds__(256, HEX_B_mix_edge2) kv_mix_edge2(HexGeo g, const float* __restrict__ div, const float* __restrict__ vort,
-                             const float* __restrict__ kdiff, const float* __restrict__ rho,
-                             const float* __restrict__ euler_ru, float* __restrict__ delsq_u,
+__global__ void __launch_bounds__(256, HEX_B_mix_edge2) kv_mix_edge2(HexGeo g, const float* div, const float* vort,
+                             const float* kdiff, const float* rho,
+                             const float* euler_ru, float* __restrict__ delsq_u,
                              float* __restrict__ mix_u) {
   HEX_VEC_PARALLEL(g.nE)
   const int e = ent, S = g.S;
@@ -1015,8 +1029,8 @@ __global__ void __launch_bounds__(256, HEX_B_mix_edge2) kv_mix_edge2(HexGeo g, c
 
 // hexcore/mixing.py:533 (w, interfaces 1..L-1) and :638 (theta) second-order
 // filters of a cell, with their Laplacians delsq_w and delsq_theta.
-__global__ void __launch_bounds__(256, HEX_B_mix_cell2) kv_mix_cell2(HexGeo g, const float* __restrict__ kdiff, const float* __restrict__ rho,
-                             const float* __restrict__ w, const float* __restrict__ theta,
+__global__ void __launch_bounds__(256, HEX_B_mix_cell2) kv_mix_cell2(HexGeo g, const float* kdiff, const float* rho,
+                             const float* w, const float* theta,
                              float* __restrict__ w_mix, float* __restrict__ delsq_w,
                              float* __restrict__ theta_mix, float* __restrict__ delsq_theta) {
   HEX_VEC_PARALLEL(g.nC)
@@ -1064,7 +1078,7 @@ __global__ void __launch_bounds__(256, HEX_B_mix_cell2) kv_mix_cell2(HexGeo g, c
 
 // hexcore/mixing.py:464-476: the Laplacians of delsq_u at vertices
 // (vorticity form) and cells (divergence form).
-__global__ void __launch_bounds__(256, HEX_B_mix_lap_vertex) kv_mix_lap_vertex(HexGeo g, const float* __restrict__ delsq_u,
+__global__ void __launch_bounds__(256, HEX_B_mix_lap_vertex) kv_mix_lap_vertex(HexGeo g, const float* delsq_u,
                                   float* __restrict__ delsq_vort) {
   HEX_VEC_PARALLEL(g.nV)
   const int v = ent, S = g.S;
@@ -1079,7 +1093,7 @@ __global__ void __launch_bounds__(256, HEX_B_mix_lap_vertex) kv_mix_lap_vertex(H
   }
   st4m(delsq_vort + v * S + k0, acc, k0, 0, g.L);
 }
-__global__ void __launch_bounds__(256, HEX_B_mix_lap_cell) kv_mix_lap_cell(HexGeo g, const float* __restrict__ delsq_u,
+__global__ void __launch_bounds__(256, HEX_B_mix_lap_cell) kv_mix_lap_cell(HexGeo g, const float* delsq_u,
                                 float* __restrict__ delsq_div) {
   HEX_VEC_PARALLEL(g.nC)
   const int c = ent, S = g.S;
@@ -1097,8 +1111,8 @@ __global__ void __launch_bounds__(256, HEX_B_mix_lap_cell) kv_mix_lap_cell(HexGe
 }
 
 // hexcore/mixing.py:478-490 fourth-order momentum filter (subtracted).
-__global__ void __launch_bounds__(256, HEX_B_mix_edge4) kv_mix_edge4(HexGeo g, const float* __restrict__ rho,
-                             const float* __restrict__ delsq_div, const float* __restrict__ delsq_vort,
+__global__ void __launch_bounds__(256, HEX_B_mix_edge4) kv_mix_edge4(HexGeo g, const float* rho,
+                             const float* delsq_div, const float* delsq_vort,
                              float* __restrict__ mix_u) {
   HEX_VEC_PARALLEL(g.nE)
   const int e = ent, S = g.S;
@@ -1112,7 +1126,7 @@ __global__ void __launch_bounds__(256, HEX_B_mix_edge4) kv_mix_edge4(HexGeo g, c
   const float scale = g.mix_del4[e] * g.smag_h4;
   const float r_dc = scale * g.smag_div_factor * g.inv_dc[e];
   const float r_dv = scale * g.inv_dv_lim[e];
-  V4 mu = ld4rw(mix_u + e * S + k0);
+  V4 mu = ld4(mix_u + e * S + k0);
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
     const float h = 0.5f * (r0.a[j] + r1.a[j]);
@@ -1124,13 +1138,13 @@ __global__ void __launch_bounds__(256, HEX_B_mix_edge4) kv_mix_edge4(HexGeo g, c
 
 // hexcore/mixing.py:576-590 and :719-733 fourth-order w and theta filters
 // (when visc4 > 0), then the saved w term euler_rw + w filter (driver.py:2870).
-__global__ void __launch_bounds__(256, HEX_B_mix_cell4) kv_mix_cell4(HexGeo g, const float* __restrict__ delsq_w,
-                             const float* __restrict__ delsq_theta, const float* __restrict__ euler_rw,
-                             const float* __restrict__ w_mix, float* __restrict__ theta_mix,
+__global__ void __launch_bounds__(256, HEX_B_mix_cell4) kv_mix_cell4(HexGeo g, const float* delsq_w,
+                             const float* delsq_theta, const float* euler_rw,
+                             const float* w_mix, float* __restrict__ theta_mix,
                              float* __restrict__ mix_w) {
   HEX_VEC_PARALLEL(g.nC)
   const int c = ent, S = g.S, L = g.L;
-  V4 tw = ld4(w_mix + c * S + k0), tt = ld4rw(theta_mix + c * S + k0);
+  V4 tw = ld4(w_mix + c * S + k0), tt = ld4(theta_mix + c * S + k0);
   if (g.smag_h4 > 0.0f) {
     const int n = g.deg[c];
     const float scale = g.smag_h4 * g.inv_area[c];
@@ -1164,10 +1178,10 @@ __global__ void __launch_bounds__(256, HEX_B_mix_cell4) kv_mix_cell4(HexGeo g, c
 // update of this substep (hexcore/acoustic_v841.py:416-460).  mode 0: first
 // substep (ru_p = dts*tend_ru); 1: damping + update; 2: damping only.
 __global__ void __launch_bounds__(256, HEX_B_ac_edge) kv_ac_edge(HexGeo g, int mode, int old_is_zero, float dts, float inv_dts,
-                           const float* __restrict__ tend_ru, const float* __restrict__ rtpp_new,
-                           const float* __restrict__ rtpp_old, const float* __restrict__ rho_pp,
-                           const float* __restrict__ theta_s, const float* __restrict__ exner_s,
-                           const float* __restrict__ cqu, float* __restrict__ ru_p, float* __restrict__ ru_avg) {
+                           const float* tend_ru, const float* rtpp_new,
+                           const float* rtpp_old, const float* rho_pp,
+                           const float* theta_s, const float* exner_s,
+                           const float* cqu, float* __restrict__ ru_p, float* __restrict__ ru_avg) {
   HEX_VEC_PARALLEL(g.nE)
   const int e = ent, S = g.S;
   const int jj = e * S + k0;
@@ -1184,7 +1198,7 @@ __global__ void __launch_bounds__(256, HEX_B_ac_edge) kv_ac_edge(HexGeo g, int m
   const int i0 = ends.x + k0, i1 = ends.y + k0;
   // smdiv_base * (1/dts), the damping coefficient of the edge's mesh
   const float damp_coef = g.smdiv_edge[e] * inv_dts;
-  V4 r = ld4rw(ru_p + jj);
+  V4 r = ld4(ru_p + jj);
   const V4 n0 = ld4(rtpp_new + i0), n1 = ld4(rtpp_new + i1);
   const V4 o0 = old_is_zero ? v4zero() : ld4(rtpp_old + i0);
   const V4 o1 = old_is_zero ? v4zero() : ld4(rtpp_old + i1);
@@ -1196,10 +1210,10 @@ __global__ void __launch_bounds__(256, HEX_B_ac_edge) kv_ac_edge(HexGeo g, int m
     r.a[j] = r.a[j] + damp_coef * (d0 - d1) * (1.0f - 0.0f) / (t0.a[j] + t1.a[j]);
   }
   if (mode == 1) {
-    const V4 z0 = ld4(g.zz + i0), z1 = ld4(g.zz + i1), x0 = ld4(exner_s + i0), x1 = ld4(exner_s + i1);
+    const V4 z0 = ldg4(g.zz + i0), z1 = ldg4(g.zz + i1), x0 = ld4(exner_s + i0), x1 = ld4(exner_s + i1);
     const V4 p0 = ld4(rho_pp + i0), p1 = ld4(rho_pp + i1);
-    const V4 cq = ld4(cqu + jj), zx = ld4(g.zxu + jj), t = ld4(tend_ru + jj);
-    V4 av = ld4rw(ru_avg + jj);
+    const V4 cq = ld4(cqu + jj), zx = ldg4(g.zxu + jj), t = ld4(tend_ru + jj);
+    V4 av = ld4(ru_avg + jj);
     const float idc = g.inv_dc[e];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
@@ -1221,19 +1235,19 @@ __global__ void __launch_bounds__(256, HEX_B_ac_edge) kv_ac_edge(HexGeo g, int m
 // damp: the divergence damping of the stage's last acoustic substep
 // (kv_ac_edge mode 2: rtpp_new/rtpp_old its output/input, old_is_zero when
 // it was the first) is applied to ru_p here, stored, and recovered from.
-__global__ void __launch_bounds__(256, HEX_B_recover_edge) kv_recover_edge(HexGeo g, const float* __restrict__ ru_s, float* ru_p,
-                                const float* __restrict__ ru_avg, const float* __restrict__ rp_s,
-                                const float* __restrict__ rho_pp, float* __restrict__ ru_out,
+__global__ void __launch_bounds__(256, HEX_B_recover_edge) kv_recover_edge(HexGeo g, const float* ru_s, float* ru_p,
+                                const float* ru_avg, const float* rp_s,
+                                const float* rho_pp, float* __restrict__ ru_out,
                                 float* __restrict__ u_out, float* __restrict__ flux_u, int flux_mode,
                                 float inv_steps, float inv_splits, int damp, int old_is_zero, float inv_dts,
-                                const float* __restrict__ rtpp_new, const float* __restrict__ rtpp_old,
-                                const float* __restrict__ theta_s) {
+                                const float* rtpp_new, const float* rtpp_old,
+                                const float* theta_s) {
   HEX_VEC_PARALLEL(g.nE)
   const int e = ent, S = g.S;
   const int jj = e * S + k0;
   const int2 ends = __ldg(g.ends + e);
   const int i0 = ends.x + k0, i1 = ends.y + k0;
-  V4 rp = ld4rw(ru_p + jj);
+  V4 rp = ld4(ru_p + jj);
   if (damp) {
     const float damp_coef = g.smdiv_edge[e] * inv_dts;
     const V4 n0 = ld4(rtpp_new + i0), n1 = ld4(rtpp_new + i1);
@@ -1249,7 +1263,7 @@ __global__ void __launch_bounds__(256, HEX_B_recover_edge) kv_recover_edge(HexGe
     st4m(ru_p + jj, rp, k0, 0, g.L);
   }
   const V4 a0 = ld4(rp_s + i0), a1 = ld4(rp_s + i1), b0 = ld4(rho_pp + i0), b1 = ld4(rho_pp + i1);
-  const V4 c0 = ld4(g.rho_base + i0), c1 = ld4(g.rho_base + i1);
+  const V4 c0 = ldg4(g.rho_base + i0), c1 = ldg4(g.rho_base + i1);
   const V4 rs = ld4(ru_s + jj);
   V4 ru, uo;
 #pragma unroll
@@ -1263,7 +1277,7 @@ __global__ void __launch_bounds__(256, HEX_B_recover_edge) kv_recover_edge(HexGe
   st4m(u_out + jj, uo, k0, 0, g.L);
   if (flux_mode & 4) {
     const V4 av = ld4(ru_avg + jj);
-    const V4 old = (flux_mode & 1) ? v4zero() : ld4rw(flux_u + jj);
+    const V4 old = (flux_mode & 1) ? v4zero() : ld4(flux_u + jj);
     V4 acc;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
@@ -1280,11 +1294,11 @@ __global__ void __launch_bounds__(256, HEX_B_recover_edge) kv_recover_edge(HexGe
 // rw end conditions, theta_m, Exner and p' at stage 3, w from
 // hexcore/terrain.py:491 recover_velocities, and the split w-flux average.
 template <int B>
-__global__ void HEX_BOUNDS(B, HEX_B_recover_cell) kv_recover_cell(HexGeo g, int stage3, const float* __restrict__ rp_s,
-                                const float* __restrict__ rtp_s, const float* __restrict__ rw_s,
-                                const float* __restrict__ rho_pp, const float* __restrict__ rtpp,
-                                const float* __restrict__ rw_p, const float* __restrict__ ww_avg,
-                                const float* __restrict__ ru_new, HexState out, HexSide side,
+__global__ void HEX_BOUNDS(B, HEX_B_recover_cell) kv_recover_cell(HexGeo g, int stage3, const float* rp_s,
+                                const float* rtp_s, const float* rw_s,
+                                const float* rho_pp, const float* rtpp,
+                                const float* rw_p, const float* ww_avg,
+                                const float* ru_new, HexState out, HexSide side,
                                 float* __restrict__ flux_w, int flux_mode, float inv_steps, float inv_splits,
                                 int* flag, float* __restrict__ hdiv_next) {
   HEX_VEC_PARALLEL(g.nC)
@@ -1298,17 +1312,17 @@ __global__ void HEX_BOUNDS(B, HEX_B_recover_cell) kv_recover_cell(HexGeo g, int 
     const int sl = __ldg(&g.slot[c * g.maxE + s].x), eo = slot_edge(sl);
     const int zi = (c * g.maxE + s) * S + k0;
     return In{slot_sign(sl),       __ldg(g.sdv + c * g.maxE + s), k0 > 0 ? (ru_new + k0 - 1)[eo] : 0.0f,
-              ld4(ru_new + k0 + eo), ld4(g.zb + zi),              ld4(g.zb3 + zi)};
+              ld4(ru_new + k0 + eo), ldg4(g.zb + zi),              ldg4(g.zb3 + zi)};
   };
   const auto edges = preload<B>(g.maxE, load);
   // candidate density at the levels k0-1 .. k0+3 (recomputed, not read back)
   const Win rpw = win<1, 0>(rp_s + c * S, k0, S), ppw = win<1, 0>(rho_pp + c * S, k0, S);
-  const Win rbw = win<1, 0>(g.rho_base + c * S, k0, S);
+  const Win rbw = win<1, 0, true>(g.rho_base + c * S, k0, S);
   float rho_w[5];
 #pragma unroll
   for (int d = -1; d < 4; ++d) rho_w[d + 1] = rpw(d) + ppw(d) + rbw(d);
   {
-    const V4 tp = ld4(rtp_s + ii), tq = ld4(rtpp + ii), tb = ld4(g.rtheta_base + ii);
+    const V4 tp = ld4(rtp_s + ii), tq = ld4(rtpp + ii), tb = ldg4(g.rtheta_base + ii);
     V4 rho, rt, rp, rtp, th;
     bool bad = false;
 #pragma unroll
@@ -1327,7 +1341,7 @@ __global__ void HEX_BOUNDS(B, HEX_B_recover_cell) kv_recover_cell(HexGeo g, int 
     st4m(side.rtheta_p + ii, rtp, k0, 0, g.L);
     st4m(side.theta_m + ii, th, k0, 0, g.L);
     if (stage3) {
-      const V4 zz = ld4(g.zz + ii), eb = ld4(g.exner_base + ii);
+      const V4 zz = ldg4(g.zz + ii), eb = ldg4(g.exner_base + ii);
       V4 ex, pp;
       int badp = 0;
 #pragma unroll
@@ -1357,11 +1371,11 @@ __global__ void HEX_BOUNDS(B, HEX_B_recover_cell) kv_recover_cell(HexGeo g, int 
   }
   st4m(out.rho_w + ii, rwv, k0, 0, g.L + 1);
   const int n = g.deg[c];
-  const Win zzw = win<1, 0>(g.zz + c * S, k0, S);
+  const Win zzw = win<1, 0, true>(g.zz + c * S, k0, S);
   float acc[4];
   bool bottom = k0 == 0;
   float bacc = 0.0f;
-  const V4 fm = ld4(g.fzm + k0), fp = ld4(g.fzp + k0);
+  const V4 fm = ldg4(g.fzm + k0), fp = ldg4(g.fzp + k0);
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
     const int k = k0 + j;
@@ -1412,7 +1426,7 @@ __global__ void HEX_BOUNDS(B, HEX_B_recover_cell) kv_recover_cell(HexGeo g, int 
   }
   if (flux_mode & 4) {
     const V4 av = ld4(ww_avg + ii);
-    const V4 old = (flux_mode & 1) ? v4zero() : ld4rw(flux_w + ii);
+    const V4 old = (flux_mode & 1) ? v4zero() : ld4(flux_w + ii);
     V4 fa;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
@@ -1437,7 +1451,7 @@ __global__ void HEX_BOUNDS(B, HEX_B_recover_cell) kv_recover_cell(HexGeo g, int 
 #define HEX_TR_GROUP 3
 #endif
 template <int B>
-__global__ void HEX_BOUNDS(B, HEX_B_tr_edge) kv_tr_edge(HexGeo g, int nT, int mono, const float* __restrict__ q, const float* __restrict__ hv,
+__global__ void HEX_BOUNDS(B, HEX_B_tr_edge) kv_tr_edge(HexGeo g, int nT, int mono, const float* q, const float* hv,
                            float* __restrict__ out) {
   HEX_VEC_TRACER(g.nE, (nT + HEX_TR_GROUP - 1) / HEX_TR_GROUP)
   constexpr int TG = HEX_TR_GROUP;
@@ -1525,10 +1539,10 @@ __device__ __forceinline__ void tr_vflux_chunk(const HexGeo& g, const Win& q, co
 
 // hexcore/transport.py:1649 advance_scalars (RK1/RK2 of split transport).
 template <int B>
-__global__ void HEX_BOUNDS(B, HEX_B_tr_std) kv_tr_std(HexGeo g, int nT, float step, float wn, const float* __restrict__ q_old,
-                          const float* __restrict__ q_stage, const float* __restrict__ rho_old,
-                          const float* __restrict__ rho_new, const float* __restrict__ hv,
-                          const float* __restrict__ ww, const float* __restrict__ edge_q,
+__global__ void HEX_BOUNDS(B, HEX_B_tr_std) kv_tr_std(HexGeo g, int nT, float step, float wn, const float* q_old,
+                          const float* q_stage, const float* rho_old,
+                          const float* rho_new, const float* hv,
+                          const float* ww, const float* edge_q,
                           float* __restrict__ q_out) {
   HEX_VEC_TRACER(g.nC, nT)
   const int c = ent, S = g.S;
@@ -1554,7 +1568,7 @@ __global__ void HEX_BOUNDS(B, HEX_B_tr_std) kv_tr_std(HexGeo g, int nT, float st
   const V4 ro = ld4(rho_old + ii), rn = ld4(rho_new + ii), qo = ld4(q_old + toff + ii);
   float vf[5];
   tr_vflux_chunk(g, qw, www, k0, vf);
-  const V4 rz = ld4(g.rdzw + k0);
+  const V4 rz = ldg4(g.rdzw + k0);
   V4 out;
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
@@ -1569,8 +1583,8 @@ __global__ void HEX_BOUNDS(B, HEX_B_tr_std) kv_tr_std(HexGeo g, int nT, float st
 
 // hexcore/transport.py:1887-1906 split-transport target density.
 template <int B>
-__global__ void HEX_BOUNDS(B, HEX_B_fct_target) kv_fct_target(HexGeo g, float step, const float* __restrict__ rho_old,
-                              const float* __restrict__ hv, const float* __restrict__ ww,
+__global__ void HEX_BOUNDS(B, HEX_B_fct_target) kv_fct_target(HexGeo g, float step, const float* rho_old,
+                              const float* hv, const float* ww,
                               float* __restrict__ target, int* flag) {
   HEX_VEC_PARALLEL(g.nC)
   const int c = ent, S = g.S, L = g.L;
@@ -1617,10 +1631,10 @@ __device__ __forceinline__ float fct_fcol_win(const Win& o, const Win& ww, int d
 // the bounds already load; the min/max over neighbours and the mass sums
 // still run in slot order, so the words are those of the two-loop form.
 template <bool ACROSS, int B>
-__global__ void HEX_BOUNDS(B, HEX_B_fct_cell1) kv_fct_cell1(HexGeo g, int nT, float step, const float* __restrict__ q_old,
-                             const float* __restrict__ q_stage, const float* __restrict__ rho_old,
-                             const float* __restrict__ hv, const float* __restrict__ ww,
-                             const float* __restrict__ high_e, const float* __restrict__ target,
+__global__ void HEX_BOUNDS(B, HEX_B_fct_cell1) kv_fct_cell1(HexGeo g, int nT, float step, const float* q_old,
+                             const float* q_stage, const float* rho_old,
+                             const float* hv, const float* ww,
+                             const float* high_e, const float* target,
                              float* __restrict__ scale_in, float* __restrict__ scale_out, float* __restrict__ mass_out,
                              float* __restrict__ vres_out) {
   HEX_VEC_TRACER(g.nC, nT)
@@ -1671,7 +1685,7 @@ __global__ void HEX_BOUNDS(B, HEX_B_fct_cell1) kv_fct_cell1(HexGeo g, int nT, fl
       }
     }
   }
-  const V4 ro = ld4(rho_old + ii), td = ld4(target + ii), rz = ld4(g.rdzw + k0);
+  const V4 ro = ld4(rho_old + ii), td = ld4(target + ii), rz = ldg4(g.rdzw + k0);
   float mass[4], s_in[4], s_out[4], vr[5];
   float fc[5];  // the low-order upwind flux at the inner interfaces
   tr_vflux_chunk(g, qw, www, k0, vr);
@@ -1738,9 +1752,9 @@ __global__ void HEX_BOUNDS(B, HEX_B_fct_cell1) kv_fct_cell1(HexGeo g, int nT, fl
 }
 
 // hexcore/transport.py:1919-2118: the limited antidiffusive edge flux.
-__global__ void __launch_bounds__(256, HEX_B_fct_edge) kv_fct_edge(HexGeo g, int nT, float step, const float* __restrict__ q_old, const float* __restrict__ hv,
-                            const float* __restrict__ high_e, const float* __restrict__ scale_in,
-                            const float* __restrict__ scale_out, float* __restrict__ hres_lim) {
+__global__ void __launch_bounds__(256, HEX_B_fct_edge) kv_fct_edge(HexGeo g, int nT, float step, const float* q_old, const float* hv,
+                            const float* high_e, const float* scale_in,
+                            const float* scale_out, float* __restrict__ hres_lim) {
   HEX_VEC_TRACER(g.nE, nT)
   const int e = ent, S = g.S;
   const size_t toff = (size_t)tr * g.nC * S;
@@ -1765,10 +1779,10 @@ __global__ void __launch_bounds__(256, HEX_B_fct_edge) kv_fct_edge(HexGeo g, int
 // hexcore/transport.py:1919-2118: limited update of the monotonic stage.
 // The vertical residual fluxes are those kv_fct_cell1 formed (vres).
 template <int B>
-__global__ void HEX_BOUNDS(B, HEX_B_fct_cell2) kv_fct_cell2(HexGeo g, int nT, const float* __restrict__ vres,
-                             const float* __restrict__ scale_in, const float* __restrict__ scale_out,
-                             const float* __restrict__ mass_in, const float* __restrict__ hres_lim,
-                             const float* __restrict__ target, float* __restrict__ q_out) {
+__global__ void HEX_BOUNDS(B, HEX_B_fct_cell2) kv_fct_cell2(HexGeo g, int nT, const float* vres,
+                             const float* scale_in, const float* scale_out,
+                             const float* mass_in, const float* hres_lim,
+                             const float* target, float* __restrict__ q_out) {
   HEX_VEC_TRACER(g.nC, nT)
   const int c = ent, S = g.S;
   const int ii = c * S + k0;
@@ -1883,9 +1897,9 @@ __device__ __forceinline__ float from_above(float a0) { return __shfl_down_sync(
 
 // hexcore/acoustic_v841.py:81 compute_vertical_implicit_coefficients_v841.
 #define HEX_VCOEFV_SMEM_ARRAYS 3
-__global__ void __launch_bounds__(256, HEX_B_vcoef) kv_vcoef(HexGeo g, float dts2, const float* __restrict__ exner, const float* __restrict__ theta,
-                         const float* __restrict__ rtp, const float* __restrict__ cqw,
-                         const float* __restrict__ qtot, float* __restrict__ cofwr, float* __restrict__ cofwz,
+__global__ void __launch_bounds__(256, HEX_B_vcoef) kv_vcoef(HexGeo g, float dts2, const float* exner, const float* theta,
+                         const float* rtp, const float* cqw,
+                         const float* qtot, float* __restrict__ cofwr, float* __restrict__ cofwz,
                          float* __restrict__ coftz, float* __restrict__ cofwt, float* __restrict__ a_tri,
                          float* __restrict__ alpha_tri, float* __restrict__ gamma_tri, int* flag) {
   extern __shared__ float sm[];
@@ -1900,14 +1914,14 @@ __global__ void __launch_bounds__(256, HEX_B_vcoef) kv_vcoef(HexGeo g, float dts
   V4 zz = v4zero(), ex = v4zero(), th = v4zero();
   V4 wr = v4zero(), wz = v4zero(), tz = v4zero(), wt = v4zero();
   if (live) {
-    zz = ld4(g.zz + ii);
+    zz = ldg4(g.zz + ii);
     ex = ld4(exner + ii);
     th = ld4(theta + ii);
   }
   const float zzm = from_below(zz.a[3]), exm = from_below(ex.a[3]), thm = from_below(th.a[3]);
   if (live) {
-    const V4 cq = ld4(cqw + ii), qt = ld4(qtot + ii), rb = ld4(g.rho_base + ii), rtb = ld4(g.rtheta_base + ii);
-    const V4 rp = ld4(rtp + ii), eb = ld4(g.exner_base + ii);
+    const V4 cq = ld4(cqw + ii), qt = ld4(qtot + ii), rb = ldg4(g.rho_base + ii), rtb = ldg4(g.rtheta_base + ii);
+    const V4 rp = ld4(rtp + ii), eb = ldg4(g.exner_base + ii);
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const int k = k0 + j;
@@ -2010,15 +2024,15 @@ __global__ void __launch_bounds__(256, HEX_B_vcoef) kv_vcoef(HexGeo g, float dts
 #define HEX_AC_DSS_ZERO_SKIP 1
 #endif
 template <int B>
-__global__ void HEX_BOUNDS(B, HEX_B_ac_cell) kv_ac_cell(HexGeo g, int first, float dts, float dts2, const float* __restrict__ ru_p,
-                           const float* __restrict__ theta_s, const float* __restrict__ tend_rho,
-                           const float* __restrict__ tend_rt, const float* __restrict__ tend_rw,
-                           const float* __restrict__ cofwr, const float* __restrict__ cofwz,
-                           const float* __restrict__ coftz, const float* __restrict__ cofwt,
-                           const float* __restrict__ a_tri, const float* __restrict__ alpha_tri,
-                           const float* __restrict__ gamma_tri, const float* __restrict__ rho_zz,
-                           const float* __restrict__ w, const float* __restrict__ rw,
-                           const float* __restrict__ rw_save, const float* __restrict__ rtpp_old,
+__global__ void HEX_BOUNDS(B, HEX_B_ac_cell) kv_ac_cell(HexGeo g, int first, float dts, float dts2, const float* ru_p,
+                           const float* theta_s, const float* tend_rho,
+                           const float* tend_rt, const float* tend_rw,
+                           const float* cofwr, const float* cofwz,
+                           const float* coftz, const float* cofwt,
+                           const float* a_tri, const float* alpha_tri,
+                           const float* gamma_tri, const float* rho_zz,
+                           const float* w, const float* rw,
+                           const float* rw_save, const float* rtpp_old,
                            float* __restrict__ rtpp_new, float* __restrict__ rho_pp, float* __restrict__ rw_p,
                            float* __restrict__ ww_avg) {
   extern __shared__ float sm[];
@@ -2040,7 +2054,7 @@ __global__ void HEX_BOUNDS(B, HEX_B_ac_cell) kv_ac_cell(HexGeo g, int first, flo
   V4 rs = v4zero(), ts = v4zero(), rho_old = v4zero(), rt_old = v4zero();
   if (live) {
     if (!first) {
-      const V4 t = ld4rw(rw_p + ii);
+      const V4 t = ld4(rw_p + ii);
 #pragma unroll
       for (int j = 0; j < 4; ++j) rwp_old.a[j] = k0 + j <= L ? t.a[j] : 0.0f;
     }
@@ -2056,7 +2070,7 @@ __global__ void HEX_BOUNDS(B, HEX_B_ac_cell) kv_ac_cell(HexGeo g, int first, flo
     sts4(s_al + k0, ld4(alpha_tri + ii));
     sts4(s_ga + k0, ld4(gamma_tri + ii));
     if (!first) {
-      rho_old = ld4rw(rho_pp + ii);
+      rho_old = ld4(rho_pp + ii);
       rt_old = ld4(rtpp_old + ii);
     }
     const int n = g.deg[c];
@@ -2082,7 +2096,7 @@ __global__ void HEX_BOUNDS(B, HEX_B_ac_cell) kv_ac_cell(HexGeo g, int first, flo
       }
     });
     const V4 trho = ld4(tend_rho + ii), trt = ld4(tend_rt + ii);
-    const V4 wav = first ? v4zero() : ld4rw(ww_avg + ii);
+    const V4 wav = first ? v4zero() : ld4(ww_avg + ii);
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const int k = k0 + j;
@@ -2101,7 +2115,7 @@ __global__ void HEX_BOUNDS(B, HEX_B_ac_cell) kv_ac_cell(HexGeo g, int first, flo
   // phase 2: right-hand side of the w system (levels k-1 from the lane below)
   V4 zz = v4zero(), cwt = v4zero();
   if (live) {
-    zz = ld4(g.zz + ii);
+    zz = ldg4(g.zz + ii);
     cwt = ld4(cofwt + ii);
   }
   const float ts_m = from_below(ts.a[3]), rt_m = from_below(rt_old.a[3]), rs_m = from_below(rs.a[3]);
@@ -2177,7 +2191,7 @@ __global__ void HEX_BOUNDS(B, HEX_B_ac_cell) kv_ac_cell(HexGeo g, int first, flo
     const V4 rsv = ld4(rw_save + ii), rwv = ld4(rw + ii);
     V4 wo;
     if (damping) {
-      const V4 dss = ld4(g.dss + ii), wv = ld4(w + ii);
+      const V4 dss = ldg4(g.dss + ii), wv = ld4(w + ii);
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         const int k = k0 + j;
