@@ -16,15 +16,11 @@ struct HexGeo {
   const int* coe;        // [E][2]
   const int* eoc;        // [C][maxE]
   const int* coc;        // [C][maxE]
-  const int* voc;        // [C][maxE]
   const int* deg;        // [C]
-  const int* voe;        // [E][2]
   const int* eov;        // [V][3]
   const int* eoe;        // [E][maxE2]
   const int* neoe;       // [E]
-  const int* adv_cells;  // [E][advW]
   const int* n_adv;      // [E]
-  const int* kite_slot;  // [C][maxE]
   // Stencil records: what a neighbour loop needs of one neighbour, packed for
   // one or two loads.  Entities are given as word offsets (index x S) into
   // their [entity][level] fields; S is a multiple of 8, so the low bits of an
@@ -49,14 +45,11 @@ struct HexGeo {
   const float* inv_dv;
   const float* inv_area;
   const float* inv_area_tri;
-  const float* kite;      // [V][3]
   const float* weights;   // [E][maxE2]
   const float* f_vertex;
   const float* f_edge;
   const float* cos_angle;
   const float* sin_angle;
-  const float* adv;       // [E][advW]
-  const float* adv3;      // [E][advW]
   // level vectors [S]
   const float* fzm;
   const float* fzp;

@@ -385,22 +385,18 @@ int build(HexDynHandle* h, const HexDynDesc& d, const std::vector<float>* smdiv_
   cudaError_t e;
 #define UP(dst, vec) \
   if ((e = upload(c, &(dst), vec)) != cudaSuccess) return cuda_fail(e, "upload " #dst);
-  UP(g.coe, coe) UP(g.eoc, eoc) UP(g.coc, coc) UP(g.voc, voc) UP(g.deg, deg) UP(g.voe, voe) UP(g.eov, eov)
-  UP(g.eoe, eoe) UP(g.neoe, neoe) UP(g.adv_cells, advc) UP(g.n_adv, nadv) UP(g.kite_slot, kite_slot)
-  UP(g.csign, csign) UP(g.vsign, vsign)
+  UP(g.coe, coe) UP(g.eoc, eoc) UP(g.coc, coc) UP(g.deg, deg) UP(g.eov, eov) UP(g.eoe, eoe) UP(g.neoe, neoe)
+  UP(g.n_adv, nadv) UP(g.csign, csign) UP(g.vsign, vsign)
   std::vector<float> tmp;
   tmp.assign(d.dc_edge, d.dc_edge + nE); UP(g.dc, tmp)
   tmp.assign(d.dv_edge, d.dv_edge + nE); UP(g.dv, tmp)
   UP(g.inv_dc, recip(d.dc_edge, nE)) UP(g.inv_dv, recip(d.dv_edge, nE))
   UP(g.inv_area, recip(d.area_cell, nC)) UP(g.inv_area_tri, recip(d.area_triangle, nV))
-  tmp.assign(d.kite_areas, d.kite_areas + 3 * (size_t)nV); UP(g.kite, tmp)
   tmp.assign(d.weights_on_edge, d.weights_on_edge + (size_t)nE * g.maxE2); UP(g.weights, tmp)
   tmp.assign(d.f_vertex, d.f_vertex + nV); UP(g.f_vertex, tmp)
   tmp.assign(d.f_edge, d.f_edge + nE); UP(g.f_edge, tmp)
   tmp.assign(d.cos_angle_edge, d.cos_angle_edge + nE); UP(g.cos_angle, tmp)
   tmp.assign(d.sin_angle_edge, d.sin_angle_edge + nE); UP(g.sin_angle, tmp)
-  tmp.assign(d.adv_coefs, d.adv_coefs + (size_t)nE * g.advW); UP(g.adv, tmp)
-  tmp.assign(d.adv_coefs_3rd, d.adv_coefs_3rd + (size_t)nE * g.advW); UP(g.adv3, tmp)
   UP(g.fzm, pad_vector(d.fzm, L, S)) UP(g.fzp, pad_vector(d.fzp, L, S))
   UP(g.rdzw, pad_vector(d.rdzw, L, S)) UP(g.rdzu, pad_vector(d.rdzu, L, S))
   UP(g.u_init, pad_vector(d.u_init, L, S)) UP(g.v_init, pad_vector(d.v_init, L, S))
