@@ -752,9 +752,9 @@ __global__ void __launch_bounds__(256) k_adam(const __grid_constant__ AdamSegmen
     const int r = r0 + y;
     if (r >= s.rows || c >= s.cols) continue;
     const size_t i = (size_t)r * s.cols + c;
-    const float gi = s.g[i] + s.decay * s.w[i];
     // (the contractions written out, so that the weights of a training run do
     // not depend on how the compiler schedules this loop)
+    const float gi = __fmaf_rn(s.decay, s.w[i], s.g[i]);
     const float m = __fmaf_rn(a.b1, s.m1[i], __fmul_rn(1.0f - a.b1, gi));
     const float v = __fmaf_rn(a.b2, s.m2[i], __fmul_rn(__fmul_rn(1.0f - a.b2, gi), gi));
     s.m1[i] = m;

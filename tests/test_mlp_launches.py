@@ -4,6 +4,7 @@ kernels at sizes that are no multiple of their 32 x 32 tiles."""
 
 import ctypes as C
 
+import numpy as np
 import pytest
 
 torch = pytest.importorskip("torch")
@@ -118,3 +119,37 @@ def test_layers_in_one_launch_equal_single_steps(n):
         exact = t.double().sum(1)
         bound = 2.0 ** -24 * 200 * t.double().abs().sum(1)
         assert bool(((db.double() - exact).abs() <= bound).all())
+
+
+def _fma32(a, b, c):
+    """a b + c of float32 arrays rounded once: the product is exact in 64 bits,
+    and the sum rounded to odd there rounds to float32 as the exact sum does."""
+    x, y = a.astype(np.float64) * b.astype(np.float64), np.asarray(c, np.float64)
+    s = x + y
+    t = s - x
+    err = (x - (s - t)) + (y - t)
+    even = (s.view(np.int64) & 1) == 0
+    s = np.where((err != 0) & even, np.nextafter(s, np.where(err > 0, np.inf, -np.inf)), s)
+    return s.astype(np.float32)
+
+
+# one rounding per operation and the three contractions that the kernel writes out
+@pytest.mark.parametrize("decay", [0.0, 0.01, 0.3])
+def test_adam_rounds_as_written(decay):
+    from hexdyn import mlp
+
+    p, f = mlp._ptr, np.float32
+    w, m1, g = (_rand(65, 97) for _ in range(3))
+    m2 = _rand(65, 97).square()
+    lr, b1, b2, eps = f(1e-3), f(0.9), f(0.999), f(1e-8)
+    hw, h1, h2, hg = (t.cpu().numpy() for t in (w, m1, m2, g))
+    gi = _fma32(np.full_like(hw, f(decay)), hw, hg)
+    m = _fma32(np.full_like(hw, b1), h1, (f(1) - b1) * gi)
+    v = _fma32(np.full_like(hw, b2), h2, ((f(1) - b2) * gi) * gi)
+    # the first step: the bias corrections are 1 - b1 and 1 - b2
+    want = hw - lr * (m / (f(1) - b1)) / (np.sqrt(v / (f(1) - b2)) + eps)
+    assert mlp.load().hexmlp_adam(p(w), p(m1), p(m2), p(g), 65, 97, float(lr), float(b1), float(b2), float(eps), 1,
+                                  decay, None, None, mlp._stream()) == 0
+    for got, expect in ((m1, m), (m2, v), (w, want)):
+        assert expect.dtype == np.float32
+        assert np.array_equal(got.cpu().numpy().view(np.uint32), expect.view(np.uint32))
