@@ -1,7 +1,16 @@
 """The third-order vertical fluxes divide by 12 in two operations
-(dycore_kernels.cuh: div12_wide, div12_any): the same words as IEEE
-division, over every mantissa and exponent range on the CPU, and in the
-step with tracers in the range where the two-operation form does not hold.
+(dycore_kernels.cuh: div12_wide, div12_any): the same words as IEEE division.
+
+The two operations are restated in NumPy here, and swept over every mantissa of
+both signs at the exponents that can differ: while x RL, x RH and the quotient
+are normal numbers (biased exponent 29 and up) every operation scales with the
+power of two, so one exponent stands for all; below, the rounding of x RL is at
+most 2^-150, which is the largest part of a step of the quotient, 1/32, at the
+smallest exponent that the form serves (9), and half of that at each above.
+Both ends of that range and exponents between are swept, and the top.  The
+64-bit form is swept where it is used, over the subnormal and smallest normal
+numbers.  On the GPU the step itself is compared with the oracle, with tracers
+in the range where the two-operation form does not hold.
 """
 
 import numpy as np
@@ -36,19 +45,21 @@ def same(a, b):
     return np.array_equal(a.view(np.uint32)[~nan], b.view(np.uint32)[~nan])
 
 
-@pytest.mark.parametrize("exponent", [9, 10, 64, 127, 250, 254])
-def test_two_operations_divide_every_mantissa(exponent):
+@pytest.mark.parametrize("sign", [0, 1])
+@pytest.mark.parametrize("exponent", [9, 10, 11, 13, 17, 29, 30, 64, 127, 250, 254])
+def test_two_operations_divide_every_mantissa(exponent, sign):
     mantissa = np.arange(1 << 23, dtype=np.uint32)
-    x = (np.uint32(exponent << 23) | mantissa).view(F32)
-    assert x[0] >= SMALL
+    x = (np.uint32(sign << 31 | exponent << 23) | mantissa).view(F32)
+    assert np.abs(x[0]) >= SMALL
     assert same(wide(x), quotient(x))
 
 
-@pytest.mark.parametrize("exponent", [0, 1, 2, 4, 8])
-def test_64_bit_form_divides_every_small_mantissa(exponent):
+@pytest.mark.parametrize("sign", [0, 1])
+@pytest.mark.parametrize("exponent", range(9))
+def test_64_bit_form_divides_every_small_mantissa(exponent, sign):
     mantissa = np.arange(1 << 23, dtype=np.uint32)
-    x = (np.uint32(exponent << 23) | mantissa).view(F32)
-    assert x[-1] < SMALL
+    x = (np.uint32(sign << 31 | exponent << 23) | mantissa).view(F32)
+    assert np.abs(x[-1]) < SMALL
     assert same(any_range(x), quotient(x))
 
 
