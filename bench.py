@@ -81,15 +81,17 @@ def kernel_bytes(name: str, C: int, E: int, V: int, L: int, T: int, maxE: int = 
     acoustic cell pass also reads dss, rho_zz and w."""
     cl, ci, el, vl = C * L, C * (L + 1), E * L, V * L
     tcl, tel = T * C * L, T * E * L
-    conn_c = C * maxE * 3 + C * 2          # eoc, csign (+ coc/voc) and deg, inv_area
-    conn_e = E * 2 + E * 4                 # coe and per-edge metrics
-    adv = E * advW * 3                     # adv, adv3, adv_cells
+    # the stencil records (csrc/dycore_geo.cuh), in words
+    conn_c = C * maxE * 3 + C * 2          # slot or eslot (2), sdv; deg, inv_area
+    conn_e = E * 2 + E * 4                 # ends (or vends) and per-edge metrics
+    adv = E * advW * 3                     # adv_off, adv_pm (2)
     zb = 2 * C * maxE * (L + 1)
     words = {
-        "k_diag_vertex": el + 2 * vl + V * 8,
-        "k_diag_cell": el + 2 * vl + 2 * cl + conn_c,
+        "k_diag_vertex": el + 2 * vl + V * 14,                      # three vedge records (4 words)
+        "k_diag_cell": el + 2 * vl + 2 * cl + conn_c + C * maxE,    # eslot and vslot
         "k_diag_edge": 3 * el + vl + cl + conn_e,                  # u, cached v, pv_edge out
-        "k_diag_edge_v": 3 * el + vl + cl + conn_e + E * 24,       # u (+ neighbours), v out, pv_edge out
+        # u (+ neighbours), v out, pv_edge out; E * 24: six nbr records of two neighbours
+        "k_diag_edge_v": 3 * el + vl + cl + conn_e + E * 24,
         "k_moist_cell": tcl + 2 * cl,
         "k_clamp_scalars": 2 * tcl,
         "k_moist_edge": tcl + el + conn_e,

@@ -26,8 +26,11 @@ struct Launcher {
   cudaStream_t main_st = nullptr;  // the caller's stream while launches go to the side stream
   bool on_side = false;            // (the caller's stream may be the legacy stream, handle 0)
   int next_event = 0;
-  // Whether the last operation of this launcher on the caller's / the side
-  // stream was a kernel launch (then the next may start early, see run()).
+  // Whether a kernel of this launcher precedes the next one on the caller's /
+  // the side stream with nothing between them but event records (then the next
+  // may start early, see run()).  A record is complete with the kernel before
+  // it, whatever follows; a wait, a host hook or an event node of a captured
+  // graph between two kernels ends the chain.
   bool chained[2] = {false, false};
   // Independent kernels: fork() makes the side stream wait for everything
   // launched so far, side() sends the following launches there, and
@@ -42,7 +45,9 @@ struct Launcher {
     const bool hooked = ctx.stage_hook != nullptr || ctx.exchange_hook != nullptr;
     return !(hooked && (long long)ctx.geo.nE * (ctx.geo.S / 4) <= RESIDENT_CHUNKS);
   }
-  // chunks of a launch that four 256-thread blocks on each of 148 SMs hold at once
+  // A launch of as many chunks as 1024 threads on each of 148 SMs: the measure
+  // of "fills the GPU" here and in run().  (What a launch really keeps resident
+  // depends on its kernel's registers, 768 to 2048 threads an SM.)
   static constexpr long long RESIDENT_CHUNKS = 256LL * 4 * 148;
   void signal(cudaStream_t from, cudaStream_t to) {
     if (err != cudaSuccess) return;
@@ -74,13 +79,14 @@ struct Launcher {
     signal(ctx.side_stream, st);
   }
   // Whether a level-vector launch over n entities (x nz) takes the kernel that
-  // preloads its neighbours (B > 0 in dycore_kernels_vec.cuh): up to two
-  // 128-thread blocks per SM, which those kernels' registers leave resident at
-  // once, the chain of dependent loads is a launch's time.  Two steps of 162
-  // cells x 12: 811 -> 696 us, of 642 x 41: 1154 -> 1032; above, resident warps
-  // count for more (2562 x 55, 36 k chunks of cells and 107 k of edges: none
-  // 1185 us, cells 1088, both 1111 us; 10242 x 55 with cells at 143 k: 3937 ->
-  // 4135).
+  // preloads its neighbours (B > 0 in dycore_kernels_vec.cuh): on a small grid
+  // the chain of dependent loads is a launch's time.  One limit for all of them,
+  // two 128-thread blocks per SM, which the largest of these kernels (206
+  // registers) just keeps resident; the smaller ones (40 registers and up) were
+  // not tried above it one by one.  Two steps of 162 cells x 12: 811 -> 696 us,
+  // of 642 x 41: 1154 -> 1032; above, resident warps count for more on the whole
+  // (2562 x 55, 36 k chunks of cells and 107 k of edges: none 1185 us, cells
+  // 1088, both 1111 us; 10242 x 55 with cells at 143 k: 3937 -> 4135).
   static constexpr long long PRELOAD_CHUNKS = 40000;
   bool pre(long long n, int nz = 1) const {
     return ctx.geo.nbrW >= 1 && n * nz * (ctx.geo.S / 4) <= PRELOAD_CHUNKS;
@@ -144,10 +150,11 @@ struct Launcher {
     // Not for grids between PRELOAD_CHUNKS and RESIDENT_CHUNKS, which share the
     // SMs with the other stream's kernel at once: waiting blocks take its slots
     // (2562 x 55: 1086 -> 1134).
-    // Nor for grids of more than three such waves, where a launch's gap is small
-    // beside the launch (x1.40962 x 55: 11085 us with, 11050 without) and the
-    // waiting blocks take slots of another group's kernels in a batch (4 x 10242
-    // and 3 x 40962: 68.2 ms with, 66.7 without).
+    // Nor for grids of more than three times RESIDENT_CHUNKS, where a launch's
+    // gap is small beside the launch (x1.40962 x 55: 11085 us with, 11050
+    // without) and the waiting blocks take slots of another group's kernels in a
+    // batch (4 x 10242 and 3 x 40962: 68.2 ms with, 66.7 without).
+    // Profiled launches (hexdyn_profile_steps, the autotuner's) are never early.
     const long long chunks = (long long)grid.x * grid.z * block.x * block.y;
     bool& ch = chained[on_side];
     const bool early = chunks <= PRELOAD_CHUNKS || (chunks > RESIDENT_CHUNKS && chunks <= 3 * RESIDENT_CHUNKS);

@@ -180,6 +180,9 @@ class TensorCoreMLP:
 
     # --------------------------------------------------------- workspace
     def _workspace(self, M: int) -> dict:
+        """Buffers of M rows, kept with the network.  Training keeps dZ^T of
+        every hidden layer (depth x p_hidden x M bf16), so that the weight
+        gradients of all layers are one launch."""
         import torch
 
         ws = self._ws.get(M)

@@ -199,15 +199,17 @@ int hexdyn_step_host(HexDynHandle* h, const float* const* in, float* const* out,
 int hexdyn_read_flag(HexDynHandle* h, void* stream, int* flag_out);
 
 /* Run nsteps eager steps with a CUDA event pair around every kernel launch
- * and write one line per kernel, "name launches total_ms", into out.
- * (Profiling entry point; the reference's launch_timed,
- * hexcore/cuda_subcycle_graphs.py:45-62.) */
+ * and write one line per kernel, "name launches total_ms", into out.  These
+ * launches run one after the other on `stream`; those of a step itself also
+ * overlap (a second stream, blocks set up early), so the times are the
+ * kernels' own and not shares of a step's.  (Profiling entry point; the
+ * reference's launch_timed, hexcore/cuda_subcycle_graphs.py:45-62.) */
 int hexdyn_profile_steps(HexDynHandle* h, void* stream, int nsteps, char* out, size_t len);
 
 /* Autotuner of launch shapes (no counterpart in the reference, whose
  * kernels launch fixed shapes): times every kernel of `steps_per_candidate`
  * eager steps with 64, 96, 128, 160, 192, 224 and 256 threads per block
- * (CUDA events per launch; a block holds threads / (S/4) cells or edges, or
+ * (CUDA events per launch, as hexdyn_profile_steps; a block holds threads / (S/4) cells or edges, or
  * threads / 16 columns in the column sweeps), keeps the fastest block size of
  * every launch label, and restores the state and sidecar the steps started
  * from; captured graphs are captured again with the tuned shapes.  Results
